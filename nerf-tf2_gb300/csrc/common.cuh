@@ -63,27 +63,26 @@ constexpr int kTableElems = kRgbBOff + 4;
 constexpr long long kFp32TableOff = kGemmWElems;  // floats
 constexpr long long kFp32PackBytes = (kGemmWElems + kTableElems) * 4;
 
-// BF16 pack: per GEMM layer, K chunks of 32; chunk (n, k) byte offset
-// (k/8)*(N*16) + n*16 + (k%8)*2 (K-major core matrices, no swizzle). Then
-// the fp32 table at a 1 KB aligned offset, then the same weights in the
-// CTA-pair layout (pair_w_byte).
+// Tensor-core weights (BF16: E = 2 bytes, FP8-e4m3: E = 1), laid out for the
+// 2-SM MMA in which each CTA of a pair holds one N-half of every weight
+// chunk. Per GEMM layer, chunks of kPairStage bytes per half (kPairStage / H
+// bytes of K for the H = N/2 rows of a half: 64 BF16 or 128 E4M3 where N is
+// 256, twice that where N is 128; the last chunk may be shorter); per chunk
+// N-half 0 then N-half 1, each as K-major core matrices of 8 rows x 16 bytes:
+// (kb/16)*(H*16) + n'*16 + kb%16 for byte kb of the chunk's K and row n', so
+// that a CTA's half of a chunk is one contiguous copy.
+constexpr uint32_t kPairStage = 16384;
+NG_HD long long pair_w_byte(int g, int k, int n, int E) {
+  const int H = gemm_n(g) / 2, per = (int)kPairStage / H, kb = k * E, c = kb / per;
+  const int kc = gemm_kp(g) * E - c * per < per ? gemm_kp(g) * E - c * per : per;
+  return gemm_w_offset(g) * E + (long long)c * (2 * kPairStage) + (long long)(n / H) * (H * kc) +
+         ((kb - c * per) / 16) * (H * 16) + (n % H) * 16 + kb % 16;
+}
+
+// BF16 pack: the weights, then the FP32 table at a 1 KB aligned offset.
 constexpr long long kBf16WBytes = kGemmWElems * 2;
 constexpr long long kBf16TableOff = (kBf16WBytes + 1023) / 1024 * 1024;  // bytes
-
-// CTA-pair layout, for the 2-SM MMA in which each CTA of a pair holds one
-// N-half of every weight chunk: per GEMM layer, chunks of kPairKch K-rows
-// (the last may be shorter, kc rows); per chunk N-half 0 then N-half 1, each
-// (k/8)*(N/2*16) + n'*16 + (k%8)*2 with n' = n mod N/2, so that a CTA's half
-// of a chunk is one contiguous copy.
-constexpr int kPairKch = 64;
-constexpr long long kBf16PairOff = (kBf16TableOff + (long long)kTableElems * 4 + 1023) / 1024 * 1024;
-constexpr long long kBf16PackBytes = kBf16PairOff + kBf16WBytes;
-NG_HD long long pair_w_byte(int g, int k, int n) {
-  const int N = gemm_n(g), H = N / 2, c = k / kPairKch, kk = k % kPairKch;
-  const int kc = gemm_kp(g) - c * kPairKch < kPairKch ? gemm_kp(g) - c * kPairKch : kPairKch;
-  return kBf16PairOff + gemm_w_offset(g) * 2 + (long long)c * (kPairKch * N * 2) + (long long)(n / H) * (kc * H * 2) +
-         (kk / 8) * (H * 16) + (n % H) * 16 + (kk % 8) * 2;
-}
+constexpr long long kBf16PackBytes = kBf16TableOff + (long long)kTableElems * 4;
 
 // Stored activations of one row for training (floats): enc_xyz [64] | h0..h7
 // [8 x 256] | bottleneck [256] | enc_dir [32] | h9 [128].
@@ -92,11 +91,19 @@ constexpr int kActsEncDir = 64 + 9 * 256;     // 2368
 constexpr int kActsLd = kActsEncDir + 32 + 128;  // 2528
 NG_HD int acts_offset(int g) { return g < 9 ? 64 + 256 * g : kActsEncDir + 32; }
 
-// FP8 pack: the same chunks as BF16 with one byte per weight, e4m3 of
-// W[k][n] / scale[n] (per output channel, scale = max_k |W[k][n]| / 448);
-// core matrices hold 16 K-elements: chunk (n, k) byte offset
-// (k/16)*(N*16) + n*16 + (k%16). Then the FP32 table, then the scales
-// [kBiasElems] (same indexing as the biases).
+// FP8 pack: e4m3 of W[k][n] / scale[n] (per output channel, scale = max_k
+// |W[k][n]| / 448), then the FP32 table, then the scales [kBiasElems] (same
+// indexing as the biases). Output channel n is row fp8_row(g, n) of the
+// layer's weights: in the layers whose epilogue reads the accumulator in
+// 16x256b fragments (all but dense_9, which feeds the rgb head row by row)
+// the channels of each 16 are ordered so that a thread's accumulator
+// pairs of two adjacent 8-column groups, rows {2q, 2q+1} and {8+2q, 9+2q},
+// are channels 4q .. 4q+3.
+NG_HD int fp8_row(int g, int n) {
+  if (g == 9) return n;
+  const int q = (n % 16) / 4, e = n % 4;
+  return n - n % 16 + (e < 2 ? 2 * q + e : 8 + 2 * q + e - 2);
+}
 constexpr long long kFp8WBytes = kGemmWElems;
 constexpr long long kFp8TableOff = (kFp8WBytes + 1023) / 1024 * 1024;  // bytes
 constexpr long long kFp8ScaleOff = kFp8TableOff + (long long)kTableElems * 4;

@@ -32,16 +32,10 @@ __global__ void pack_kernel(const float *__restrict__ flat, int precision, unsig
       reinterpret_cast<float *>(out)[i] = v;
     } else if (precision == NERFGB_PREC_FP8) {
       const float sc = reinterpret_cast<const float *>(out + kFp8ScaleOff)[bias_offset(g) + n];
-      int c = k >> 5, kk = k & 31;
-      long long byte = gemm_w_offset(g) + (long long)c * (32 * N) + (kk >> 4) * (N * 16) + n * 16 + (kk & 15);
       __nv_fp8_e4m3 q(sc > 0.0f ? v / sc : 0.0f);
-      out[byte] = *reinterpret_cast<unsigned char *>(&q);
+      out[pair_w_byte(g, k, fp8_row(g, n), 1)] = *reinterpret_cast<unsigned char *>(&q);
     } else {
-      int c = k >> 5, kk = k & 31;
-      long long byte = gemm_w_offset(g) * 2 + (long long)c * (32 * N * 2) + (kk >> 3) * (N * 16) + n * 16 +
-                       (kk & 7) * 2;
-      *reinterpret_cast<__nv_bfloat16 *>(out + byte) = __float2bfloat16_rn(v);
-      *reinterpret_cast<__nv_bfloat16 *>(out + pair_w_byte(g, k, n)) = __float2bfloat16_rn(v);
+      *reinterpret_cast<__nv_bfloat16 *>(out + pair_w_byte(g, k, n, 2)) = __float2bfloat16_rn(v);
     }
     return;
   }
