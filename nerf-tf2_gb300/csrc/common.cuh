@@ -119,6 +119,25 @@ __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b)
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 
+// (x0 + y0, x1 + y1) in one paired FP32 add (round to nearest even, as two
+// FADDs).
+__device__ __forceinline__ void add_f32x2(float &d0, float &d1, float x0, float x1, float y0, float y1) {
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\n"
+      "mov.b64 {%0, %1}, d;\n}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+}
+
+// (x0 * y0 + z0, x1 * y1 + z1) in one paired FP32 FMA (each rounded once,
+// as fmaf).
+__device__ __forceinline__ void fma_f32x2(float &d0, float &d1, float x0, float x1, float y0, float y1, float z0,
+                                          float z1) {
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(x0), "f"(x1), "f"(y0), "f"(y1), "f"(z0), "f"(z1));
+}
+
 // fp32(2^l) * fp32(pi): PositionalEncoder multipliers (model.py:309-311).
 __device__ __forceinline__ float enc_multiplier(int l) {
   return fmul((float)(1u << l), 3.14159265358979323846f);

@@ -1,16 +1,17 @@
 // NeRF MLP (nerf/core/model.py:334-394): weight packing, the FP32 SIMT
 // forward (the plain path) and the precision dispatcher.
 //
-// FP32 SIMT forward: one CTA of 256 threads owns a 64-row tile. The tile's
-// activations stay in shared memory for all ten GEMM layers
+// FP32 SIMT forward: one CTA of 256 threads owns a 64-row tile, two CTAs per
+// SM. The tile's activations stay in shared memory for all ten GEMM layers
 // (X[64][320]: hidden state in columns 0..255, enc_xyz in 256..319, later
-// enc_dir in 256..287). Weights stream from L2 in K-chunks of 32 rows,
-// double-buffered with cp.async. Each thread accumulates an 8x8 register
-// block: 8 rows x (4 + 4) columns.
+// enc_dir in 256..287); the product and its tiling are fp32_tile.cuh's. 100,003
+// rows: 2.21 ms, 54 TFLOP/s (3.18 ms with one CTA per SM, scalar FMAs and
+// warps of 8 rows x 256 columns), the same outputs bit for bit.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
 #include "common.cuh"
+#include "fp32_tile.cuh"
 #include "mlp_internal.cuh"
 
 namespace nerfgb {
@@ -78,76 +79,8 @@ __global__ void fp8_scale_kernel(const float *__restrict__ flat, unsigned char *
 // ---------------------------------------------------------------------------
 // FP32 SIMT forward
 // ---------------------------------------------------------------------------
-constexpr int kTM = 64;    // rows per tile
-constexpr int kKC = 32;    // K rows per weight chunk
-constexpr int kXLD = 320;  // X row stride (floats)
-constexpr int kChunksPerTile = (64 + 256 * 4 + 320 + 256 * 3 + 288) / kKC;  // 77
-constexpr size_t kFp32Smem = (size_t)(kTM * kXLD + 2 * kKC * 256) * sizeof(float);
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
-
-// Chunk q of the per-tile sequence -> (layer, chunk-in-layer).
-__device__ __forceinline__ void chunk_of(int q, int &g, int &c) {
-  g = 0;
-  int base = 0;
-  while (true) {
-    int nch = gemm_kp(g) / kKC;
-    if (q < base + nch) break;
-    base += nch;
-    ++g;
-  }
-  c = q - base;
-}
-
-__device__ __forceinline__ void load_chunk(const float *__restrict__ W, float *dst, int q, int tid) {
-  int g, c;
-  chunk_of(q, g, c);
-  const int N = gemm_n(g);
-  const float *src = W + gemm_w_offset(g) + (long long)c * kKC * N;
-  const int pieces = kKC * N / 4;
-  for (int p = tid; p < pieces; p += 256) cp_async16(dst + 4 * p, src + 4 * p);
-}
-
-__device__ __forceinline__ float f4c(const float4 &v, int k) {
-  return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
-}
-
-template <int NCH>
-__device__ __forceinline__ void fp32_chunk(const float *__restrict__ Xr, const float *__restrict__ Wc,
-                                           int tx, float (&acc)[8][8]) {
-  constexpr int N = 128 * NCH;
-#pragma unroll
-  for (int kk = 0; kk < kKC; kk += 4) {
-    float4 a[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4 *>(Xr + i * kXLD + kk);
-#pragma unroll
-    for (int kq = 0; kq < 4; ++kq) {
-      float4 b0 = *reinterpret_cast<const float4 *>(Wc + (kk + kq) * N + tx * 4);
-      float4 b1 = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (NCH == 2) b1 = *reinterpret_cast<const float4 *>(Wc + (kk + kq) * N + 128 + tx * 4);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float av = f4c(a[i], kq);
-        acc[i][0] = fmaf(av, b0.x, acc[i][0]);
-        acc[i][1] = fmaf(av, b0.y, acc[i][1]);
-        acc[i][2] = fmaf(av, b0.z, acc[i][2]);
-        acc[i][3] = fmaf(av, b0.w, acc[i][3]);
-        if (NCH == 2) {
-          acc[i][4] = fmaf(av, b1.x, acc[i][4]);
-          acc[i][5] = fmaf(av, b1.y, acc[i][5]);
-          acc[i][6] = fmaf(av, b1.z, acc[i][6]);
-          acc[i][7] = fmaf(av, b1.w, acc[i][7]);
-        }
-      }
-    }
-  }
-}
+using fp32::kTM;
+using fp32::kXLD;
 
 // Copies columns [c0, c0 + nc) of the tile's X rows to acts[row][off ..].
 __device__ __forceinline__ void store_cols(float *__restrict__ acts, long long row0, long long n, const float *X,
@@ -165,7 +98,7 @@ __device__ __forceinline__ void store_cols(float *__restrict__ acts, long long r
 // rm: optional row map (logical row k reads and writes physical row
 // rm.map[k]) and device row count; not used with STORE.
 template <bool STORE>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(fp32::kThreads, 2)
     mlp_fp32_kernel(const float *__restrict__ pk, const float *__restrict__ xyz,
                     const float *__restrict__ dirs, long long n_max, int rpd, float *__restrict__ rgb,
                     float *__restrict__ sigma, float *__restrict__ acts, RowMap rm) {
@@ -173,18 +106,18 @@ __global__ void __launch_bounds__(256, 1)
   float *X = sm;
   float *Wb = sm + kTM * kXLD;
   const float *table = pk + kFp32TableOff;
-  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  const int tid = threadIdx.x;
+  const fp32::Place p256(tid, 256), p128(tid, 128);
   const long long n = rm.n_dev ? min((long long)*rm.n_dev, n_max) : n_max;
   const long long ntiles = (n + kTM - 1) / kTM;
   auto phys = [&](long long k) -> long long {
     return rm.map ? (long long)NG_IDX(rm.map[k], n_max, kSiteMlpRowMapFp32) : k;
   };
+  int buf = 0;
+  if ((long long)blockIdx.x < ntiles) fp32::load_chunk<256>(pk, Wb, tid);  // the first weight chunk
 
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long row0 = tile * kTM;
-    // First weight chunk of the tile.
-    load_chunk(pk, Wb, 0, tid);
-    cp_async_commit();
     // enc_xyz -> X[:, 256..319] (model.py:319-331), column 319 = 0.
     for (int e = tid; e < kTM * 33; e += 256) {
       int r = e / 33, j = e - r * 33;
@@ -205,36 +138,27 @@ __global__ void __launch_bounds__(256, 1)
     }
     if (tid < kTM) X[tid * kXLD + 319] = 0.0f;
 
-    int q = 0;
     for (int g = 0; g < kNumGemm; ++g) {
       const int N = gemm_n(g);
-      const int nch = gemm_kp(g) / kKC;
       const int kin = (g == 0) ? 256 : 0;
+      // the chunk that follows this layer's last: the next layer's (the next tile's) first
+      const bool more = g + 1 < kNumGemm || tile + gridDim.x < ntiles;
+      const int gn = g + 1 < kNumGemm ? g + 1 : 0;
+      const float *W = pk + gemm_w_offset(g), *Wn = pk + gemm_w_offset(gn);
+      const int next_n = more ? gemm_n(gn) : 0;
       float acc[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-      for (int c = 0; c < nch; ++c, ++q) {
-        if (q + 1 < kChunksPerTile) load_chunk(pk, Wb + ((q + 1) & 1) * kKC * 256, q + 1, tid);
-        cp_async_commit();
-        cp_async_wait1();
-        __syncthreads();
-        const float *Xr = X + (ty * 8) * kXLD + kin + c * kKC;
-        const float *Wc = Wb + (q & 1) * kKC * 256;
-        if (N == 256)
-          fp32_chunk<2>(Xr, Wc, tx, acc);
-        else
-          fp32_chunk<1>(Xr, Wc, tx, acc);
-        __syncthreads();
-      }
+      if (N == 256)
+        fp32::layer<256>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p256, acc);
+      else
+        fp32::layer<128>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p128, acc);
       // Epilogue: bias (+ReLU) into X[:, 0..N).
+      const fp32::Place &pl = N == 256 ? p256 : p128;
       const float *bias = table + bias_offset(g);
       const bool relu = gemm_relu(g);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (h == 1 && N != 256) break;
-        int col = h * 128 + tx * 4;
+        const int col = pl.col(h);
         float4 bv = *reinterpret_cast<const float4 *>(bias + col);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -246,7 +170,7 @@ __global__ void __launch_bounds__(256, 1)
             v.z = fmaxf(v.z, 0.f);
             v.w = fmaxf(v.w, 0.f);
           }
-          *reinterpret_cast<float4 *>(X + (ty * 8 + i) * kXLD + col) = v;
+          *reinterpret_cast<float4 *>(X + pl.row(i) * kXLD + col) = v;
         }
       }
       if (g == 8) {
@@ -330,28 +254,28 @@ extern "C" int nerfgb_mlp_pack(const float *params, int precision, void *packed,
 namespace nerfgb {
 int launch_mlp_fp32(const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
                     float *rgb, float *sigma, cudaStream_t stream, const RowMap &rm) {
-  if (cudaFuncSetAttribute(mlp_fp32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFp32Smem) !=
+  if (cudaFuncSetAttribute(mlp_fp32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) !=
       cudaSuccess)
     return NERFGB_E_CUDA;
   long long ntiles = (n + kTM - 1) / kTM;
   int sms = num_sms();
   if (sms <= 0) return NERFGB_E_DEVICE;
-  int grid = (int)(ntiles < sms ? ntiles : sms);
-  mlp_fp32_kernel<false><<<grid, 256, kFp32Smem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs,
+  const int grid = (int)(ntiles < 2 * sms ? ntiles : 2 * sms);  // two CTAs per SM
+  mlp_fp32_kernel<false><<<grid, 256, fp32::kSmem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs,
                                                             n, rpd, rgb, sigma, nullptr, rm);
   return launch_status();
 }
 
 int launch_mlp_fp32_store(const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
                           float *rgb, float *sigma, float *acts, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(mlp_fp32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFp32Smem) !=
+  if (cudaFuncSetAttribute(mlp_fp32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) !=
       cudaSuccess)
     return NERFGB_E_CUDA;
   long long ntiles = (n + kTM - 1) / kTM;
   int sms = num_sms();
   if (sms <= 0) return NERFGB_E_DEVICE;
-  int grid = (int)(ntiles < sms ? ntiles : sms);
-  mlp_fp32_kernel<true><<<grid, 256, kFp32Smem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs, n,
+  const int grid = (int)(ntiles < 2 * sms ? ntiles : 2 * sms);
+  mlp_fp32_kernel<true><<<grid, 256, fp32::kSmem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs, n,
                                                            rpd, rgb, sigma, acts, RowMap());
   return launch_status();
 }
