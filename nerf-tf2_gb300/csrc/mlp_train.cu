@@ -3,22 +3,27 @@
 // weights.
 //
 // The forward (mlp.cu, STORE variant) writes every layer's post-activation
-// rows to `acts` (kActsLd floats per row). The backward then runs layer by
-// layer from the heads down:
+// rows to `acts` (kActsLd floats per row). The backward takes the rows in
+// chunks of kChunkRows; per chunk
 //   head kernel   rgb = sigmoid(h9 Wr + br), sigma = ReLU(h7 ws + bs):
 //                 dZ9 = (dpre_rgb Wr^T) * [h9 > 0], dpre_sigma, head grads
-//   dW kernel     dW[k][n] += sum_m In[m][k] dZ[m][n]  (split over m, atomics)
-//   dX kernel     dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
+//   chain kernel  for every layer from dense_9 down, a tile of rows staying
+//                 in shared memory:
+//                 dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
 //                                 * [h_prev[m][k] > 0]
+//   dW kernel     for every layer: dW[k][n] += sum_m In[m][k] dZ[m][n]
 // Gradients land in the flat Keras layout of the parameter blob.
 #include "common.cuh"
+#include "fp32_tile.cuh"
 #include "mlp_internal.cuh"
 
 namespace nerfgb {
 namespace train {
 
-constexpr int kTM = 64;
 constexpr int kDzLd = 256;  // row stride of the dZ buffers
+// Rows per chunk: the workspace holds every layer's dZ of one chunk (four
+// 64-row tiles per CTA of the chain kernel, two CTAs per SM, 152 SMs).
+constexpr long long kChunkRows = 4LL * 2 * 152 * 64;
 
 // ---------------------------------------------------------------------------
 // Heads
@@ -172,164 +177,199 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
 }
 
 // ---------------------------------------------------------------------------
-// dX: dz_out[m][k] = (sum_n dz_in[m][n] W[k][n] + dsp[m] ws[k]) * mask, k < 256
+// Chain
 // ---------------------------------------------------------------------------
-constexpr int kNC = 32;
-constexpr size_t kDxSmem = (size_t)(kTM * (kNC + 4) + kNC * (256 + 4)) * sizeof(float);
+// Transposed weights of GEMM layer g >= 1, [n][k < 256], for the chain.
+__host__ __device__ constexpr long long wt_offset(int g) {
+  long long off = 0;
+  for (int i = 1; i < g; ++i) off += (long long)gemm_n(i) * 256;
+  return off;
+}
+constexpr long long kWtElems = wt_offset(kNumGemm);
 
-__global__ void __launch_bounds__(256)
-    dx_kernel(const float *__restrict__ W, int N, const float *__restrict__ dz_in, long long n,
-              const float *__restrict__ dsp, const float *__restrict__ ws, const float *__restrict__ acts, int mask_off,
-              float *__restrict__ dz_out) {
+__global__ void transpose_kernel(const float *__restrict__ W, float *__restrict__ wt) {
+  __shared__ float t[32][33];
+  const int g = blockIdx.z + 1, N = gemm_n(g), n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  if (n0 >= N) return;
+  const float *src = W + gemm_w_offset(g);
+  for (int i = threadIdx.y; i < 32; i += 8) t[i][threadIdx.x] = src[(long long)(k0 + i) * N + n0 + threadIdx.x];
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += 8) wt[wt_offset(g) + (long long)(n0 + i) * 256 + k0 + threadIdx.x] = t[threadIdx.x][i];
+}
+
+// dz [10][rows][kDzLd]: dz[9] (128 columns, from the heads) in, dz[8] .. dz[0]
+// out. The layers' products are the forward's (fp32_tile.cuh: X the tile's
+// dZ, the transposed weights streamed); every output is one chain of FMAs
+// over n in order. Taking the layers one kernel at a time re-read and
+// re-staged dZ and gathered W transposed for every 64-row tile (8.4 ms of a
+// 1,024-ray step's two networks, against 5.5 here).
+__global__ void __launch_bounds__(fp32::kThreads, 2)
+    chain_kernel(const float *__restrict__ wt, const float *__restrict__ table, const float *__restrict__ acts,
+                 long long n, const float *__restrict__ dsp, float *__restrict__ dz) {
+  using fp32::kTM;
+  using fp32::kXLD;
   extern __shared__ __align__(16) float sm[];
-  float *sA = sm;                      // [kTM][kNC + 4]
-  float *sB = sm + kTM * (kNC + 4);    // [kNC][256 + 4]: sB[nn][k] = W[k][n0 + nn]
-  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  float *X = sm, *Wb = sm + kTM * kXLD;
+  const int tid = threadIdx.x;
+  const fp32::Place pl(tid, 256);
   const long long ntiles = (n + kTM - 1) / kTM;
+  int buf = 0;
+  if ((long long)blockIdx.x < ntiles) fp32::load_chunk<256>(wt + wt_offset(9), Wb, tid);
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const long long row0 = tile * kTM;
-    float acc[8][8];
+    for (int e = tid; e < kTM * 32; e += fp32::kThreads) {
+      const int r = e >> 5, q = e & 31;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row0 + r < n) v = *reinterpret_cast<const float4 *>(dz + (9 * n + row0 + r) * kDzLd + 4 * q);
+      *reinterpret_cast<float4 *>(X + r * kXLD + 4 * q) = v;
+    }
+#pragma unroll 1
+    for (int g = 9; g >= 1; --g) {
+      const bool more = g > 1 || tile + gridDim.x < ntiles;
+      float acc[8][8];
+      fp32::layer<256>(X, Wb, buf, wt + wt_offset(g), gemm_n(g), 0, wt + wt_offset(g > 1 ? g - 1 : 9), more ? 256 : 0,
+                       tid, pl, acc);
+      // dense_9's input, the bottleneck, is linear: no mask; dense_8's input h7 also feeds the sigma head
+      const int mask_off = g == 9 ? -1 : acts_offset(g - 1);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) {
+        const long long m = row0 + pl.row(i);
+        const bool valid = m < n;
+        const float ds = g == 8 && valid ? dsp[m] : 0.0f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-    for (int n0 = 0; n0 < N; n0 += kNC) {
-      __syncthreads();
-      for (int e = tid; e < kTM * (kNC / 4); e += 256) {
-        const int r = e / (kNC / 4), q = e % (kNC / 4);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row0 + r < n) v = *reinterpret_cast<const float4 *>(dz_in + (row0 + r) * kDzLd + n0 + 4 * q);
-        *reinterpret_cast<float4 *>(sA + r * (kNC + 4) + 4 * q) = v;
-      }
-      {
-        const int k = tid;  // one W row per thread
-#pragma unroll
-        for (int q = 0; q < kNC / 4; ++q) {
-          const float4 v = *reinterpret_cast<const float4 *>(W + (long long)k * N + n0 + 4 * q);
-          sB[(4 * q) * (256 + 4) + k] = v.x;
-          sB[(4 * q + 1) * (256 + 4) + k] = v.y;
-          sB[(4 * q + 2) * (256 + 4) + k] = v.z;
-          sB[(4 * q + 3) * (256 + 4) + k] = v.w;
-        }
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int nn = 0; nn < kNC; ++nn) {
-        float a[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = sA[(ty * 8 + i) * (kNC + 4) + nn];
-        const float4 b0 = *reinterpret_cast<const float4 *>(sB + nn * (256 + 4) + tx * 4);
-        const float4 b1 = *reinterpret_cast<const float4 *>(sB + nn * (256 + 4) + 128 + tx * 4);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          acc[i][0] = fmaf(a[i], b0.x, acc[i][0]);
-          acc[i][1] = fmaf(a[i], b0.y, acc[i][1]);
-          acc[i][2] = fmaf(a[i], b0.z, acc[i][2]);
-          acc[i][3] = fmaf(a[i], b0.w, acc[i][3]);
-          acc[i][4] = fmaf(a[i], b1.x, acc[i][4]);
-          acc[i][5] = fmaf(a[i], b1.y, acc[i][5]);
-          acc[i][6] = fmaf(a[i], b1.z, acc[i][6]);
-          acc[i][7] = fmaf(a[i], b1.w, acc[i][7]);
+        for (int h = 0; h < 2; ++h) {
+          const int k = pl.col(h);
+          float4 v = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+          if (g == 8) {
+            const float4 ws = *reinterpret_cast<const float4 *>(table + kSigmaWOff + k);
+            v.x = fmaf(ds, ws.x, v.x);
+            v.y = fmaf(ds, ws.y, v.y);
+            v.z = fmaf(ds, ws.z, v.z);
+            v.w = fmaf(ds, ws.w, v.w);
+          }
+          if (mask_off >= 0 && valid) {
+            const float4 hm = *reinterpret_cast<const float4 *>(acts + m * kActsLd + mask_off + k);
+            v.x = hm.x > 0.0f ? v.x : 0.0f;
+            v.y = hm.y > 0.0f ? v.y : 0.0f;
+            v.z = hm.z > 0.0f ? v.z : 0.0f;
+            v.w = hm.w > 0.0f ? v.w : 0.0f;
+          }
+          *reinterpret_cast<float4 *>(X + pl.row(i) * kXLD + k) = v;
+          if (valid) *reinterpret_cast<float4 *>(dz + ((g - 1) * n + m) * kDzLd + k) = v;
         }
       }
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const long long m = row0 + ty * 8 + i;
-      if (m >= n) continue;
-      const float ds = dsp ? dsp[m] : 0.0f;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int k = h * 128 + tx * 4;
-        float4 v = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
-        if (dsp) {
-          v.x = fmaf(ds, ws[k], v.x);
-          v.y = fmaf(ds, ws[k + 1], v.y);
-          v.z = fmaf(ds, ws[k + 2], v.z);
-          v.w = fmaf(ds, ws[k + 3], v.w);
-        }
-        if (mask_off >= 0) {
-          const float4 hm = *reinterpret_cast<const float4 *>(acts + m * kActsLd + mask_off + k);
-          v.x = hm.x > 0.0f ? v.x : 0.0f;
-          v.y = hm.y > 0.0f ? v.y : 0.0f;
-          v.z = hm.z > 0.0f ? v.z : 0.0f;
-          v.w = hm.w > 0.0f ? v.w : 0.0f;
-        }
-        *reinterpret_cast<float4 *>(dz_out + m * kDzLd + k) = v;
-      }
-    }
+    __syncthreads();  // X is rewritten
   }
 }
 
 // ---------------------------------------------------------------------------
 // dW: dW[(k_dst0 + k) * out + n] += sum_m In[m][k] dZ[m][n]; db[n] += sum dZ.
-// grid (N/64, ceil(K/64), m-slices); 4x4 outputs per thread.
 // ---------------------------------------------------------------------------
-constexpr int kMC = 32;
-constexpr long long kMSlice = 8192;
+// All layers in one launch: grid (128 x 128 tiles of all the jobs, m-slices).
+// A thread holds 8 x 8 outputs as paired FMAs along n (fp32_tile.cuh gives
+// the reason); the rows stream through two 16-row stages of cp.async. A 4 x 4
+// tile per thread with guarded 4-byte loads was bound by its loads: 33 of the
+// 39 ms of a 1,024-ray step, 6.2 of 17.6 here.
+constexpr int kMC = 16, kTN = 128;
 
-__global__ void __launch_bounds__(256)
-    dw_kernel(const float *__restrict__ acts, int in_off, int K, const float *__restrict__ dz, int N, long long n,
-              float *__restrict__ dW, int out, int k_dst0, float *__restrict__ db) {
-  __shared__ __align__(16) float sA[kMC][64 + 4];
-  __shared__ __align__(16) float sB[kMC][64 + 4];
+struct DwJob {
+  int in_off, K, slot, flat, k_dst0;  // tape columns, dZ buffer, destination layer and rows
+};
+constexpr int kJobs = 12;
+__host__ __device__ constexpr DwJob dw_job(int j) {
+  return j == 0   ? DwJob{acts_offset(8), 256, 9, 10, 0}
+         : j == 1 ? DwJob{kActsEncDir, 27, 9, 10, 256}
+         : j == 2 ? DwJob{acts_offset(7), 256, 8, 9, 0}
+         : j == 3 ? DwJob{kActsEncXyz, 63, 5, 5, 256}
+         : j == 4 ? DwJob{kActsEncXyz, 63, 0, 0, 0}
+                  : DwJob{acts_offset(j - 5), 256, j - 4, j - 4, 0};  // dense_1 .. dense_7
+}
+__host__ __device__ constexpr int dw_tiles(int j) {
+  return ((dw_job(j).K + kTN - 1) / kTN) * (flat_out(dw_job(j).flat) / kTN);
+}
+__host__ __device__ constexpr int dw_first(int j) {
+  int t = 0;
+  for (int i = 0; i < j; ++i) t += dw_tiles(i);
+  return t;
+}
+constexpr int kDwTiles = dw_first(kJobs);
+static_assert(kActsEncDir + kTN <= kActsLd, "a tile's columns stay inside the row");
+
+__device__ __forceinline__ void cp_async16z(float *smem, const float *gmem, bool valid) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(valid ? 16u : 0u));
+}
+
+__global__ void __launch_bounds__(256, 2)
+    dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, long long n, long long slice,
+              float *__restrict__ grads) {
+  __shared__ __align__(16) float sA[2][kMC][kTN];
+  __shared__ __align__(16) float sB[2][kMC][kTN];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int n0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
-  const long long m_begin = (long long)blockIdx.z * kMSlice;
-  const long long m_end = m_begin + kMSlice < n ? m_begin + kMSlice : n;
-  float acc[4][4];
+  int j = 0;
+  while (j + 1 < kJobs && (int)blockIdx.x >= dw_first(j + 1)) ++j;
+  const DwJob job = dw_job(j);
+  const int N = flat_out(job.flat), t = blockIdx.x - dw_first(j), ntn = N / kTN;
+  const int n0 = (t % ntn) * kTN, k0 = (t / ntn) * kTN;
+  const long long m_begin = blockIdx.y * slice, m_end = m_begin + slice < n ? m_begin + slice : n;
+  const float *A = acts + job.in_off + k0, *B = dz + job.slot * n * kDzLd + n0;
+  auto load = [&](long long m0, int st) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  float bacc[4] = {0.f, 0.f, 0.f, 0.f};
-  const bool do_bias = db && blockIdx.y == 0 && ty == 0;
-  for (long long m0 = m_begin; m0 < m_end; m0 += kMC) {
-    __syncthreads();
-    for (int e = tid; e < kMC * 64; e += 256) {
-      const int mm = e >> 6, c = e & 63;
-      const long long m = m0 + mm;
-      sA[mm][c] = (m < m_end && k0 + c < K) ? acts[m * kActsLd + in_off + k0 + c] : 0.0f;
-      sB[mm][c] = (m < m_end && n0 + c < N) ? dz[m * kDzLd + n0 + c] : 0.0f;
+    for (int p = tid; p < kMC * kTN / 4; p += 256) {
+      const int mm = p / (kTN / 4), q = p % (kTN / 4);
+      const bool v = m0 + mm < m_end;
+      const long long m = v ? m0 + mm : m_begin;
+      cp_async16z(&sA[st][mm][4 * q], A + m * kActsLd + 4 * q, v);
+      cp_async16z(&sB[st][mm][4 * q], B + m * kDzLd + 4 * q, v);
     }
-    __syncthreads();
-#pragma unroll 8
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[i][q] = 0.0f;
+  float bacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const bool do_bias = job.k_dst0 == 0 && k0 == 0 && tid < 32;  // a warp holding the tile's columns (twice)
+  load(m_begin, 0);
+  int st = 0;
+#pragma unroll 1
+  for (long long m0 = m_begin; m0 < m_end; m0 += kMC, st ^= 1) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // the stage is there, the other one used up
+    if (m0 + kMC < m_end) load(m0 + kMC, st ^ 1);
+#pragma unroll
     for (int mm = 0; mm < kMC; ++mm) {
-      const float4 a = *reinterpret_cast<const float4 *>(&sA[mm][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4 *>(&sB[mm][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+      float a[8], b[8];
+      *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(&sA[st][mm][4 * ty]);
+      *reinterpret_cast<float4 *>(a + 4) = *reinterpret_cast<const float4 *>(&sA[st][mm][64 + 4 * ty]);
+      *reinterpret_cast<float4 *>(b) = *reinterpret_cast<const float4 *>(&sB[st][mm][4 * tx]);
+      *reinterpret_cast<float4 *>(b + 4) = *reinterpret_cast<const float4 *>(&sB[st][mm][64 + 4 * tx]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        for (int q = 0; q < 8; q += 2)
+          fma_f32x2(acc[i][q], acc[i][q + 1], a[i], a[i], b[q], b[q + 1], acc[i][q], acc[i][q + 1]);
       if (do_bias) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) bacc[j] += bv[j];
+        for (int q = 0; q < 8; ++q) bacc[q] += b[q];
       }
     }
   }
+  float *dW = grads + flat_offset(job.flat), *db = dW + (long long)flat_in(job.flat) * N;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int k = k0 + ty * 4 + i;
-    if (k >= K) continue;
+  for (int i = 0; i < 8; ++i) {
+    const int k = k0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
+    if (k >= job.K) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int nn = n0 + tx * 4 + j;
-      if (nn < N) atomicAdd(dW + (long long)(k_dst0 + k) * out + nn, acc[i][j]);
-    }
+    for (int q = 0; q < 8; ++q)
+      atomicAdd(dW + (long long)(job.k_dst0 + k) * N + n0 + (q < 4 ? 4 * tx + q : 64 + 4 * tx + q - 4), acc[i][q]);
   }
-  if (do_bias) {
+  if (do_bias && ty == 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (n0 + tx * 4 + j < N) atomicAdd(db + n0 + tx * 4 + j, bacc[j]);
+    for (int q = 0; q < 8; ++q) atomicAdd(db + n0 + (q < 4 ? 4 * tx + q : 64 + 4 * tx + q - 4), bacc[q]);
   }
-}
-
-static int persistent_grid(long long n) {
-  const long long tiles = (n + kTM - 1) / kTM;
-  const int sms = num_sms();
-  const long long cap = (long long)(sms > 0 ? sms : 148) * 2;
-  return (int)(tiles < cap ? tiles : cap);
 }
 
 }  // namespace train
@@ -360,23 +400,19 @@ int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const
 
 namespace train {
 
-static int launch_dw(const float *acts, int in_off, int K, const float *dz, int N, long long n, float *grads,
-                     int flat_layer, int k_dst0, bool bias, cudaStream_t st) {
-  const int out = flat_out(flat_layer);
-  float *dW = grads + flat_offset(flat_layer);
-  float *db = bias ? dW + (long long)flat_in(flat_layer) * out : nullptr;
-  dim3 grid((N + 63) / 64, (K + 63) / 64, (unsigned)((n + kMSlice - 1) / kMSlice));
-  dw_kernel<<<grid, 256, 0, st>>>(acts, in_off, K, dz, N, n, dW, out, k_dst0, db);
-  return launch_status();
-}
-
-static int launch_dx(const float *table_base_W, int g, const float *dz_in, long long n, const float *dsp,
-                     const float *ws, const float *acts, int mask_off, float *dz_out, cudaStream_t st) {
-  if (cudaFuncSetAttribute(dx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDxSmem) != cudaSuccess)
-    return NERFGB_E_CUDA;
-  dx_kernel<<<persistent_grid(n), 256, kDxSmem, st>>>(table_base_W + gemm_w_offset(g), gemm_n(g), dz_in, n, dsp,
-                                                      ws, acts, mask_off, dz_out);
-  return launch_status();
+struct Ws {
+  float *wt, *dsp, *dz;
+  long long rows, bytes;
+};
+static Ws carve(void *base, long long n) {
+  Ws w{};
+  float *p = reinterpret_cast<float *>(base);
+  w.rows = n < kChunkRows ? n : kChunkRows;
+  w.wt = p;
+  w.dz = p + kWtElems;
+  w.dsp = w.dz + kNumGemm * w.rows * kDzLd;
+  w.bytes = (kWtElems + w.rows * (kNumGemm * kDzLd + 1)) * (long long)sizeof(float);
+  return w;
 }
 
 }  // namespace train
@@ -388,7 +424,7 @@ extern "C" long long nerfgb_mlp_acts_floats_per_row(void) { return kActsLd; }
 
 extern "C" long long nerfgb_mlp_backward_workspace_bytes(long long n_rows) {
   if (n_rows < 0) return -1;
-  return (2 * n_rows * train::kDzLd + n_rows) * (long long)sizeof(float);
+  return train::carve(nullptr, n_rows).bytes;
 }
 
 extern "C" int nerfgb_mlp_forward_train(const void *packed, const float *xyz, const float *dirs, long long n_rows,
@@ -409,43 +445,32 @@ extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long l
       !aligned(workspace, 16))
     return NERFGB_E_INVALID_ARG;
   cudaStream_t st = as_stream(stream);
-  const long long n = n_rows;
   const float *W = reinterpret_cast<const float *>(packed);  // FP32 pack: padded [Kp][N] blocks
   const float *table = W + kFp32TableOff;
-  float *bufA = reinterpret_cast<float *>(workspace);
-  float *bufB = bufA + n * kDzLd;
-  float *dsp = bufB + n * kDzLd;
+  const Ws w = carve(workspace, n_rows);
+  const int sms = num_sms();
+  if (sms <= 0) return NERFGB_E_DEVICE;
+  if (cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) != cudaSuccess)
+    return NERFGB_E_CUDA;
+  transpose_kernel<<<dim3(8, 8, kNumGemm - 1), dim3(32, 8), 0, st>>>(W, w.wt);
   int rc;
-  if ((rc = launch_head_bwd(table, acts, n, d_rgb, d_sigma, bufA, dsp, grad_params, st)) != NERFGB_OK) return rc;
-  // dense_9 (flat 10): input [bottleneck | enc_dir], output 128.
-  if ((rc = launch_dw(acts, acts_offset(8), 256, bufA, 128, n, grad_params, 10, 0, true, st)) != NERFGB_OK) return rc;
-  if ((rc = launch_dw(acts, kActsEncDir, 27, bufA, 128, n, grad_params, 10, 256, false, st)) != NERFGB_OK) return rc;
-  // dBottleneck = dZ9 W9[0:256]^T (dense_8 is linear: no mask).
-  if ((rc = launch_dx(W, 9, bufA, n, nullptr, nullptr, acts, -1, bufB, st)) != NERFGB_OK) return rc;
-  // dense_8 (flat 9): input h7.
-  if ((rc = launch_dw(acts, acts_offset(7), 256, bufB, 256, n, grad_params, 9, 0, true, st)) != NERFGB_OK) return rc;
-  // dZ7 = (dBott W8^T + dpre_sigma ws) * [h7 > 0]
-  if ((rc = launch_dx(W, 8, bufB, n, dsp, table + kSigmaWOff, acts, acts_offset(7), bufA, st)) != NERFGB_OK)
-    return rc;
-  float *cur = bufA, *nxt = bufB;
-  for (int l = 7; l >= 0; --l) {
-    if (l == 0) {
-      if ((rc = launch_dw(acts, kActsEncXyz, 63, cur, 256, n, grad_params, 0, 0, true, st)) != NERFGB_OK) return rc;
-      break;
-    }
-    if (l == 5) {
-      if ((rc = launch_dw(acts, acts_offset(4), 256, cur, 256, n, grad_params, 5, 0, true, st)) != NERFGB_OK)
-        return rc;
-      if ((rc = launch_dw(acts, kActsEncXyz, 63, cur, 256, n, grad_params, 5, 256, false, st)) != NERFGB_OK)
-        return rc;
-    } else {
-      if ((rc = launch_dw(acts, acts_offset(l - 1), 256, cur, 256, n, grad_params, l, 0, true, st)) != NERFGB_OK)
-        return rc;
-    }
-    if ((rc = launch_dx(W, l, cur, n, nullptr, nullptr, acts, acts_offset(l - 1), nxt, st)) != NERFGB_OK) return rc;
-    float *t = cur;
-    cur = nxt;
-    nxt = t;
+  if ((rc = launch_status()) != NERFGB_OK) return rc;
+  for (long long r0 = 0; r0 < n_rows; r0 += kChunkRows) {
+    const long long n = n_rows - r0 < kChunkRows ? n_rows - r0 : kChunkRows;
+    const float *a = acts + r0 * kActsLd;
+    if ((rc = launch_head_bwd(table, a, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * kDzLd,
+                              w.dsp, grad_params, st)) != NERFGB_OK)
+      return rc;
+    const long long tiles = (n + fp32::kTM - 1) / fp32::kTM;
+    chain_kernel<<<(unsigned)(tiles < 2 * sms ? tiles : 2 * sms), fp32::kThreads, fp32::kSmem, st>>>(w.wt, table, a, n,
+                                                                                                w.dsp, w.dz);
+    if ((rc = launch_status()) != NERFGB_OK) return rc;
+    // slices of at least 256 rows, enough of them for eight waves of two CTAs per SM
+    const long long want = (16LL * sms + kDwTiles - 1) / kDwTiles, most = (n + 255) / 256;
+    const long long slices = want < most ? want : most;
+    const long long slice = ((n + slices - 1) / slices + kMC - 1) / kMC * kMC;
+    dw_kernel<<<dim3(kDwTiles, (unsigned)((n + slice - 1) / slice)), 256, 0, st>>>(a, w.dz, n, slice, grad_params);
+    if ((rc = launch_status()) != NERFGB_OK) return rc;
   }
   return NERFGB_OK;
 }
