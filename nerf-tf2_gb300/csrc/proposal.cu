@@ -13,11 +13,11 @@
 // Parameters (flat float32, 6,785 values): W1 [39,64], b1 [64], W2 [64,64],
 // b2 [64], W3 [64], b3 [1].
 //
-// Forward: one thread per sample, weights broadcast from shared memory.
-// Backward: recompute per 128-sample tile; per-sample vectors go to shared
-// memory (odd row strides, conflict-free), then each thread reduces its own
-// slice of dW over the tile in registers and adds it to the CTA's gradient
-// in shared memory; one atomicAdd per parameter per CTA at the end.
+// FP32 forward and backward: 128-sample tiles per CTA of 256 threads, every
+// step a small matrix product from shared memory (tile_product), vectors of a
+// tile stored [component][sample]. The weight gradients of a CTA stay in its
+// threads' registers over all of its tiles and are added to the blob at the
+// end, one atomicAdd per parameter per CTA.
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -31,79 +31,133 @@ namespace prop {
 constexpr int kIn = 39, kH = 64;
 constexpr int kW1 = 0, kB1 = kW1 + kIn * kH, kW2 = kB1 + kH, kB2 = kW2 + kH * kH, kW3 = kB2 + kH, kB3 = kW3 + kH;
 constexpr int kParams = kB3 + 1;  // 6785
-constexpr int kThreads = 128;
-constexpr int kEncLd = 41, kRowLd = 65;
-
-__device__ __forceinline__ void encode6(const float x[3], float enc[kIn]) {
-  enc[0] = x[0];
-  enc[1] = x[1];
-  enc[2] = x[2];
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int l = 0; l < 6; ++l) {
-      float s, co;
-      sincosf(fmul(x[c], enc_multiplier(l)), &s, &co);
-      enc[3 + c * 12 + 2 * l] = s;
-      enc[3 + c * 12 + 2 * l + 1] = co;
-    }
-}
+constexpr int kThreads = 256;
+constexpr int kTS = 128;          // samples per tile
+constexpr int kLdS = kTS + 4;     // row stride of the tile's [component][sample] arrays
 
 __device__ __forceinline__ float softplus(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
+
+// What bounds these kernels is the FP32 FMA pipe, given enough reuse: a
+// thread per sample with the weights broadcast from shared memory spent two
+// shared-memory wavefronts per four FMAs (262,144 samples: forward 127 us,
+// backward 634 us, against 99 and 256 here). A thread holds 8 samples x 4
+// outputs: samples 4*sg .. +3 and 64 + 4*sg .. +3 (sg = 4*(warp/2) + lane/8),
+// outputs 4*og .. +3 (og = 8*(warp%2) + lane%8). Tiles of 64 samples (4 x 4 per
+// thread, two CTAs per SM in the backward) ran 373 us together against 355.
+struct Place {
+  int s0, j0;
+  __device__ __forceinline__ explicit Place(int tid) {
+    const int warp = tid >> 5, lane = tid & 31;
+    s0 = 4 * ((warp >> 1) * 4 + (lane >> 3));
+    j0 = 4 * ((warp & 1) * 8 + (lane & 7));
+  }
+  __device__ __forceinline__ int sample(int i) const { return s0 + (i & 3) + (i >> 2) * 64; }
+};
+
+// acc[i][j] += sum_k A[k][sample i] B[k][output j], k in order, paired FMAs
+// over adjacent outputs (each half rounded as fmaf).
+template <int K>
+__device__ __forceinline__ void tile_product(const float *A, const float *B, const Place &pl, float (&acc)[8][4]) {
+#pragma unroll 8
+  for (int k = 0; k < K; ++k) {
+    float a[8];
+    *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(A + k * kLdS + pl.s0);
+    *reinterpret_cast<float4 *>(a + 4) = *reinterpret_cast<const float4 *>(A + k * kLdS + 64 + pl.s0);
+    const float4 b = *reinterpret_cast<const float4 *>(B + k * kH + pl.j0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      fma_f32x2(acc[i][0], acc[i][1], a[i], a[i], b.x, b.y, acc[i][0], acc[i][1]);
+      fma_f32x2(acc[i][2], acc[i][3], a[i], a[i], b.z, b.w, acc[i][2], acc[i][3]);
+    }
+  }
+}
+// The thread's 8 x 4 values to dst [output][sample].
+__device__ __forceinline__ void store_tile(float *dst, const Place &pl, const float (&v)[8][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float *d = dst + (pl.j0 + j) * kLdS + pl.s0;
+    *reinterpret_cast<float4 *>(d) = make_float4(v[0][j], v[1][j], v[2][j], v[3][j]);
+    *reinterpret_cast<float4 *>(d + 64) = make_float4(v[4][j], v[5][j], v[6][j], v[7][j]);
+  }
+}
+
+// Tile of samples [i0, i0 + 128): the encodings into enc [39][kLdS], h1 =
+// ReLU(enc W1 + b1) into h1 [64][kLdS], and this thread's z2 = h1 W2 + b2 in
+// z2. sw: the parameters. All threads; h1 is complete on return (and enc).
+__device__ __forceinline__ void hidden_tile(const float *sw, const float *__restrict__ xyz, long long i0, long long n,
+                                            float *enc, float *h1, const Place &pl, float (&z2)[8][4]) {
+  for (int e = threadIdx.x; e < kTS * 21; e += kThreads) {
+    const int q = e / kTS, sidx = e % kTS;
+    const int c = q < 3 ? q : (q - 3) / 6, l = (q - 3) % 6;
+    const float x = i0 + sidx < n ? xyz[3 * (i0 + sidx) + c] : 0.0f;
+    if (q < 3) {
+      enc[c * kLdS + sidx] = x;
+    } else {
+      float sn, cs;
+      sincosf(fmul(x, enc_multiplier(l)), &sn, &cs);
+      enc[(3 + c * 12 + 2 * l) * kLdS + sidx] = sn;
+      enc[(3 + c * 12 + 2 * l + 1) * kLdS + sidx] = cs;
+    }
+  }
+  __syncthreads();
+  float acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = sw[kB1 + pl.j0 + j];
+  tile_product<kIn>(enc, sw + kW1, pl, acc);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[i][j] = fmaxf(acc[i][j], 0.0f);
+      z2[i][j] = sw[kB2 + pl.j0 + j];
+    }
+  store_tile(h1, pl, acc);
+  __syncthreads();
+  tile_product<kH>(h1, sw + kW2, pl, z2);
+}
+
+// z3 = b3 + relu(z2) . W3 of one sample from h2 = ReLU(z2) [64][kLdS], in order.
+__device__ __forceinline__ float head(const float *sw, const float *h2, int sidx) {
+  float z3 = sw[kB3];
+#pragma unroll 16
+  for (int j = 0; j < kH; ++j) z3 = fmaf(h2[j * kLdS + sidx], sw[kW3 + j], z3);
+  return z3;
+}
 
 __device__ __forceinline__ void load_params(const float *__restrict__ p, float *sw) {
   for (int i = threadIdx.x; i < kParams; i += blockDim.x) sw[i] = p[i];
 }
 
-// h1 = ReLU(enc W1 + b1), z2 = h1 W2 + b2.
-__device__ __forceinline__ void hidden(const float *sw, const float enc[kIn], float h1[kH], float z2[kH]) {
-#pragma unroll
-  for (int j = 0; j < kH; ++j) h1[j] = sw[kB1 + j];
-#pragma unroll
-  for (int k = 0; k < kIn; ++k) {
-    const float e = enc[k];
-#pragma unroll
-    for (int j = 0; j < kH; j += 4) {
-      const float4 w = *reinterpret_cast<const float4 *>(sw + kW1 + k * kH + j);
-      h1[j] = fmaf(e, w.x, h1[j]);
-      h1[j + 1] = fmaf(e, w.y, h1[j + 1]);
-      h1[j + 2] = fmaf(e, w.z, h1[j + 2]);
-      h1[j + 3] = fmaf(e, w.w, h1[j + 3]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < kH; ++j) h1[j] = fmaxf(h1[j], 0.0f);
-#pragma unroll
-  for (int j = 0; j < kH; ++j) z2[j] = sw[kB2 + j];
-#pragma unroll 4
-  for (int k = 0; k < kH; ++k) {
-    const float h = h1[k];
-#pragma unroll
-    for (int j = 0; j < kH; j += 4) {
-      const float4 w = *reinterpret_cast<const float4 *>(sw + kW2 + k * kH + j);
-      z2[j] = fmaf(h, w.x, z2[j]);
-      z2[j + 1] = fmaf(h, w.y, z2[j + 1]);
-      z2[j + 2] = fmaf(h, w.z, z2[j + 2]);
-      z2[j + 3] = fmaf(h, w.w, z2[j + 3]);
-    }
-  }
-}
+constexpr int kParamsPad = (kParams + 3) / 4 * 4;
+constexpr size_t kFwdSmem = (size_t)(kParamsPad + kIn * kLdS + kH * kLdS) * sizeof(float);  // two CTAs per SM
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
     prop_fwd_kernel(const float *__restrict__ params, const float *__restrict__ xyz, long long n,
                     float *__restrict__ sigma) {
-  __shared__ __align__(16) float sw[kParams + 3];
+  extern __shared__ __align__(16) float sm[];
+  float *sw = sm, *enc = sm + kParamsPad, *h1 = enc + kIn * kLdS;
+  const Place pl(threadIdx.x);
   load_params(params, sw);
   __syncthreads();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    float x[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
-    float enc[kIn], h1[kH], z2[kH];
-    encode6(x, enc);
-    hidden(sw, enc, h1, z2);
-    float z3 = sw[kB3];
+  const long long ntiles = (n + kTS - 1) / kTS;
+  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    float z2[8][4];
+    hidden_tile(sw, xyz, tile * kTS, n, enc, h1, pl, z2);
+    __syncthreads();  // h1 is used up: h2 takes its place
 #pragma unroll
-    for (int j = 0; j < kH; ++j) z3 = fmaf(fmaxf(z2[j], 0.0f), sw[kW3 + j], z3);
-    sigma[i] = softplus(z3);
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z2[i][j] = fmaxf(z2[i][j], 0.0f);
+    store_tile(h1, pl, z2);
+    __syncthreads();
+    if (threadIdx.x < kTS) {
+      const long long i = tile * kTS + threadIdx.x;
+      const float z3 = head(sw, h1, threadIdx.x);
+      if (i < n) sigma[i] = softplus(z3);
+    }
+    __syncthreads();
   }
 }
 
@@ -369,115 +423,136 @@ __global__ void __launch_bounds__(32 * kFwdWarps)
 }
 
 constexpr size_t kBwdSmem =
-    (size_t)(2 * (kParams + 3) + kThreads * kEncLd + 4 * kThreads * kRowLd + kThreads) * sizeof(float);
+    (size_t)(kParamsPad + kH * kH + 48 * kLdS + 3 * kH * kLdS + kTS) * sizeof(float);
+
+// dW[r][c] of sum_s A[r][s] B[c][s] over the tile's samples: thread (tr, tc)
+// holds rows tr + 16 i, columns tc + 16 j, as sums over even and odd samples.
+template <int NR>
+__device__ __forceinline__ void outer_tile(const float *A, const float *B, int tr, int tc, float (&acc)[NR][4][2]) {
+#pragma unroll 4
+  for (int q = 0; q < kTS; q += 4) {
+    float4 b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(B + (tc + 16 * j) * kLdS + q);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      const float4 a = *reinterpret_cast<const float4 *>(A + (tr + 16 * i) * kLdS + q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float(&c)[2] = acc[i][j];
+        fma_f32x2(c[0], c[1], a.x, a.y, b[j].x, b[j].y, c[0], c[1]);
+        fma_f32x2(c[0], c[1], a.z, a.w, b[j].z, b[j].w, c[0], c[1]);
+      }
+    }
+  }
+}
 
 // grads += d/dparams sum_i dsigma_i * sigma_i.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     prop_bwd_kernel(const float *__restrict__ params, const float *__restrict__ xyz, const float *__restrict__ dsig,
                     long long n, float *__restrict__ grads) {
   extern __shared__ __align__(16) float sm[];
   float *sw = sm;
-  float *sacc = sw + kParams + 3;  // this CTA's gradient, one slice per thread
-  float *sENC = sacc + kParams + 3;
-  float *sH1 = sENC + kThreads * kEncLd;
-  float *sH2 = sH1 + kThreads * kRowLd;
-  float *sDZ2 = sH2 + kThreads * kRowLd;
-  float *sDZ1 = sDZ2 + kThreads * kRowLd;
-  float *sDZ3 = sDZ1 + kThreads * kRowLd;
-  const int tid = threadIdx.x, j = tid & 63, half = tid >> 6;
+  float *w2t = sw + kParamsPad;      // W2 transposed
+  float *enc = w2t + kH * kH;        // 39 rows (48 for the weight gradient's row tiles, the rest 0)
+  float *h1 = enc + 48 * kLdS;
+  float *dz2 = h1 + kH * kLdS;       // first h2
+  float *dz1 = dz2 + kH * kLdS;
+  float *dz3 = dz1 + kH * kLdS;
+  const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
+  const Place pl(tid);
   load_params(params, sw);
-  for (int q = tid; q < kParams; q += kThreads) sacc[q] = 0.0f;
+  for (int e = tid; e < (48 - kIn) * kLdS; e += kThreads) enc[kIn * kLdS + e] = 0.0f;
   __syncthreads();
-  const long long ntiles = (n + kThreads - 1) / kThreads;
+  for (int e = tid; e < kH * kH; e += kThreads) w2t[(e % kH) * kH + e / kH] = sw[kW2 + e];
+  float gw2[4][4][2] = {}, gw1[3][4][2] = {};
+  float gb1[4] = {}, gb2[4] = {}, gw3[4] = {}, gb3 = 0.0f;
+  const long long ntiles = (n + kTS - 1) / kTS;
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long i = tile * kThreads + tid;
-    const bool valid = i < n;
-    float x[3] = {0.f, 0.f, 0.f};
-    if (valid) {
-      x[0] = xyz[3 * i];
-      x[1] = xyz[3 * i + 1];
-      x[2] = xyz[3 * i + 2];
-    }
-    float enc[kIn], h1[kH], z2[kH];
-    encode6(x, enc);
-    hidden(sw, enc, h1, z2);
+    const long long i0 = tile * kTS;
+    float z2[8][4], v[8][4];
+    hidden_tile(sw, xyz, i0, n, enc, h1, pl, z2);
 #pragma unroll
-    for (int k = 0; k < kIn; ++k) sENC[tid * kEncLd + k] = enc[k];
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int k = 0; k < kH; ++k) sH1[tid * kRowLd + k] = h1[k];
-    float z3 = sw[kB3];
-#pragma unroll
-    for (int q = 0; q < kH; ++q) z3 = fmaf(fmaxf(z2[q], 0.0f), sw[kW3 + q], z3);
-    const float dz3 = valid ? dsig[i] / (1.0f + expf(-z3)) : 0.0f;  // softplus' = sigmoid
-    sDZ3[tid] = dz3;
-#pragma unroll
-    for (int q = 0; q < kH; ++q) {
-      sH2[tid * kRowLd + q] = fmaxf(z2[q], 0.0f);
-      z2[q] = z2[q] > 0.0f ? sw[kW3 + q] * dz3 : 0.0f;  // z2 now holds dz2
-      sDZ2[tid * kRowLd + q] = z2[q];
-    }
-    // dz1 = (W2 dz2) * [h1 > 0]
-#pragma unroll 4
-    for (int k = 0; k < kH; ++k) {
-      float acc = 0.0f;
-#pragma unroll
-      for (int q = 0; q < kH; q += 4) {
-        const float4 w = *reinterpret_cast<const float4 *>(sw + kW2 + k * kH + q);
-        acc = fmaf(w.x, z2[q], acc);
-        acc = fmaf(w.y, z2[q + 1], acc);
-        acc = fmaf(w.z, z2[q + 2], acc);
-        acc = fmaf(w.w, z2[q + 3], acc);
-      }
-      sDZ1[tid * kRowLd + k] = sH1[tid * kRowLd + k] > 0.0f ? acc : 0.0f;
+      for (int j = 0; j < 4; ++j) v[i][j] = fmaxf(z2[i][j], 0.0f);
+    store_tile(dz2, pl, v);
+    __syncthreads();
+    if (tid < kTS) {
+      const float z3 = head(sw, dz2, tid);
+      const float d = i0 + tid < n ? dsig[i0 + tid] / (1.0f + expf(-z3)) : 0.0f;  // softplus' = sigmoid
+      dz3[tid] = d;
+      gb3 += d;
     }
     __syncthreads();
-    // Reduce this tile into the thread's slice: column j, rows of its half.
-    float aW2[32], aW1[20], aB1 = 0.f, aB2 = 0.f, aW3 = 0.f, aB3 = 0.f;
 #pragma unroll
-    for (int q = 0; q < 32; ++q) aW2[q] = 0.f;
+    for (int i = 0; i < 8; ++i) {
+      const float d = dz3[pl.sample(i)];
 #pragma unroll
-    for (int q = 0; q < 20; ++q) aW1[q] = 0.f;
-    for (int t = 0; t < kThreads; ++t) {
-      const float d2 = sDZ2[t * kRowLd + j], d1 = sDZ1[t * kRowLd + j];
-#pragma unroll
-      for (int q = 0; q < 32; ++q) aW2[q] = fmaf(sH1[t * kRowLd + half * 32 + q], d2, aW2[q]);
-#pragma unroll
-      for (int q = 0; q < 20; ++q)
-        if (half * 20 + q < kIn) aW1[q] = fmaf(sENC[t * kEncLd + half * 20 + q], d1, aW1[q]);
-      if (half == 0) {
-        aB1 += d1;
-        aB2 += d2;
-        aW3 = fmaf(sH2[t * kRowLd + j], sDZ3[t], aW3);
-        if (j == 0) aB3 += sDZ3[t];
+      for (int j = 0; j < 4; ++j) {
+        gw3[j] = fmaf(v[i][j], d, gw3[j]);
+        v[i][j] = z2[i][j] > 0.0f ? sw[kW3 + pl.j0 + j] * d : 0.0f;
+        gb2[j] += v[i][j];
+        z2[i][j] = 0.0f;
       }
     }
-#pragma unroll
-    for (int q = 0; q < 32; ++q) sacc[kW2 + (half * 32 + q) * kH + j] += aW2[q];
-#pragma unroll
-    for (int q = 0; q < 20; ++q)
-      if (half * 20 + q < kIn) sacc[kW1 + (half * 20 + q) * kH + j] += aW1[q];
-    if (half == 0) {
-      sacc[kB1 + j] += aB1;
-      sacc[kB2 + j] += aB2;
-      sacc[kW3 + j] += aW3;
-      if (j == 0) sacc[kB3] += aB3;
-    }
+    store_tile(dz2, pl, v);
     __syncthreads();
+    // dz1 = (dz2 W2^T) * [h1 > 0]
+    tile_product<kH>(dz2, w2t, pl, z2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float *h = h1 + (pl.j0 + j) * kLdS;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (!(h[pl.sample(i)] > 0.0f)) z2[i][j] = 0.0f;
+        gb1[j] += z2[i][j];
+      }
+    }
+    store_tile(dz1, pl, z2);
+    outer_tile<4>(h1, dz2, tr, tc, gw2);
+    __syncthreads();
+    outer_tile<3>(enc, dz1, tr, tc, gw1);
+    __syncthreads();  // the tile's arrays are rewritten
   }
-  for (int q = tid; q < kParams; q += kThreads) atomicAdd(grads + q, sacc[q]);
-}
-
-static int grid_for(long long n, int per_cta_items) {
-  long long g = (n + per_cta_items - 1) / per_cta_items;
-  int sms = num_sms();
-  long long cap = (long long)(sms > 0 ? sms : 148) * 8;
-  return (int)(g < cap ? (g > 0 ? g : 1) : cap);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) atomicAdd(grads + kW2 + (tr + 16 * i) * kH + tc + 16 * j, gw2[i][j][0] + gw2[i][j][1]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (tr + 16 * i < kIn) atomicAdd(grads + kW1 + (tr + 16 * i) * kH + tc + 16 * j, gw1[i][j][0] + gw1[i][j][1]);
+    float b1 = gb1[j], b2 = gb2[j], w3 = gw3[j];
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {  // over the warp's sample groups
+      b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+      b2 += __shfl_xor_sync(0xffffffffu, b2, o);
+      w3 += __shfl_xor_sync(0xffffffffu, w3, o);
+    }
+    if ((tid & 31) < 8) {
+      atomicAdd(grads + kB1 + pl.j0 + j, b1);
+      atomicAdd(grads + kB2 + pl.j0 + j, b2);
+      atomicAdd(grads + kW3 + pl.j0 + j, w3);
+    }
+  }
+  if (tid < kTS) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
+    if ((tid & 31) == 0) atomicAdd(grads + kB3, gb3);
+  }
 }
 
 }  // namespace prop
 
 int launch_proposal_forward(const float *params, const float *xyz, long long n, float *sigma, cudaStream_t stream) {
-  prop::prop_fwd_kernel<<<prop::grid_for(n, prop::kThreads), prop::kThreads, 0, stream>>>(params, xyz, n, sigma);
+  if (cudaFuncSetAttribute(prop::prop_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)prop::kFwdSmem) != cudaSuccess)
+    return NERFGB_E_CUDA;
+  const long long tiles = (n + prop::kTS - 1) / prop::kTS;
+  const int sms = num_sms();
+  const long long cap = (long long)(sms > 0 ? sms : 148) * 2;
+  prop::prop_fwd_kernel<<<(unsigned)(tiles < cap ? tiles : cap), prop::kThreads, prop::kFwdSmem, stream>>>(params, xyz,
+                                                                                                         n, sigma);
   return launch_status();
 }
 
@@ -564,7 +639,7 @@ extern "C" int nerfgb_proposal_backward(const float *params, const float *xyz, c
   if (cudaFuncSetAttribute(prop::prop_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)prop::kBwdSmem) != cudaSuccess)
     return NERFGB_E_CUDA;
-  const long long ntiles = (n + prop::kThreads - 1) / prop::kThreads;
+  const long long ntiles = (n + prop::kTS - 1) / prop::kTS;
   int sms = num_sms();
   int grid = (int)(ntiles < sms ? ntiles : sms);
   prop::prop_bwd_kernel<<<grid, prop::kThreads, prop::kBwdSmem, as_stream(stream)>>>(params, xyz, grad_sigma, n,
