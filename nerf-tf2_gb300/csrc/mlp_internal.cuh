@@ -45,25 +45,29 @@ int launch_mlp_bf16_train(const void *packed, const float *xyz, const float *dir
                           float *rgb, float *sigma, uint16_t *tape, int *err_word, cudaStream_t stream);
 
 // Backward of the sigma and rgb heads (mlp_train.cu) from an FP32 or a BF16
-// activation tape: dz9 [n][256] (128 used) = dL/d(dense_9 pre-activation),
-// dsp [n] = dL/d(sigma pre-activation), head gradients into grads.
+// activation tape: dz9 = dL/d(dense_9 pre-activation), row stride 256 (128
+// used), FP32, or BF16 with dense_9's bias gradient added to grads; dsp [n] =
+// dL/d(sigma pre-activation); head gradients into grads.
 int launch_head_bwd(const float *table, const float *tape, long long n, const float *d_rgb, const float *d_sigma,
                     float *dz9, float *dsp, float *grads, cudaStream_t stream);
 int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const float *d_rgb,
-                    const float *d_sigma, float *dz9, float *dsp, float *grads, cudaStream_t stream);
+                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *grads, cudaStream_t stream);
 
-// Tensor-core GEMMs of the BF16 backward (gemm_tc.cu). dX [M][256] (BF16) =
-// dZ [M][n_out] (BF16, row stride 256) W^T with W the layer's BF16 weights
-// [k_in][n_out] (rows 0..255 used).
-int launch_gemm_dx(const __nv_bfloat16 *dz, long long M, int n_out, const __nv_bfloat16 *W, __nv_bfloat16 *dx,
-                   int *err, cudaStream_t stream);
-// grads [k][n] (row stride n_out) += sum_m In[m][k] dZ[m][n], k < k_in <= 256,
-// In BF16 with row stride ld_in, dZ BF16 with row stride 256; the rows are
-// reduced in `splits` parts whose partial sums go to `part`
-// (gemm_dw_partial_floats(splits) floats) before they are added.
-int launch_gemm_dw(const __nv_bfloat16 *in, long long ld_in, int k_in, const __nv_bfloat16 *dz, int n_out,
-                   long long M, float *grads, float *part, int splits, int *err, cudaStream_t stream);
-long long gemm_dw_partial_floats(int splits);
+// The dX products of the BF16 backward (mlp_bwd_tc.cu): dz [10][n][256] BF16,
+// dz[9] in, dz[8] .. dz[0] out, the bias gradients of dense_0 .. dense_8 added
+// to grads. wpack (mlp_chain_pack_bytes, 16-byte aligned) from the FP32 pack's
+// weights by launch_mlp_chain_pack; sigma_w: the sigma head's weights.
+long long mlp_chain_pack_bytes();
+int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t stream);
+int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
+                     __nv_bfloat16 *dz, float *grads, int *err, cudaStream_t stream);
+
+// Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
+// layer's In^T dZ over M rows added to the flat gradient blob, In from the
+// BF16 tape, dz [10][M][256] BF16; part: gemm_dw_partial_floats(M) floats.
+int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long M, float *grads, float *part, int *err,
+                   cudaStream_t stream);
+long long gemm_dw_partial_floats(long long M);
 // The BF16 (pair) or FP8 tensor-core forward with a chosen limit on every
 // bounded wait (ns) and the weight chunk at position `withhold` of the load
 // sequence of the (even) CTA left unloaded, so that a wait runs out: the

@@ -13,6 +13,10 @@
 //                                 * [h_prev[m][k] > 0]
 //   dW kernel     for every layer: dW[k][n] += sum_m In[m][k] dZ[m][n]
 // Gradients land in the flat Keras layout of the parameter blob.
+#include <cuda_bf16.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 #include "fp32_tile.cuh"
 #include "mlp_internal.cuh"
@@ -62,14 +66,18 @@ __device__ __forceinline__ void tape8(const uint16_t *p, float (&v)[8]) {
 constexpr int kHeadWarps = 8;
 constexpr int kHeadRows = 2;
 
-template <typename T>
+// TZ: dz9's type. BF16 (the tensor-core backward's operand): dense_9's bias
+// gradient, the column sums of the FP32 values, is taken here too.
+template <typename T, typename TZ>
 __global__ void __launch_bounds__(32 * kHeadWarps, 2)
     head_bwd_kernel(const float *__restrict__ table, const T *__restrict__ acts, long long n,
-                    const float *__restrict__ d_rgb, const float *__restrict__ d_sigma, float *__restrict__ dz9,
+                    const float *__restrict__ d_rgb, const float *__restrict__ d_sigma, TZ *__restrict__ dz9,
                     float *__restrict__ dsp_out, float *__restrict__ grads) {
-  __shared__ float sAcc[644];  // dWr [128][3], dbr [3], dws [256], dbs [1]
+  constexpr bool kBf16 = !std::is_same<TZ, float>::value;
+  constexpr int kAcc = kBf16 ? 772 : 644;
+  __shared__ float sAcc[kAcc];  // dWr [128][3], dbr [3], dws [256], dbs [1] (BF16: db9 [128])
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < 644; e += blockDim.x) sAcc[e] = 0.0f;
+  for (int e = threadIdx.x; e < kAcc; e += blockDim.x) sAcc[e] = 0.0f;
   float wr[4][3], wsg[8];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -79,7 +87,7 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
   for (int j = 0; j < 8; ++j) wsg[j] = table[kSigmaWOff + 8 * lane + j];
   const float br[3] = {table[kRgbBOff], table[kRgbBOff + 1], table[kRgbBOff + 2]};
   const float bs = table[kSigmaBOff];
-  float gwr[4][3], gws[8], gbr[3] = {0.f, 0.f, 0.f}, gbs = 0.0f;
+  float gwr[4][3], gws[8], gbr[3] = {0.f, 0.f, 0.f}, gbs = 0.0f, gb9[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int j = 0; j < 4; ++j) gwr[j][0] = gwr[j][1] = gwr[j][2] = 0.0f;
 #pragma unroll
@@ -143,7 +151,15 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
           const float g = drp[0] * wr[j][0] + drp[1] * wr[j][1] + drp[2] * wr[j][2];
           o[j] = h9[q][j] > 0.0f ? g : 0.0f;
         }
-        *reinterpret_cast<float4 *>(dz9 + r * kDzLd + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
+        if constexpr (kBf16) {
+          const __nv_bfloat162 p0 = __floats2bfloat162_rn(o[0], o[1]), p1 = __floats2bfloat162_rn(o[2], o[3]);
+          *reinterpret_cast<uint2 *>(dz9 + r * kDzLd + 4 * lane) =
+              make_uint2(*reinterpret_cast<const uint32_t *>(&p0), *reinterpret_cast<const uint32_t *>(&p1));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) gb9[j] += o[j];
+        } else {
+          *reinterpret_cast<float4 *>(dz9 + r * kDzLd + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
+        }
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -162,6 +178,10 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
     for (int c = 0; c < 3; ++c) atomicAdd(&sAcc[(4 * lane + j) * 3 + c], gwr[j][c]);
 #pragma unroll
   for (int j = 0; j < 8; ++j) atomicAdd(&sAcc[387 + 8 * lane + j], gws[j]);
+  if (kBf16) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(&sAcc[(kBf16 ? 644 : 0) + 4 * lane + j], gb9[j]);
+  }
   if (lane == 0) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) atomicAdd(&sAcc[384 + c], gbr[c]);
@@ -170,8 +190,13 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
   __syncthreads();
   float *gWr = grads + flat_offset(11), *gbr_out = gWr + 128 * 3;
   float *gws_out = grads + flat_offset(8), *gbs_out = gws_out + 256;
-  for (int e = threadIdx.x; e < 644; e += blockDim.x) {
-    float *dst = e < 384 ? gWr + e : e < 387 ? gbr_out + (e - 384) : e < 643 ? gws_out + (e - 387) : gbs_out;
+  float *gb9_out = grads + flat_offset(10) + (long long)flat_in(10) * flat_out(10);
+  for (int e = threadIdx.x; e < kAcc; e += blockDim.x) {
+    float *dst = e < 384   ? gWr + e
+                 : e < 387 ? gbr_out + (e - 384)
+                 : e < 643 ? gws_out + (e - 387)
+                 : e < 644 ? gbs_out
+                           : gb9_out + (e - 644);
     atomicAdd(dst, sAcc[e]);
   }
 }
@@ -374,16 +399,16 @@ __global__ void __launch_bounds__(256, 2)
 
 }  // namespace train
 
-template <typename T>
+template <typename T, typename TZ>
 static int launch_head_bwd_t(const float *table, const T *tape, long long n, const float *d_rgb,
-                             const float *d_sigma, float *dz9, float *dsp, float *grads, cudaStream_t st) {
+                             const float *d_sigma, TZ *dz9, float *dsp, float *grads, cudaStream_t st) {
   using namespace train;
   if (n == 0) return NERFGB_OK;
   const long long rows_per_block = (long long)kHeadWarps * kHeadRows;
   const long long blocks = (n + rows_per_block - 1) / rows_per_block;
   const int sms = num_sms();
   const long long cap = (long long)(sms > 0 ? sms : 148) * 2;  // two blocks per SM (launch bounds)
-  head_bwd_kernel<T><<<(unsigned)(blocks < cap ? blocks : cap), 32 * kHeadWarps, 0, st>>>(table, tape, n, d_rgb,
+  head_bwd_kernel<T, TZ><<<(unsigned)(blocks < cap ? blocks : cap), 32 * kHeadWarps, 0, st>>>(table, tape, n, d_rgb,
                                                                                         d_sigma, dz9, dsp, grads);
   return launch_status();
 }
@@ -394,7 +419,7 @@ int launch_head_bwd(const float *table, const float *tape, long long n, const fl
 }
 
 int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const float *d_rgb,
-                    const float *d_sigma, float *dz9, float *dsp, float *grads, cudaStream_t st) {
+                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *grads, cudaStream_t st) {
   return launch_head_bwd_t(table, tape, n, d_rgb, d_sigma, dz9, dsp, grads, st);
 }
 

@@ -224,14 +224,6 @@ __device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
                : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major, no swizzle (layout type 0),
-// descriptor version 1 at bit 46. lbo = byte stride between core matrices
-// adjacent in K, sbo = byte stride between 8-row groups.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-         (1ull << 46);
-}
-
 // Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
