@@ -121,7 +121,7 @@ def status_name(status):
 
 def call(name, *args):
     """Calls entry point `name`; raises NerfgbError on a non-zero status."""
-    rc = getattr(lib(), name)(*args)
+    rc = getattr(_lib or lib(), name)(*args)
     if rc != OK:
         raise NerfgbError(name, rc, status_name(rc))
     return rc

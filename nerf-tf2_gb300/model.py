@@ -340,6 +340,12 @@ class NeRF:
             min(chunk, R), Sc, Sf)
         pc, pf = self.coarse_model.packed(precision), self.fine_model.packed(precision)
         n_st = min(int(streams), max(1, (R + chunk - 1) // chunk))
+        if R <= chunk:  # one chunk: the whole batch on the caller's stream
+            if R > 0:
+                self._render_chunk(lib, gated, proposal, pc, pf, prec, rays_o, rays_d, near, far, u_coarse, u_fine,
+                                   seed, 0, None, R, Sc, Sf, gate_tau, gate_fine_draws, return_coarse, out,
+                                   torch.empty(ws_bytes, dtype=torch.uint8, device=rays_o.device))
+            return out
         main = torch.cuda.current_stream()
         sts = [main] + self._side_streams(n_st - 1)
         wss = [torch.empty(ws_bytes, dtype=torch.uint8, device=rays_o.device) for _ in range(n_st)]
@@ -374,44 +380,27 @@ class NeRF:
 
     def _render_chunk(self, lib, gated, proposal, pc, pf, prec, rays_o, rays_d, near, far, u_coarse, u_fine,
                       seed, s, sl, e, Sc, Sf, gate_tau, gate_fine_draws, return_coarse, out, ws):
-        """One chunk's library call, on the current stream."""
+        """One chunk's library call, on the current stream (sl: its rays; None:
+        all of them, taken as they are)."""
+        cut = (lambda x: ptr(x)) if sl is None else (lambda x: None if x is None else ptr(x[sl]))
+        sampling = self.params.sampling
+        rays = (prec, cut(rays_o), cut(rays_d), cut(near), cut(far), cut(u_coarse), cut(u_fine),
+                ctypes.c_ulonglong(int(seed) + s), e - s, Sc, Sf, int(bool(sampling.perturb)),
+                int(bool(sampling.lin_inv_depth)), int(self.white_bg), int(self.trans_mode))
+        maps = (cut(out["rgb"]), cut(out["depth"]), cut(out["acc"]), ptr(ws))
         if gated:
-            _lib.call("nerfgb_render_rays_gated", ptr(proposal.params), ptr(pc), ptr(pf), prec,
-                      ptr(rays_o[sl]), ptr(rays_d[sl]), ptr(near[sl]), ptr(far[sl]),
-                      ptr(u_coarse[sl]) if u_coarse is not None else None,
-                      ptr(u_fine[sl]) if u_fine is not None else None,
-                      ctypes.c_ulonglong(int(seed) + s), e - s, Sc, Sf,
-                      int(bool(self.params.sampling.perturb)),
-                      int(bool(self.params.sampling.lin_inv_depth)), int(self.white_bg),
-                      int(self.trans_mode), ctypes.c_float(gate_tau),
-                      _lib.GATE_FINE_DRAWS if gate_fine_draws else 0, ptr(out["rgb"][sl]),
-                      ptr(out["depth"][sl]), ptr(out["acc"][sl]), ptr(ws),
+            _lib.call("nerfgb_render_rays_gated", ptr(proposal.params), ptr(pc), ptr(pf), *rays,
+                      ctypes.c_float(gate_tau), _lib.GATE_FINE_DRAWS if gate_fine_draws else 0, *maps,
                       ptr(self.coarse_model.err_word), stream())
             return
         if proposal is not None:
-            _lib.call("nerfgb_render_rays_proposal", ptr(proposal.params), ptr(pf), prec,
-                      ptr(rays_o[sl]), ptr(rays_d[sl]), ptr(near[sl]), ptr(far[sl]),
-                      ptr(u_coarse[sl]) if u_coarse is not None else None,
-                      ptr(u_fine[sl]) if u_fine is not None else None,
-                      ctypes.c_ulonglong(int(seed) + s), e - s, Sc, Sf,
-                      int(bool(self.params.sampling.perturb)),
-                      int(bool(self.params.sampling.lin_inv_depth)), int(self.white_bg),
-                      int(self.trans_mode), ptr(out["rgb"][sl]), ptr(out["depth"][sl]),
-                      ptr(out["acc"][sl]), ptr(ws), ptr(self.fine_model.err_word), stream())
+            _lib.call("nerfgb_render_rays_proposal", ptr(proposal.params), ptr(pf), *rays, *maps,
+                      ptr(self.fine_model.err_word), stream())
             return
-        _lib.call("nerfgb_render_rays", ptr(pc), ptr(pf), prec, ptr(rays_o[sl]), ptr(rays_d[sl]),
-                  ptr(near[sl]), ptr(far[sl]),
-                  ptr(u_coarse[sl]) if u_coarse is not None else None,
-                  ptr(u_fine[sl]) if u_fine is not None else None,
-                  ctypes.c_ulonglong(int(seed) + s), e - s, Sc, Sf,
-                  int(bool(self.params.sampling.perturb)),
-                  int(bool(self.params.sampling.lin_inv_depth)), int(self.white_bg),
-                  int(self.trans_mode),
-                  ptr(out["rgb_coarse"][sl]) if return_coarse else None,
-                  ptr(out["depth_coarse"][sl]) if return_coarse else None,
-                  ptr(out["acc_coarse"][sl]) if return_coarse else None,
-                  ptr(out["rgb"][sl]), ptr(out["depth"][sl]), ptr(out["acc"][sl]), ptr(ws),
-                  ptr(self.coarse_model.err_word), stream())
+        _lib.call("nerfgb_render_rays", ptr(pc), ptr(pf), *rays,
+                  *((cut(out["rgb_coarse"]), cut(out["depth_coarse"]), cut(out["acc_coarse"])) if return_coarse
+                    else (None, None, None)),
+                  *maps, ptr(self.coarse_model.err_word), stream())
 
     def load_model(self, load_dir, load_tag, skip_optimizer=False):
         """NeRF.set_everything (nerf/core/model.py:238-287): unless
