@@ -14,18 +14,19 @@
 // so a small batch (one sub-tile per pair) has half the latency of a whole
 // tile and the last wave of a large one is half as coarse.
 //
-// Warp roles (10 warps; 11 with the tape):
-//   warp 0      weight producer: one thread copying weight chunks in ring
-//               order (full/empty mbarriers) with 2-SM tensor copies that
-//               complete on the even CTA's barrier
-//   warp 1      TMEM allocator and, in the even CTA, MMA issuer (one thread;
-//               its issue code is generated per layer at compile time)
-//   warps 2-9   epilogue, all on one sub-tile at a time: positional
-//               encodings, then per layer the accumulator (tcgen05.ld), bias,
-//               ReLU, rounding to BF16 (or E4M3) and the next layer's A
-//               operand; the sigma and rgb heads run in FP32
-//   warp 10     (training tape only) one thread storing each written operand
-//               region to the tape by a tensor store
+// Warp roles (14 warps; 15 with the tape):
+//   warp 0       weight producer: one thread copying weight chunks in ring
+//                order (full/empty mbarriers) with 2-SM tensor copies that
+//                complete on the even CTA's barrier
+//   warp 1       TMEM allocator and, in the even CTA, MMA issuer (one thread;
+//                its issue code is generated per kind of layer at compile time)
+//   warps 2-9    epilogue of layers 0-8, all on one sub-tile at a time: the
+//                accumulator (tcgen05.ld), bias, ReLU, rounding to BF16 (or
+//                E4M3) and the next layer's A operand; the sigma head in FP32
+//   warps 10-13  beside it, a row per lane: the positional encodings, dense_9
+//                and the rgb head in FP32
+//   warp 14      (training tape only) one thread storing each written operand
+//                region to the tape by a tensor store
 //
 // What bounds it and why it is laid out so (a 256-wide layer of a sub-tile is
 // 2,048 cycles of MMAs in BF16, half that in E4M3; the L1/shared data pipe
@@ -41,7 +42,7 @@
 //   columns of the sub-tile's activation region; the region E holds A's
 //   encoding for dense_5, then (once A's dense_5 MMAs are done) B's, then
 //   both sub-tiles' direction encodings for dense_9. The encodings are
-//   computed again for each write, in the epilogue warps' waits.
+//   computed again for each write (by one copy of the code).
 // - The epilogue of a plain layer reads the accumulator in the 16x256b
 //   fragment layout and stores it with stmatrix: a thread then adds 2 biases
 //   per 8 columns instead of 8 (a broadcast LDG.128 costs four wavefronts of
@@ -50,21 +51,28 @@
 //   where the sigma head reads it a row per lane: the heads' sums run along a
 //   row in a fixed order. The head weights sit in shared memory (a broadcast
 //   LDS.128 costs two wavefronts).
-// - Eight epilogue warps with 168 registers rather than sixteen with 96:
-//   nothing may spill, as the 28 KB of L1 beside this much shared memory do
-//   not hold spills and a reload is a trip to L2 (sixteen warps: 648 us, and
-//   1,190 with 200 bytes of spills, against 610).
-// - At the tile boundary dense_0's operand is written as soon as dense_9's
-//   accumulator has been read, before the rgb head.
+// - Eight epilogue warps and four side warps with 128 registers: nothing may
+//   spill, as the 28 KB of L1 beside this much shared memory do not hold
+//   spills and a reload is a trip to L2 (sixteen epilogue warps with 96: 648
+//   us, and 1,190 with 200 bytes of spills, against 610).
+// - The encodings and dense_9 are the side warps': with the epilogue's eight
+//   warps doing them the tensor core waited ~7k cycles per tile for the heads
+//   at the tile's end and ~2k more behind the sigma head (BF16 607 us, FP8
+//   620, with the tape 930). The rgb head takes a side warp ~2.7k cycles per
+//   sub-tile (its broadcast loads alone ~1.3k of the data pipe); shared with
+//   the epilogue's warps, which then start dense_0 later, it was 554 and 459.
+// - dense_0's operand is written as soon as dense_9 is done, before the rgb
+//   head, and its MMAs wait only for the head's reads of the accumulator.
+// - E4M3's ReLU runs on the packed words (relu_e4m3x4): 484 -> 452 us.
 // - Even deals of 256-row sub-tiles: see above.
 // Measured against the kernels before (a 4-stage pair kernel in BF16, one CTA
-// per tile in FP8): 786,432 rows BF16 783 -> 610 us, with the tape 1,613 ->
-// 953, FP8 904 -> 622; 1,000 rows BF16 43 -> 31 us. A BF16 tile takes ~56k
-// cycles, 37k of them MMAs; the largest waits left are the heads at the tile
-// boundary (~7k) and dense_8 behind the sigma head (~2k).
+// per tile in FP8): 786,432 rows BF16 783 -> 546 us, with the tape 1,613 ->
+// 805, FP8 904 -> 452; 1,000 rows BF16 43 -> 31 us, FP8 41 -> 26. A BF16 tile
+// takes ~51k cycles, 37k of them MMAs; the largest waits left are the rgb
+// heads at the tile boundary (~5k).
 //
-// Shared memory: ring [0,80K) | E [80K,96K) | actA, actB | barriers, sigma
-// weights and partials (in the 3 KB left). Operands are K-major in the
+// Shared memory: ring [0,80K) | E [80K,96K) | actA, actB | barriers and head
+// weights (in the 3 KB left). Operands are K-major in the
 // 128-byte swizzled layout: atoms of 128 bytes of K (64 BF16 or 128 E4M3) by
 // 128 rows, 16 KB each; row r at r*128, its 16-byte chunk c at (c ^ (r&7))*16,
 // so that a region goes to the row-major tape as whole 128-byte rows. Weights:
@@ -93,11 +101,13 @@ namespace nerfgb {
 namespace tc {
 
 constexpr int kSubRows = 256;  // rows of a sub-tile: 128 per CTA of the pair
-// Column parts of the epilogue: one warp per part and TMEM lane quadrant.
+// Warps: producer, issuer, the epilogue's (one per column part and TMEM lane
+// quadrant), the side warps (one per quadrant: encodings and the rgb head) and,
+// in the kernel that writes the activation tape, one whose first lane stores
+// each written operand region to the tape.
 constexpr int kParts = 2, kEpiWarps = 4 * kParts;
-// The kernel that writes the activation tape has one more warp, whose first
-// lane stores each written operand region to the tape.
-__host__ __device__ constexpr int threads_of(bool tape) { return (2 + kEpiWarps + (tape ? 1 : 0)) * 32; }
+constexpr int kSideWarp = 2 + kEpiWarps, kTapeWarp = kSideWarp + 4;
+__host__ __device__ constexpr int threads_of(bool tape) { return (kTapeWarp + (tape ? 1 : 0)) * 32; }
 
 // Tensor maps of the pack's weights (2-D, 256-byte rows), one per size of a
 // CTA's half of a chunk: 16 KB, 8 KB and dense_9's last chunk (4 KB BF16, 2 KB
@@ -122,24 +132,26 @@ struct Layout {
   static constexpr uint32_t kMisc = kActOff + 2 * kActBytes;
   static constexpr uint32_t kBarFull = kMisc;              // [kNst]
   static constexpr uint32_t kBarEmpty = kMisc + 64;        // [kNst]
-  static constexpr uint32_t kBarAccf = kMisc + 128;        // [2] accumulators full
-  static constexpr uint32_t kBarActr = kMisc + 144;        // [2] operands ready
-  static constexpr uint32_t kBarRgb = kMisc + 160;         // [2] rgb partials written
-  static constexpr uint32_t kBarFree = kMisc + 176;        // [2] rgb partials read
-  static constexpr uint32_t kBarEncB = kMisc + 192;        // B's encoding in E
-  static constexpr uint32_t kBarDrain = kMisc + 200;
-  static constexpr uint32_t kBarTapeRdy = kMisc + 208;     // [2]
-  static constexpr uint32_t kBarTapeDone = kMisc + 224;    // [2]
-  static constexpr uint32_t kTmemSlot = kMisc + 240;
-  static constexpr uint32_t kAbort = kMisc + 248;          // int, then the wait limit (u64) at +8
-  static constexpr uint32_t kBarTapeTail = kMisc + 264;    // [2]
-  static constexpr uint32_t kBarSig = kMisc + 280;         // [2] sigma's half sum written
-  static constexpr uint32_t kHeadW = kMisc + 304;          // the sigma head's weights [256], the rgb head's [128][3]
-  static constexpr uint32_t kSmemBytes = kHeadW + (256 + 384) * 4;
-  // The rgb head's partial sums of half the columns, float [3][parts - 1][128], in the
-  // sub-tile's last activation atom (last read by dense_9, rewritten by the
-  // next dense_0's epilogue, which waits for kBarFree).
-  static constexpr uint32_t kRgbPart = kActBytes - kAtom;
+  static constexpr uint32_t kBarAccf = kMisc + 128;        // [2] accumulator full (layers 0-8)
+  static constexpr uint32_t kBarAcc5 = kMisc + 144;        // [2] ... of dense_5, for the side warps
+  static constexpr uint32_t kBarAcc9 = kMisc + 160;        // [2] ... of dense_9
+  static constexpr uint32_t kBarActr = kMisc + 176;        // [2] operand ready (layers 1-9)
+  static constexpr uint32_t kBarAct0 = kMisc + 192;        // [2] dense_0's operand, dense_9's accumulator read
+  static constexpr uint32_t kBarEncA = kMisc + 208;        // A's encoding in E
+  static constexpr uint32_t kBarEncB = kMisc + 216;        // B's
+  static constexpr uint32_t kBarDir = kMisc + 224;         // the direction encodings
+  static constexpr uint32_t kBarRead8 = kMisc + 232;       // [2] the second part has read dense_8's accumulator
+  static constexpr uint32_t kBarSig = kMisc + 248;         // [2] sigma's sums in TMEM
+  static constexpr uint32_t kBarDrain = kMisc + 264;
+  static constexpr uint32_t kBarTapeRdy = kMisc + 272;     // [2] h0 .. h8
+  static constexpr uint32_t kBarTapeEnc = kMisc + 288;     // [2] enc_xyz
+  static constexpr uint32_t kBarTapeTail = kMisc + 304;    // [2] enc_dir and h9
+  static constexpr uint32_t kBarTapeDone = kMisc + 320;    // [2]
+  static constexpr uint32_t kTmemSlot = kMisc + 336;
+  static constexpr uint32_t kAbort = kMisc + 344;          // int, then the wait limit (u64) at +8
+  static constexpr uint32_t kHeadW = kMisc + 368;          // the sigma head's weights [256], the rgb head's [128][3]
+  static constexpr uint32_t kHeadB = kHeadW + (256 + 384) * 4;  // FP8: dense_9's biases and scales [2][128]
+  static constexpr uint32_t kSmemBytes = kHeadB + (F8 ? 1024 : 0);
   static_assert(kSmemBytes <= 227 * 1024 && kAbort % 8 == 0 && kHeadW % 16 == 0, "shared memory");
 };
 
@@ -203,25 +215,16 @@ __device__ __forceinline__ void store_chunks(uint32_t atom, int r, uint32_t c0, 
     st_shared_v4(row + (((c0 + i) ^ x) << 4), pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
 }
 
-// Part Q of the encodings, packed: enc_xyz's 64 columns (63 values, column
-// 63 = 0), enc_dir's 32 (27 values, 5 zero pad).
-template <int Q, bool F8, bool DIR>
-__device__ __forceinline__ void encode_part(const float (&x)[3],
-                                            uint32_t (&pk)[(DIR ? 32 : 64) / kParts / (F8 ? 4 : 2)]) {
-  constexpr int W = (DIR ? 32 : 64) / kParts;
+// A row's encoding, packed: enc_xyz's 64 columns (63 values, column 63 = 0) or
+// enc_dir's 32 (27 values, 5 zero pad).
+template <bool F8, bool DIR>
+__device__ __forceinline__ void encode_row(const float (&x)[3], uint32_t (&pk)[(DIR ? 32 : 64) / (F8 ? 4 : 2)]) {
+  constexpr int W = DIR ? 32 : 64;
   float v[W];
 #pragma unroll
-  for (int i = 0; i < W; ++i) v[i] = (Q == 0 && i < 3) ? x[i % 3] : 0.0f;
-  encode_pairs_q<DIR ? 12 : 30, DIR ? 4 : 10, W, Q>(x, v);
+  for (int i = 0; i < W; ++i) v[i] = i < 3 ? x[i % 3] : 0.0f;
+  encode_pairs_q<DIR ? 12 : 30, DIR ? 4 : 10, W, 0>(x, v);
   pack_cols<W, F8>(v, pk);
-}
-template <bool F8, bool DIR>
-__device__ __forceinline__ void encode_any(int q, const float (&x)[3],
-                                           uint32_t (&pk)[(DIR ? 32 : 64) / kParts / (F8 ? 4 : 2)]) {
-  if (q == 0)
-    encode_part<0, F8, DIR>(x, pk);
-  else
-    encode_part<1, F8, DIR>(x, pk);
 }
 
 // ---------------------------------------------------------------------------
@@ -258,6 +261,16 @@ struct FragBias {
   }
 };
 
+// max(x, 0) of four E4M3 values as fmaxf would have it before the rounding:
+// zero where the byte's sign is set, and for NaN (0x7F). Three operations on
+// the word instead of four FP32 maxima (two cycles each).
+__device__ __forceinline__ uint32_t relu_e4m3x4(uint32_t w) {
+  // bit 7 of a byte + 1: negative (0x80 .. 0xFE) or 0x7F; no byte is 0xFF, so none carries
+  uint32_t m;
+  asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(m) : "r"(w + 0x01010101u));  // each byte its sign
+  return w & ~m;
+}
+
 // 16 rows x 32 columns of fragments (raw: group i's four registers: the pair
 // of row lane/4, then of row lane/4 + 8) to the operand: `addr` this lane's
 // stmatrix row (row 8*((lane>>3)&1) + lane%8 of the 16, chunk 0), cx = (lane>>4) ^
@@ -270,12 +283,11 @@ __device__ __forceinline__ void store_frag(uint32_t addr, uint32_t cx, uint32_t 
   float v[16];
 #pragma unroll
   for (int i = 0; i < 8; ++i) fb.apply(i / 2, raw[2 * i], raw[2 * i + 1], v[2 * i], v[2 * i + 1]);
-  if (F8 || KEEP) {
+  if (KEEP) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float m = KEEP || relu ? fmaxf(v[i], 0.0f) : v[i];
-      if (KEEP) raw[i] = __float_as_uint(m);
-      if (F8) v[i] = m;
+      v[i] = fmaxf(v[i], 0.0f);
+      raw[i] = __float_as_uint(v[i]);
     }
   }
   uint32_t w[F8 ? 4 : 8];
@@ -284,6 +296,10 @@ __device__ __forceinline__ void store_frag(uint32_t addr, uint32_t cx, uint32_t 
     for (int j = 0; j < 2; ++j) {  // chunk j: rows lane/4 (2j), lane/4 + 8 (2j + 1)
       w[2 * j] = pack_e4m3x4(v[8 * j], v[8 * j + 1], v[8 * j + 4], v[8 * j + 5]);
       w[2 * j + 1] = pack_e4m3x4(v[8 * j + 2], v[8 * j + 3], v[8 * j + 6], v[8 * j + 7]);
+      if (!KEEP && relu) {
+        w[2 * j] = relu_e4m3x4(w[2 * j]);
+        w[2 * j + 1] = relu_e4m3x4(w[2 * j + 1]);
+      }
     }
   } else {
 #pragma unroll
@@ -324,23 +340,6 @@ __device__ __forceinline__ float4 lds_here(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
-// acc (FP8: * scale) + bias; the accumulator loads complete here.
-template <bool F8>
-__device__ __forceinline__ void row_bias(uint32_t (&raw)[32], const float *bias, const float *scale, float (&v)[32]) {
-  tmem_wait32(raw);
-#pragma unroll
-  for (int i = 0; i < 32; i += 4) {
-    const float4 b4 = ld_here(bias + i);
-    if (F8) {
-      const float4 s4 = ld_here(scale + i);
-      fma_f32x2(v[i], v[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), s4.x, s4.y, b4.x, b4.y);
-      fma_f32x2(v[i + 2], v[i + 3], __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]), s4.z, s4.w, b4.z, b4.w);
-    } else {
-      add_f32x2(v[i], v[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), b4.x, b4.y);
-      add_f32x2(v[i + 2], v[i + 3], __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]), b4.z, b4.w);
-    }
-  }
-}
 // ---------------------------------------------------------------------------
 // MMA issue (pair_tc.cuh): per layer, generated at compile time
 // ---------------------------------------------------------------------------
@@ -348,7 +347,7 @@ __device__ __forceinline__ void row_bias(uint32_t (&raw)[32], const float *bias,
 // encoding (the rest)] for dense_5 and dense_9, the encoding (in the
 // activation region) for dense_0 and the activation alone otherwise.
 template <int G, int S, bool F8>
-__device__ __forceinline__ void issue_gemm(uint32_t sbase, uint32_t tmem, bool release, uint32_t encb_phase,
+__device__ __forceinline__ void issue_gemm(uint32_t sbase, uint32_t tmem, bool release, uint32_t tile_phase,
                                            RingPos &rp, volatile int *abort_flag, int *err) {
   using L = Layout<F8>;
   constexpr int N = gemm_n(G), H = N / 2;
@@ -372,9 +371,9 @@ __device__ __forceinline__ void issue_gemm(uint32_t sbase, uint32_t tmem, bool r
     issue_run<L::kNst, 1, kAct, H, F8, true, S == 0>(bar_full, bar_empty, ring_lo, act_lo, acc, idesc, release, rp, abort_flag,
                                             err);
   if constexpr (kEnc > 0) {
-    if (G == 5 && S == 1) {
-      // B's encoding replaces A's in E once A's MMAs are done
-      wait_fast(sbase + L::kBarEncB, encb_phase, abort_flag, err);
+    if (G == 5 || S == 0) {
+      // E holds A's encoding, then B's, then the direction encodings
+      wait_fast(sbase + (G == 9 ? L::kBarDir : S == 0 ? L::kBarEncA : L::kBarEncB), tile_phase, abort_flag, err);
       tc_fence_after();
     }
     const uint32_t enc_lo = ((sw + L::kEncOff + (G == 9 ? S * 64u : 0u)) >> 4) | (1u << 16);
@@ -383,26 +382,34 @@ __device__ __forceinline__ void issue_gemm(uint32_t sbase, uint32_t tmem, bool r
   }
 }
 
-// One layer: per sub-tile, wait until the epilogue has written the A operand
-// (and read the accumulator), issue, then signal the accumulator full. The
-// last sub-tile's MMAs release the layer's stages.
-template <int G, bool F8>
-__device__ __forceinline__ void issue_layer(uint32_t sbase, uint32_t tmem, int nsub, RingPos &rp, uint32_t actr_phase,
-                                            uint32_t encb_phase, volatile int *abort_flag, int *err) {
+// One layer: per sub-tile, wait until its A operand is written (and its
+// accumulator read), issue, then signal the accumulator full. The last
+// sub-tile's MMAs release the layer's stages. actr_phase: the parity of the
+// epilogue's operand barriers, toggled per layer from dense_1 on; tile_phase:
+// of the barriers that complete once per tile.
+template <int G, int S, bool F8>
+__device__ __forceinline__ void issue_sub(uint32_t sbase, uint32_t tmem, bool release, RingPos &rp, uint32_t actr_phase,
+                                          uint32_t tile_phase, volatile int *abort_flag, int *err) {
   using L = Layout<F8>;
-  const uint32_t actr = sbase + L::kBarActr, accf = sbase + L::kBarAccf;
-  wait_fast(actr, actr_phase, abort_flag, err);
+  if (G == 0)
+    wait_fast(sbase + L::kBarAct0 + 8 * S, tile_phase, abort_flag, err);
+  else
+    wait_fast(sbase + L::kBarActr + 8 * S, actr_phase, abort_flag, err);
   tc_fence_after();
+  issue_gemm<G, S, F8>(sbase, tmem, release, tile_phase, rp, abort_flag, err);
+  if (G == 5) tc_commit_pair(sbase + L::kBarAcc5 + 8 * S);
+  tc_commit_pair(sbase + (G == 9 ? L::kBarAcc9 : L::kBarAccf) + 8 * S);
+}
+template <int G, bool F8>
+__device__ __forceinline__ void issue_layer(uint32_t sbase, uint32_t tmem, int nsub, RingPos &rp, uint32_t &actr_phase,
+                                            uint32_t tile_phase, volatile int *abort_flag, int *err) {
   const RingPos start = rp;
-  issue_gemm<G, 0, F8>(sbase, tmem, nsub == 1, encb_phase, rp, abort_flag, err);
-  tc_commit_pair(accf);
+  issue_sub<G, 0, F8>(sbase, tmem, nsub == 1, rp, actr_phase, tile_phase, abort_flag, err);
   if (nsub == 2) {
-    wait_fast(actr + 8, actr_phase, abort_flag, err);
-    tc_fence_after();
     rp = start;
-    issue_gemm<G, 1, F8>(sbase, tmem, true, encb_phase, rp, abort_flag, err);
-    tc_commit_pair(accf + 8);
+    issue_sub<G, 1, F8>(sbase, tmem, true, rp, actr_phase, tile_phase, abort_flag, err);
   }
+  if (G > 0) actr_phase ^= 1u;
 }
 
 // ---------------------------------------------------------------------------
@@ -451,6 +458,9 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
 
   // head weights: table[kSigmaWOff ..] (256 floats), table[kRgbWOff ..] (384)
   static_assert(kSigmaWOff % 4 == 0 && kRgbWOff % 4 == 0, "float4 copies");
+  if (F8 && threadIdx.x < 64)
+    reinterpret_cast<float4 *>(smem + L::kHeadB)[threadIdx.x] = reinterpret_cast<const float4 *>(
+        (threadIdx.x < 32 ? table : scales - 128) + bias_offset(9))[threadIdx.x];
   if (threadIdx.x < 64 + 96)
     reinterpret_cast<float4 *>(smem + L::kHeadW)[threadIdx.x] = reinterpret_cast<const float4 *>(
         table + (threadIdx.x < 64 ? kSigmaWOff : kRgbWOff - 256))[threadIdx.x];
@@ -463,15 +473,20 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(sbase + L::kBarAccf + 8 * s, 1);
+      mbar_init(sbase + L::kBarAcc5 + 8 * s, 1);
+      mbar_init(sbase + L::kBarAcc9 + 8 * s, 1);
       mbar_init(sbase + L::kBarActr + 8 * s, 2 * kEpiWarps);  // one arrival per epilogue warp of both CTAs
-      mbar_init(sbase + L::kBarSig + 8 * s, kEpiWarps / kParts);
-      mbar_init(sbase + L::kBarRgb + 8 * s, kEpiWarps / kParts);
-      mbar_init(sbase + L::kBarFree + 8 * s, 4);   // one arrival per warp that reads the partials
+      mbar_init(sbase + L::kBarAct0 + 8 * s, 2 * 4);          // ... per side warp of both CTAs
+      mbar_init(sbase + L::kBarRead8 + 8 * s, 4);
+      mbar_init(sbase + L::kBarSig + 8 * s, 4);
       mbar_init(sbase + L::kBarTapeRdy + 8 * s, kEpiWarps);
+      mbar_init(sbase + L::kBarTapeEnc + 8 * s, 4);
+      mbar_init(sbase + L::kBarTapeTail + 8 * s, 4);
       mbar_init(sbase + L::kBarTapeDone + 8 * s, 1);
-      mbar_init(sbase + L::kBarTapeTail + 8 * s, kEpiWarps);
     }
-    mbar_init(sbase + L::kBarEncB, 2 * kEpiWarps);
+    mbar_init(sbase + L::kBarEncA, 2 * 4);
+    mbar_init(sbase + L::kBarEncB, 2 * 4);
+    mbar_init(sbase + L::kBarDir, 2 * 4);
     mbar_init(sbase + L::kBarDrain, 1);
     *abort_flag = 0;
     set_wait_limit(abort_flag, wait_ns);
@@ -548,22 +563,21 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
       // After an abort every wait returns at once: the remaining MMAs of the
       // tile read stale (in-bounds) shared memory and the tile loop ends.
       RingPos rp{0, 0u};
-      uint32_t encb_phase = 0;
+      uint32_t actr_phase = 0;
       for (int tile = 0; tile < ntiles; ++tile) {
         if (*abort_flag) break;
         const int nsub = 2 * tile + 1 < count ? 2 : 1;
-        issue_layer<0, F8>(sbase, tmem, nsub, rp, 0u, encb_phase, abort_flag, err);
-        issue_layer<1, F8>(sbase, tmem, nsub, rp, 1u, encb_phase, abort_flag, err);
-        issue_layer<2, F8>(sbase, tmem, nsub, rp, 0u, encb_phase, abort_flag, err);
-        issue_layer<3, F8>(sbase, tmem, nsub, rp, 1u, encb_phase, abort_flag, err);
-        issue_layer<4, F8>(sbase, tmem, nsub, rp, 0u, encb_phase, abort_flag, err);
-        issue_layer<5, F8>(sbase, tmem, nsub, rp, 1u, encb_phase, abort_flag, err);
-        issue_layer<6, F8>(sbase, tmem, nsub, rp, 0u, encb_phase, abort_flag, err);
-        issue_layer<7, F8>(sbase, tmem, nsub, rp, 1u, encb_phase, abort_flag, err);
-        issue_layer<8, F8>(sbase, tmem, nsub, rp, 0u, encb_phase, abort_flag, err);
-        issue_layer<9, F8>(sbase, tmem, nsub, rp, 1u, encb_phase, abort_flag, err);
-        static_assert(kNumGemm == 10, "one issue_layer per GEMM, operand barriers' parity = g % 2");
-        encb_phase ^= 1;
+        const uint32_t ph = (uint32_t)(tile & 1);
+        issue_layer<0, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+        // (one copy of the issue code for the layers of one shape: the
+        // kernel's code is several times the instruction cache's first levels)
+#pragma unroll 1
+        for (int g = 1; g <= 4; ++g) issue_layer<1, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+        issue_layer<5, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+#pragma unroll 1
+        for (int g = 6; g <= 8; ++g) issue_layer<6, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+        issue_layer<9, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+        static_assert(kNumGemm == 10, "layers 1-4 and 6-8 are alike");
       }
       if (ntiles > 0) {
         // Drain every MMA issued by this thread before TMEM is released (in
@@ -574,76 +588,62 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
         }
       }
     }
-  } else if (STORE && warp == 2 + kEpiWarps) {
+  } else if (STORE && warp == kTapeWarp) {
     // ---------------- tape writer ----------------
-    // Per tile and sub-tile the epilogue signals ten regions on tape_rdy, in
-    // order: enc_xyz (dense_0's operand), then h0 .. h8 (each layer's output,
-    // the next layer's operand). Each goes to its tape columns of the
-    // sub-tile's 128 rows as one tensor store of 128-byte rows (rows past n
-    // are not written); once the store has read shared memory, tape_done
-    // tells the epilogue that the region may be rewritten. The row's last
+    // Per tile and sub-tile ten regions are signalled in order: enc_xyz
+    // (dense_0's operand, by the side warps), then h0 .. h8 (each layer's
+    // output, the next layer's operand, by the epilogue). Each goes to its
+    // tape columns of the sub-tile's 128 rows as one tensor store of 128-byte
+    // rows (rows past n are not written); once the store has read shared
+    // memory, tape_done tells that the region may be rewritten. The row's last
     // columns, enc_dir and h9, follow in the region's second and third atom
     // on a barrier of their own (before the next tile's enc_xyz, whose
     // tape_done covers them), but for h9's last 32 columns, half an atom,
-    // which the epilogue stores itself.
+    // which the side warps store themselves.
     if (lane == 0) {
       uint32_t rdy_phase[2] = {0u, 0u};
       bool ok = true;
-      for (int tile = 0; tile < ntiles && ok; ++tile) {
-        const int nsub = 2 * tile + 1 < count ? 2 : 1;
-        for (int e = 0; e < 11 && ok; ++e) {
-          for (int s = 0; s < nsub; ++s) {
-            const bool tail = e == 10;
-            if (!wait_bar(sbase + (tail ? L::kBarTapeTail : L::kBarTapeRdy) + 8 * s,
-                          tail ? (uint32_t)(tile & 1) : rdy_phase[s], abort_flag, err)) {
-              ok = false;
-              break;
-            }
-            if (!tail) rdy_phase[s] ^= 1u;
-            const long long row = row_of(tile, s, 0);
-            if (row < n) {  // (a box from row n on would write nothing)
-              const uint32_t act = sbase + L::kActOff + s * L::kActBytes;
-              if (tail)
-                tma_store_3d(&maps.tape[2], act + kAtom, 0, (int)row, kActsEncDir / 64);
-              else
-                tma_store_3d(&maps.tape[e == 0 ? 1 : 0], act, 0, (int)row, e == 0 ? 0 : acts_offset(e - 1) / 64);
-              bulk_commit();
-              bulk_wait_read();
-            }
-            if (!tail) mbar_arrive(sbase + L::kBarTapeDone + 8 * s);
+      // one region: sub-tile s of tile k, from atom A of the operand to column group z of the tape
+      auto store = [&](uint32_t bar, uint32_t parity, const CUtensorMap *map, int k, int s, uint32_t atom, int z) {
+        if (!wait_bar(sbase + bar + 8 * s, parity, abort_flag, err)) return false;
+        const long long row = row_of(k, s, 0);
+        if (row < n) {  // (a box from row n on would write nothing)
+          tma_store_3d(map, sbase + L::kActOff + s * L::kActBytes + atom * kAtom, 0, (int)row, z);
+          bulk_commit();
+          bulk_wait_read();
+        }
+        return true;
+      };
+      for (int tile = -1; tile < ntiles && ok; ++tile) {
+        const int next_subs = min(2, count - 2 * (tile + 1));
+        const int nsub = tile < 0 ? next_subs : 2 * tile + 1 < count ? 2 : 1;
+        for (int e = 0; e < 9 && tile >= 0 && ok; ++e)
+          for (int s = 0; s < nsub && ok; ++s) {
+            ok = store(L::kBarTapeRdy, rdy_phase[s], &maps.tape[0], tile, s, 0, acts_offset(e) / 64);
+            rdy_phase[s] ^= 1u;
+            if (ok) mbar_arrive(sbase + L::kBarTapeDone + 8 * s);
+          }
+        for (int s = 0; s < nsub && ok; ++s) {
+          if (tile >= 0)
+            ok = store(L::kBarTapeTail, (uint32_t)(tile & 1), &maps.tape[2], tile, s, 1, kActsEncDir / 64);
+          if (ok && s < next_subs) {
+            ok = store(L::kBarTapeEnc, (uint32_t)((tile + 1) & 1), &maps.tape[1], tile + 1, s, 0, 0);
+            if (ok) mbar_arrive(sbase + L::kBarTapeDone + 8 * s);
           }
         }
       }
       bulk_wait_all();  // no store still reads this CTA's shared memory or writes the tape
     }
-  } else {
-    // ---------------- epilogue warps ----------------
-    // All epilogue warps serve whichever sub-tile's accumulator is ready (A,
-    // then B, every layer). Warp w reads TMEM lane quadrant qd = w % 4 (rows
-    // 32*qd ..) and column part cq: kCols columns (half as many of dense_9's
-    // 128); the heads' sums over the parts meet in one warp per quadrant.
-    // (Nothing here may spill: the 28 KB of L1 beside this much shared memory
-    // do not hold spilled registers, and each reload is a trip to L2.)
-    constexpr int kCols = 256 / kParts;
-    const int qd = warp & 3, cq = (warp - 2) >> 2;
-    const int r_ = 32 * qd + lane;  // row within a sub-tile (= TMEM lane)
+  } else if (warp >= kSideWarp && warp < kTapeWarp) {
+    // ---------------- side warps ----------------
+    // One warp per TMEM lane quadrant, a row per lane: the encodings and
+    // dense_9 with the rgb head (model.py:385-386).
+    const int qd = warp & 3, r = 32 * qd + lane;  // row within a sub-tile (= TMEM lane)
     const uint32_t tlane = tmem + ((uint32_t)(32 * qd) << 16);
-    // stmatrix row of this lane in the part's first atom, and its swizzle (store_frag)
-    const uint32_t frag_row = (uint32_t)(32 * qd + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u +
-                              (uint32_t)(cq * kCols * (int)L::kE / 128) * kAtom;
-    const uint32_t cx = (uint32_t)((lane >> 4) ^ (lane & 7));
     const uint32_t enc = sbase + L::kEncOff;
-    // With the tape: a region signalled to the tape writer is not rewritten
-    // before its store has read it (tape_done; at most one pending per
-    // sub-tile, so a parity wait cannot miss a phase).
-    uint32_t tape_pending = 0, tape_phase = 0;  // bit s
-    auto tape_settle = [&](int s) -> bool {
-      if (!STORE || !(tape_pending >> s & 1u)) return true;
-      tape_pending ^= 1u << s;
-      const bool done = __all_sync(0xffffffffu, wait_bar(sbase + L::kBarTapeDone + 8 * s, tape_phase >> s & 1u,
-                                                         abort_flag, err));
-      tape_phase ^= 1u << s;
-      return done;
+    auto arrive_local = [&](uint32_t bar) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
     };
     // One arrival per warp on the even CTA's barrier: what the warp wrote to
     // shared memory is visible to the MMAs that wait for it (and what it read
@@ -654,336 +654,357 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(peer_addr(bar, 0));
     };
-    // The operand of sub-tile s's next layer is written and its accumulator
-    // read (with the tape, also on this CTA's tape_rdy).
-    auto operands_ready = [&](int s) {
-      arrive_even(sbase + L::kBarActr + 8 * s);
-      if (STORE) {
-        if (lane == 0) mbar_arrive(sbase + L::kBarTapeRdy + 8 * s);
-        tape_pending |= 1u << s;
-      }
+    auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, err));
     };
+    // Physical row of a logical row: the row map's entry (without a map the row
+    // itself; the last one for rows past n).
+    auto phys = [&](long long grow) -> long long {
+      const long long g = grow < n ? grow : n - 1;
+      return rm.map ? (long long)NG_IDX(rm.map[g], n_max, kSiteMlpRowMap) : g;
+    };
+    constexpr int kPk = 64 / (F8 ? 4 : 2);
+    const float4 bias9 = ld_here(table + bias_offset(9) + 4 * lane);  // dense_9's of columns 4 lane .. + 3 (BF16)
+        auto from_lane = [](const float4 &v, int src) {
+      return float4{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                    __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src)};
+    };
+    // dense_0's operand of sub-tile s is written and its accumulator read
+    auto start_layer0 = [&](int s) {
+      arrive_even(sbase + L::kBarAct0 + 8 * s);
+      if (STORE && lane == 0) mbar_arrive(sbase + L::kBarTapeEnc + 8 * s);
+    };
+    bool ok = true;
+    // (tile -1 is the first tile's start: the end of its dense_9 alone, so that
+    // there is one copy of the encoding's code)
+#pragma unroll 1
+    for (int tile = -1; tile < ntiles && ok; ++tile) {
+      const uint32_t ph = (uint32_t)(tile & 1);
+      const int next_subs = max(0, min(2, count - 2 * (tile + 1)));  // of the next tile
+      const int nsub = 2 * tile + 1 < count ? 2 : 1;
+      // The encodings in the order that they are due (one copy of the code):
+      // this tile's into E (A's now, as the tile before's dense_9 is done, B's
+      // once A's dense_5 is, then the direction encodings once B's is), then
+      // the next tile's, kept packed until its operand regions are free.
+      uint32_t cur[kPk] = {}, nxt[kPk] = {};
+#pragma unroll 1
+      for (int q = tile < 0 ? 2 : 0; q < 2 + next_subs; ++q) {
+        const int s = q & 1;
+        if (q < nsub || q >= 2) {
+          const long long grow = row_of(tile + (q >> 1), s, r), p = phys(grow);
+          float x[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) x[c] = grow < n ? xyz[p * 3 + c] : 0.0f;
+#pragma unroll
+          for (int i = 0; i < kPk; ++i) cur[i] = nxt[i];
+          encode_row<F8, false>(x, nxt);
+        }
+        if (q < 2) {
+          if (q < nsub) {
+            if (q == 1 && !wait_all(sbase + L::kBarAcc5, ph)) {
+              ok = false;
+              break;
+            }
+            store_chunks(enc, r, 0u, nxt);
+            arrive_even(sbase + (q == 0 ? L::kBarEncA : L::kBarEncB));
+          }
+          if (q == 1) {
+            if (!wait_all(sbase + L::kBarAcc5 + 8 * (nsub - 1), ph)) {
+              ok = false;
+              break;
+            }
+#pragma unroll 1
+            for (int d = 0; d < nsub; ++d) {
+              const long long dr = phys(row_of(tile, d, r)) / rpd;
+              float dir[3];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) dir[c] = dirs[dr * 3 + c];
+              uint32_t pd[kPk / 2];
+              encode_row<F8, true>(dir, pd);
+              store_chunks(enc, r, (uint32_t)(4 * d), pd);
+            }
+            arrive_even(sbase + L::kBarDir);
+          }
+        } else if (tile < 0) {
+          store_chunks(sbase + L::kActOff + s * L::kActBytes, r, 0u, nxt);
+          start_layer0(s);
+        }
+      }
+      if (tile < 0) continue;
+      if (!ok) break;
+      if (next_subs == 1) {
+#pragma unroll
+        for (int i = 0; i < kPk; ++i) cur[i] = nxt[i];
+      }
+#pragma unroll 1
+      for (int s = 0; s < nsub; ++s) {
+        const uint32_t act = sbase + L::kActOff + s * L::kActBytes;
+        // dense_9 is done (with the tape: and h8 stored, the last of the tile's ten regions)
+        if (!wait_all(sbase + L::kBarAcc9 + 8 * s, ph) || (STORE && !wait_all(sbase + L::kBarTapeDone + 8 * s, 1u)) ||
+            !wait_all(sbase + L::kBarSig + 8 * s, ph)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (s < next_subs) store_chunks(act, r, 0u, cur);
+#pragma unroll
+        for (int i = 0; i < kPk; ++i) cur[i] = nxt[i];
+        const long long grow = row_of(tile, s, r);
+        const long long p = phys(grow);
+        {
+          const float a = tmem_ld1(tlane + s * 256 + 254), b = tmem_ld1(tlane + s * 256 + 255);
+          if (grow < n) sigma_out[p] = fmaxf((a + b) + table[kSigmaBOff], 0.0f);
+        }
+        // rgb = sigmoid(h9 . W + b) in FP32. BF16: ((q0 + q1) + (q2 + q3)) of the
+        // quarters' sums of 32 columns; FP8: the 128 columns in order.
+        float rgb[3] = {0.f, 0.f, 0.f}, half[3] = {0.f, 0.f, 0.f};
+        uint32_t ra[16], rb[16];
+        tmem_ld16(tlane + s * 256, ra);
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          float acc[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) acc[c] = F8 ? rgb[c] : 0.0f;
+          uint32_t h9[16];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            // 16 columns, the next 16 on their way
+            uint32_t(&raw)[16] = k == 0 ? ra : rb;
+            const int col = 32 * j + 16 * k;
+            tmem_wait16(raw);
+            if (k == 0)
+              tmem_ld16(tlane + s * 256 + col + 16, rb);
+            else if (j < 3)
+              tmem_ld16(tlane + s * 256 + col + 16, ra);
+            else if (s < next_subs)
+              start_layer0(s);  // the accumulator is read
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 b4 = F8 ? lds_here(sbase + L::kHeadB + 4 * (col + i)) : from_lane(bias9, (col + i) / 4);
+              float v[4];
+              if (F8) {
+                const float4 s4 = lds_here(sbase + L::kHeadB + 512 + 4 * (col + i));
+                fma_f32x2(v[0], v[1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), s4.x, s4.y, b4.x, b4.y);
+                fma_f32x2(v[2], v[3], __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]), s4.z, s4.w, b4.z, b4.w);
+              } else {
+                add_f32x2(v[0], v[1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), b4.x, b4.y);
+                add_f32x2(v[2], v[3], __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]), b4.z, b4.w);
+              }
+              // rows col + i .. + 3 of the [128][3] rgb kernel: 12 floats
+              const uint32_t wr = sbase + L::kHeadW + 1024 + (col + i) * 12;
+              const float4 a4 = lds_here(wr), c4 = lds_here(wr + 16), e4 = lds_here(wr + 32);
+              const float w12[12] = {a4.x, a4.y, a4.z, a4.w, c4.x, c4.y, c4.z, c4.w, e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float h = fmaxf(v[q], 0.0f);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[c] = fmaf(h, w12[3 * q + c], acc[c]);
+              }
+              if (STORE) {
+                h9[8 * k + i / 2] = pack_bf16_relu(v[0], v[1]);
+                h9[8 * k + i / 2 + 1] = pack_bf16_relu(v[2], v[3]);
+              }
+            }
+          }
+          if (F8) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) rgb[c] = acc[c];
+          } else if (j & 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              half[c] += acc[c];
+              rgb[c] = j == 1 ? half[c] : rgb[c] + half[c];
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) half[c] = acc[c];
+          }
+          if (STORE) {
+            // h9's columns as columns 32 + 32j .. of [enc_dir | h9] in the region's atoms 1, 2
+            if (j < 3)
+              store_chunks(act + kAtom * (1u + (uint32_t)(j + 1) / 2), r, (uint32_t)(((j + 1) & 1) * 4), h9);
+            else if (grow < n)
+              tape_store32(tape + grow * kActsLd + acts_offset(9) + 96, h9);
+          }
+        }
+        if (STORE) {
+          // enc_dir beside h9, then the tail goes to the tape
+          uint32_t u[16];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            ld_shared_v4(enc + (uint32_t)r * 128u + (((uint32_t)(4 * s + i) ^ ((uint32_t)r & 7u)) << 4), u[4 * i],
+                         u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+          store_chunks(act + kAtom, r, 0u, u);
+          fence_proxy_async();
+          arrive_local(sbase + L::kBarTapeTail + 8 * s);
+        }
+        if (grow < n) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) rgb_out[p * 3 + c] = 1.0f / (1.0f + expf(-(rgb[c] + table[kRgbBOff + c])));
+        }
+      }
+    }
+  } else {
+    // ---------------- epilogue warps ----------------
+    // All eight warps serve whichever sub-tile's accumulator is ready (A, then
+    // B, every layer but dense_9). Warp w reads TMEM lane quadrant qd = w % 4
+    // (rows 32*qd ..) and column part cq: kCols columns. (Nothing here may
+    // spill: the 28 KB of L1 beside this much shared memory do not hold
+    // spilled registers, and each reload is a trip to L2.)
+    constexpr int kCols = 256 / kParts;
+    const int qd = warp & 3, cq = (warp - 2) >> 2;
+    const uint32_t tlane = tmem + ((uint32_t)(32 * qd) << 16);
+    // stmatrix row of this lane in the part's first atom, and its swizzle (store_frag)
+    const uint32_t frag_row = (uint32_t)(32 * qd + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u +
+                              (uint32_t)(cq * kCols * (int)L::kE / 128) * kAtom;
+    const uint32_t cx = (uint32_t)((lane >> 4) ^ (lane & 7));
     auto arrive_local = [&](uint32_t bar) {
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    // Physical row of a logical row: the row map's entry (0 without a map), and
-    // the row itself (the last one for rows past n).
-    auto map_row = [&](long long grow) -> int {
-      return rm.map ? (int)NG_IDX(rm.map[grow < n ? grow : n - 1], n_max, kSiteMlpRowMap) : 0;
-    };
-    auto phys = [&](long long grow, int mapped) -> long long {
-      return rm.map ? (long long)mapped : grow < n ? grow : n - 1;
-    };
-    // The sub-tiles' points, A's and B's (selected by s, so that one copy of
-    // the code serves both); after layer 5 the next tile's (its mapped row
-    // first, kept in x[0]).
-    constexpr int kPk = 64 / kParts / (F8 ? 4 : 2);
-    float x0[3], x1[3];
-    auto load_row = [&](int k, int s, int r) {
-      const float m = __int_as_float(map_row(row_of(k, s, r)));
-      if (s == 0)
-        x0[0] = m;
-      else
-        x1[0] = m;
-    };
-    auto load_x = [&](int k, int s, int r) {
-      const long long grow = row_of(k, s, r), p = phys(grow, __float_as_int(s == 0 ? x0[0] : x1[0]));
-      const bool v = grow < n;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float x = v ? xyz[p * 3 + c] : 0.0f;
-        if (s == 0)
-          x0[c] = x;
-        else
-          x1[c] = x;
-      }
-    };
-    auto encode = [&](int s, uint32_t (&pk)[kPk]) {
-      float x[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = s == 0 ? x0[c] : x1[c];
-      encode_any<F8, false>(cq, x, pk);
-    };
-    auto store_enc = [&](uint32_t atom, int r, const uint32_t (&pk)[kPk]) {
-      store_chunks(atom, r, (uint32_t)(cq * (kPk / 4)), pk);
-    };
-    float sig0 = 0.0f, sig1 = 0.0f;  // the sigma head's half sums
-    uint32_t accf_phase = 0;  // both sub-tiles' accumulator barriers, per layer
+    float sig0 = 0.0f, sig1 = 0.0f;  // the sigma head's part sums
+    uint32_t accf_phase = 0;         // both sub-tiles' accumulator barriers, per layer
     bool ok = true;
-#pragma unroll 1
-    for (int s = 0; s < min(2, count); ++s) {
-      load_row(0, s, r_);
-      load_x(0, s, r_);
-      uint32_t pk[kPk];
-      encode(s, pk);
-      store_enc(sbase + L::kActOff + s * L::kActBytes, r_, pk);
-      operands_ready(s);
-    }
 #pragma unroll 1
     for (int tile = 0; tile < ntiles && ok; ++tile) {
       const int nsub = 2 * tile + 1 < count ? 2 : 1;
-      const int next_subs = min(2, count - 2 * (tile + 1));  // of the next tile (<= 0: none)
 #pragma unroll 1
-      for (int g = 0; g < kNumGemm && ok; ++g) {
-        const float *bias = table + bias_offset(g);
+      for (int g = 0; g < 9 && ok; ++g) {
 #pragma unroll 1
         for (int s = 0; s < nsub; ++s) {
-          const uint32_t act = sbase + L::kActOff + s * L::kActBytes;
-          // (opaque, so that addresses derived from it are not hoisted out of the loops into registers)
-          int r = r_;
-          asm volatile("" : "+r"(r));
-          // While the accumulator is computed: the first biases, and the
-          // encodings that take the place of what its MMAs read (the next
-          // tile's dense_0 operand, B's dense_5 encoding).
+          // the first biases, while the accumulator is computed
           FragBias<F8> fb[2];
-          const float *fbias = bias + kCols * cq, *fscale = scales + bias_offset(g) + kCols * cq;
-          if (g != 9) {
-            fb[0].load(fbias, fscale, lane & 3);
-            fb[1].load(fbias + 32, fscale + 32, lane & 3);
+          const float *fbias = table + bias_offset(g) + kCols * cq, *fscale = scales + bias_offset(g) + kCols * cq;
+          fb[0].load(fbias, fscale, lane & 3);
+          fb[1].load(fbias + 32, fscale + 32, lane & 3);
+          bool got = wait_bar(sbase + L::kBarAccf + 8 * s, accf_phase, abort_flag, err);
+          if (STORE && got) {
+            // the tape has what the region held: enc_xyz for g = 0 (of the ten
+            // regions of a tile, the side warps wait for the last, h8)
+            got = wait_bar(sbase + L::kBarTapeDone + 8 * s, (uint32_t)(g & 1), abort_flag, err);
           }
-          const bool start_next = g == 9 && s < next_subs, enc_b = g == 5 && s == 0 && nsub == 2;
-          uint32_t pk[kPk];
-          if (start_next || enc_b) encode(enc_b ? 1 : s, pk);
           // warp-uniform outcome, so that the warp leaves together
-          if (!__all_sync(0xffffffffu, wait_bar(sbase + L::kBarAccf + 8 * s, accf_phase, abort_flag, err))) {
+          if (!__all_sync(0xffffffffu, got)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          // the sub-tile's region is rewritten below once the tape has it
-          // and, for h0, once the rgb partials of the tile before are read
-          if (!tape_settle(s) ||
-              (g == 0 && tile > 0 &&
-               !__all_sync(0xffffffffu, wait_bar(sbase + L::kBarFree + 8 * s, (uint32_t)(tile & 1) ^ 1u, abort_flag, err)))) {
-            ok = false;
-            break;
-          }
-          if (enc_b) {
-            // A's dense_5 is done with E: B's encoding for the end of its dense_5
-            store_enc(enc, r, pk);
-            arrive_even(sbase + L::kBarEncB);
-          }
-          if (g != 9) {
-            // 16 rows x 32 columns at a time, each loaded while the one before
-            // is stored (dense_8 is linear, model.py:377-378)
-            const uint32_t fr = act + frag_row, ta = tlane + s * 256 + kCols * cq;
-            if (!F8 && g != 7) {
-              uint32_t ra[32], rb[32];
-              tmem_ld_frag64(ta, ra);
+          // 16 rows x 64 (or 32) columns at a time, each loaded while the one
+          // before is stored (dense_8 is linear, model.py:377-378)
+          const uint32_t fr = sbase + L::kActOff + s * L::kActBytes + frag_row, ta = tlane + s * 256 + kCols * cq;
+          if (!F8 && g != 7) {
+            uint32_t ra[32], rb[32];
+            tmem_ld_frag64(ta, ra);
 #pragma unroll
-              for (int c = 0; c < 2; ++c) {
-                const uint32_t dst = fr + (uint32_t)c * kAtom;
-                tmem_wait32(ra);
-                tmem_ld_frag64(ta + (16u << 16) + 64 * c, rb);
-                store_frag64<F8>(dst, cx, 0u, ra, fb, g != 8);
-                tmem_wait32(rb);
-                if (c == 0) tmem_ld_frag64(ta + 64, ra);
-                store_frag64<F8>(dst + 16 * 128, cx, 0u, rb, fb, g != 8);
-                if (c == 0) {
-                  fb[0].load(fbias + 64, fscale + 64, lane & 3);
-                  fb[1].load(fbias + 96, fscale + 96, lane & 3);
-                }
+            for (int c = 0; c < 2; ++c) {
+              const uint32_t dst = fr + (uint32_t)c * kAtom;
+              tmem_wait32(ra);
+              tmem_ld_frag64(ta + (16u << 16) + 64 * c, rb);
+              store_frag64<F8>(dst, cx, 0u, ra, fb, g != 8);
+              tmem_wait32(rb);
+              if (c == 0) tmem_ld_frag64(ta + 64, ra);
+              store_frag64<F8>(dst + 16 * 128, cx, 0u, rb, fb, g != 8);
+              if (c == 0) {
+                fb[0].load(fbias + 64, fscale + 64, lane & 3);
+                fb[1].load(fbias + 96, fscale + 96, lane & 3);
               }
-            } else if (g != 7) {
-              uint32_t ra[16], rb[16];
-              tmem_ld_frag32(ta, ra);
+            }
+          } else if (g != 7) {
+            uint32_t ra[16], rb[16];
+            tmem_ld_frag32(ta, ra);
 #pragma unroll
-              for (int c = 0; c < kCols / 32; ++c) {
-                const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
-                tmem_wait16(ra);
-                tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
-                store_frag<F8, false>(dst, cx, ch, ra, fb[c % 2], g != 8);
-                tmem_wait16(rb);
-                if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
-                store_frag<F8, false>(dst + 16 * 128, cx, ch, rb, fb[c % 2], g != 8);
-                if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
-              }
-            } else {
-              // dense_7: the same, and its FP32 ReLU goes back to the
-              // accumulator, from where the sigma head (model.py:374-375)
-              // reads it a row per lane
-              uint32_t ra[16], rb[16];
-              tmem_ld_frag32(ta, ra);
+            for (int c = 0; c < kCols / 32; ++c) {
+              const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
+              tmem_wait16(ra);
+              tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
+              store_frag<F8, false>(dst, cx, ch, ra, fb[c % 2], g != 8);
+              tmem_wait16(rb);
+              if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
+              store_frag<F8, false>(dst + 16 * 128, cx, ch, rb, fb[c % 2], g != 8);
+              if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
+            }
+          } else {
+            // dense_7: the same, and its FP32 ReLU goes back to the
+            // accumulator, from where the sigma head (model.py:374-375)
+            // reads it a row per lane
+            uint32_t ra[16], rb[16];
+            tmem_ld_frag32(ta, ra);
 #pragma unroll
-              for (int c = 0; c < kCols / 32; ++c) {
-                const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
-                tmem_wait16(ra);
-                tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
-                store_frag<F8, true>(dst, cx, ch, ra, fb[c % 2], true);
-                tmem_st_frag32(ta + 32 * c, ra);
-                tmem_wait16(rb);
-                if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
-                store_frag<F8, true>(dst + 16 * 128, cx, ch, rb, fb[c % 2], true);
-                tmem_st_frag32(ta + (16u << 16) + 32 * c, rb);
-                if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
-              }
-              tmem_wait_st();
-              // the head's FP32 sum over the part's columns, in order (BF16:
-              // as two sums of 64)
-              const uint32_t sw = sbase + L::kHeadW + 4 * kCols * cq;
-              float part_sum = 0.0f, first = 0.0f;
+            for (int c = 0; c < kCols / 32; ++c) {
+              const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
+              tmem_wait16(ra);
+              tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
+              store_frag<F8, true>(dst, cx, ch, ra, fb[c % 2], true);
+              tmem_st_frag32(ta + 32 * c, ra);
+              tmem_wait16(rb);
+              if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
+              store_frag<F8, true>(dst + 16 * 128, cx, ch, rb, fb[c % 2], true);
+              tmem_st_frag32(ta + (16u << 16) + 32 * c, rb);
+              if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
+            }
+            tmem_wait_st();
+            // the head's FP32 sums: BF16 two of 64 columns each, side by side
+            // and then added, FP8 one over the part's columns in order
+            const uint32_t sw = sbase + L::kHeadW + 4 * kCols * cq;
+            float part_sum = 0.0f, second = 0.0f;
+            // channel i of the 32 at accumulator column fp8_row (BF16: in place)
+            auto add4 = [&](float &sum, const uint32_t(&v)[32], int i, uint32_t w) {
+              const float4 w4 = lds_here(w);
+              sum = fmaf(__uint_as_float(v[F8 ? fp8_row(7, i) : i]), w4.x, sum);
+              sum = fmaf(__uint_as_float(v[F8 ? fp8_row(7, i + 1) : i + 1]), w4.y, sum);
+              sum = fmaf(__uint_as_float(v[F8 ? fp8_row(7, i + 2) : i + 2]), w4.z, sum);
+              sum = fmaf(__uint_as_float(v[F8 ? fp8_row(7, i + 3) : i + 3]), w4.w, sum);
+            };
 #pragma unroll 1
-              for (int c = 0; c < kCols; c += 32) {
-                uint32_t raw[32];
-                tmem_ld32(ta + c, raw);
-                if (!F8 && c == 64) {
-                  first = part_sum;
-                  part_sum = 0.0f;
-                }
-                tmem_wait32(raw);
+            for (int c = 0; c < kCols / 2; c += 32) {
+              const int c0 = F8 ? 2 * c : c, c1 = F8 ? 2 * c + 32 : c + 64;
+              uint32_t raw[2][32];
+              tmem_ld32(ta + c0, raw[0]);
+              tmem_ld32(ta + c1, raw[1]);
+              tmem_wait32(raw[0]);
+              tmem_wait32(raw[1]);
+              if (F8) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) add4(part_sum, raw[0], i, sw + 4 * (c0 + i));
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) add4(part_sum, raw[1], i, sw + 4 * (c1 + i));
+              } else {
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                  const float4 w4 = lds_here(sw + 4 * (c + i));
-                  // channel i of the 32 at accumulator column fp8_row (BF16: in place)
-                  part_sum = fmaf(__uint_as_float(raw[F8 ? fp8_row(7, i) : i]), w4.x, part_sum);
-                  part_sum = fmaf(__uint_as_float(raw[F8 ? fp8_row(7, i + 1) : i + 1]), w4.y, part_sum);
-                  part_sum = fmaf(__uint_as_float(raw[F8 ? fp8_row(7, i + 2) : i + 2]), w4.z, part_sum);
-                  part_sum = fmaf(__uint_as_float(raw[F8 ? fp8_row(7, i + 3) : i + 3]), w4.w, part_sum);
+                  add4(part_sum, raw[0], i, sw + 4 * (c0 + i));
+                  add4(second, raw[1], i, sw + 4 * (c1 + i));
                 }
               }
-              if (!F8) part_sum = first + part_sum;
-              if (s == 0)
-                sig0 = part_sum;
-              else
-                sig1 = part_sum;
             }
-            operands_ready(s);
-          } else {
-            // dense_9 and the rgb head (model.py:385-386), a row per lane
-            const int colh = kCols / 2 * cq;
-            const long long grow = row_of(tile, s, r);
-            float sig_half = 0.0f;
-            if (cq == 0) {
-              if (!__all_sync(0xffffffffu, wait_bar(sbase + L::kBarSig + 8 * s, (uint32_t)(tile & 1), abort_flag, err))) {
-                ok = false;
-                break;
-              }
-              tc_fence_after();
-              sig_half = tmem_ld1(tlane + s * 256 + 255);
-            }
-            constexpr int kPieces = kCols / 64;  // 32 columns each
-            uint32_t raw[kPieces][32];
-#pragma unroll
-            for (int j = 0; j < kPieces; ++j) tmem_ld32(tlane + s * 256 + colh + 32 * j, raw[j]);
-#pragma unroll
-            for (int j = 0; j < kPieces; ++j) tmem_wait32(raw[j]);
-            if (start_next) {
-              // the accumulator is read and the activation region idle: dense_0 of the next tile may start
-              store_enc(act, r, pk);
-              operands_ready(s);
-            }
-            if (cq == 0 && grow < n)
-              sigma_out[phys(grow, map_row(grow))] =
-                  fmaxf(((s == 0 ? sig0 : sig1) + sig_half) + table[kSigmaBOff], 0.0f);
-            // rgb = sigmoid(h9 . W + b) in FP32. BF16: sums of quarters of 32
-            // columns, two per warp, the second half's added by the first's
-            // warp. FP8: the 128 columns in order, the second half's warp going
-            // on from the first's sum. part: what the finishing warp (cq ==
-            // last) takes over.
-            constexpr int last = F8 ? 1 : 0;
-            float *part = reinterpret_cast<float *>(smem + L::kActOff + s * L::kActBytes + L::kRgbPart);
-            float rgb[3] = {0.f, 0.f, 0.f};
-            if (F8 && cq == last) {
-              if (!__all_sync(0xffffffffu, wait_bar(sbase + L::kBarRgb + 8 * s, (uint32_t)(tile & 1), abort_flag, err))) {
-                ok = false;
-                break;
-              }
-#pragma unroll
-              for (int c = 0; c < 3; ++c) rgb[c] = part[c * 128 + r];
-            }
-#pragma unroll
-            for (int j = 0; j < kPieces; ++j) {
-              const int col0 = colh + 32 * j;
-              float v[32];
-              row_bias<F8>(raw[j], bias + col0, scales + bias_offset(9) + col0, v);
-              if (STORE) {
-                // h9's columns as columns 32 + col0 .. of [enc_dir | h9] in the region's atoms 1, 2
-                uint32_t u[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) u[i] = pack_bf16_relu(v[2 * i], v[2 * i + 1]);
-                if (col0 < 96)
-                  store_chunks(act + kAtom * (1u + (uint32_t)(32 + col0) / 64), r, (uint32_t)((32 + col0) % 64) / 8, u);
-                else if (grow < n)
-                  tape_store32(tape + grow * kActsLd + acts_offset(9) + col0, u);
-              }
-              float acc[3];
-#pragma unroll
-              for (int c = 0; c < 3; ++c) acc[c] = F8 ? rgb[c] : 0.0f;
-#pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                // rows col0+i .. col0+i+3 of the [128][3] rgb kernel: 12 floats
-                const uint32_t wr = sbase + L::kHeadW + 1024 + (col0 + i) * 12;
-                const float4 a4 = lds_here(wr), b4 = lds_here(wr + 16), c4 = lds_here(wr + 32);
-                const float w12[12] = {a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const float h = fmaxf(v[i + q], 0.0f);
-                  acc[0] = fmaf(h, w12[3 * q], acc[0]);
-                  acc[1] = fmaf(h, w12[3 * q + 1], acc[1]);
-                  acc[2] = fmaf(h, w12[3 * q + 2], acc[2]);
-                }
-              }
-#pragma unroll
-              for (int c = 0; c < 3; ++c) rgb[c] = F8 || j == 0 ? acc[c] : rgb[c] + acc[c];
-            }
-            if (STORE) {
-              // this part's enc_dir columns beside h9, then the tail goes to the tape
-              uint32_t u[8];
-#pragma unroll
-              for (int i = 0; i < 2; ++i)
-                ld_shared_v4(enc + (uint32_t)r * 128u + (((uint32_t)(4 * s + 2 * cq + i) ^ ((uint32_t)r & 7u)) << 4),
-                             u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
-              store_chunks(act + kAtom, r, (uint32_t)(2 * cq), u);
-              fence_proxy_async();
-              arrive_local(sbase + L::kBarTapeTail + 8 * s);
-            }
-            if (cq != last) {
-#pragma unroll
-              for (int c = 0; c < 3; ++c) part[c * 128 + r] = rgb[c];
-              arrive_local(sbase + L::kBarRgb + 8 * s);
-            } else {
-              if (!F8) {
-                if (!__all_sync(0xffffffffu, wait_bar(sbase + L::kBarRgb + 8 * s, (uint32_t)(tile & 1), abort_flag, err))) {
-                  ok = false;
-                  break;
-                }
-#pragma unroll
-                for (int c = 0; c < 3; ++c) rgb[c] += part[c * 128 + r];
-              }
-              arrive_local(sbase + L::kBarFree + 8 * s);
-              if (grow < n) {
-                const long long p = phys(grow, map_row(grow));
-#pragma unroll
-                for (int c = 0; c < 3; ++c) rgb_out[p * 3 + c] = 1.0f / (1.0f + expf(-(rgb[c] + table[kRgbBOff + c])));
-              }
-            }
+            if (!F8) part_sum += second;
+            if (s == 0)
+              sig0 = part_sum;
+            else
+              sig1 = part_sum;
           }
-          // Behind the signals: what later layers need.
-          if (g == 0 && s == 0) {
-            // E (last read by the tile before's dense_9): A's encoding for dense_5
-            encode(0, pk);
-            store_enc(enc, r, pk);
-          } else if (g == 6) {
-            // dense_5 is done with E: the direction encodings for dense_9
-            const long long grow = row_of(tile, s, r);
-            const long long dr = phys(grow, map_row(grow)) / rpd;
-            float d[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) d[c] = dirs[dr * 3 + c];
-            uint32_t pd[kPk / 2];
-            encode_any<F8, true>(cq, d, pd);
-            store_chunks(enc, r, (uint32_t)(4 * s + cq * (kPk / 8)), pd);
-            if (s < next_subs) load_row(tile + 1, s, r);
-          } else if (g == 7) {
-            if (s < next_subs) load_x(tile + 1, s, r);
-          } else if (g == 8 && cq == 1) {
-            // the second half's sigma sum to the first's warp, in a column of
-            // the accumulator that dense_9 does not write
-            tmem_st1(tlane + s * 256 + 255, s == 0 ? sig0 : sig1);
+          // the operand of the sub-tile's next layer is written and its
+          // accumulator read: one arrival per warp on the even CTA's barrier
+          fence_proxy_async();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive_remote(peer_addr(sbase + L::kBarActr + 8 * s, 0));
+            if (STORE) mbar_arrive(sbase + L::kBarTapeRdy + 8 * s);
+          }
+          if (g == 8) {
+            // sigma's part sums to the side warps, in columns 254 and 255 of the
+            // accumulator, which dense_9 does not write: the second part's own,
+            // so the first part's warp waits until they have been read
+            if (cq == 0 && !__all_sync(0xffffffffu, wait_bar(sbase + L::kBarRead8 + 8 * s, (uint32_t)(tile & 1),
+                                                             abort_flag, err))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            tmem_st1(tlane + s * 256 + 254 + cq, s == 0 ? sig0 : sig1);
             tmem_wait_st();
             tc_fence_before();
-            arrive_local(sbase + L::kBarSig + 8 * s);
+            arrive_local(sbase + (cq == 0 ? L::kBarSig : L::kBarRead8) + 8 * s);
           }
         }
         accf_phase ^= 1;

@@ -57,3 +57,24 @@ def test_counts_around_the_subtiles(ng, oracle, cuda, precision):
     tol = {"bf16": 2e-3, "fp8": 3e-2}[precision]
     assert np.abs(rgb[:600].cpu().numpy() - want_rgb).max() < tol
     assert np.abs(sig[:600].cpu().numpy() - want_sig).max() < tol * max(1.0, float(np.abs(want_sig).max()))
+
+
+def test_fp8_relu_of_not_a_number(ng, cuda):
+    """ReLU on packed E4M3 words is max(x, 0) of the FP32 value, NaN included
+    (fmaxf(NaN, 0) = 0): rows with a NaN coordinate give what a zero dense_0
+    and dense_5 give, finite and the same for each such row of one direction,
+    and leave the other rows alone."""
+    x, d = _points(600, 32)
+    X, D = torch.from_numpy(x).cuda(), torch.from_numpy(np.repeat(d[:1], 600, 0)).cuda()
+    mlp = ng.get_coarse_or_fine_model("fine", params=ng.weights.glorot_blob(8), precision="fp8")
+    rgb, sig = mlp((X, D))
+    bad = torch.tensor([0, 3, 127, 128, 300, 599], device="cuda")
+    Y = X.clone()
+    Y[bad, torch.arange(6, device="cuda") % 3] = float("nan")
+    r, s = mlp((Y, D))
+    mlp.check_device_errors()
+    keep = torch.ones(600, dtype=torch.bool, device="cuda")
+    keep[bad] = False
+    assert torch.equal(r[keep], rgb[keep]) and torch.equal(s[keep], sig[keep])
+    assert bool(torch.isfinite(r[bad]).all()) and bool(torch.isfinite(s[bad]).all())
+    assert bool((r[bad] == r[bad[0]]).all()) and bool((s[bad] == s[bad[0]]).all())
