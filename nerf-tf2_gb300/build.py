@@ -18,7 +18,7 @@ CSRC = HERE / "csrc"
 INCLUDE = ROOT / "include"
 BUILD = HERE / "_build"
 LIB = HERE / "libnerfgb.so"
-SOURCES = ["ray_ops.cu", "mlp.cu", "mlp_tc.cu", "mlp_bwd_tc.cu", "gemm_tc.cu", "render.cu", "render_noalloc.cu", "train.cu",
+SOURCES = ["ray_ops.cu", "mlp.cu", "mlp_tc.cu", "mlp_bwd_tc.cu", "gemm_tc.cu", "gemm_fp32_tc.cu", "render.cu", "render_noalloc.cu", "train.cu",
            "proposal.cu", "mlp_train.cu", "mlp_train_bf16.cu", "gate.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

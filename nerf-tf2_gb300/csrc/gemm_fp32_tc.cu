@@ -1,0 +1,469 @@
+// FP32 weight gradients of the MLP backward on the tensor cores (the gradient
+// tf.GradientTape takes at nerf/core/model.py:148-170 through the Dense
+// layers of model.py:366-387): for every layer
+//
+//   dW[k][n] += sum_m In[m][k] dZ[m][n],   db[n] += sum_m dZ[m][n]
+//
+// in FP32 accuracy from BF16 products. An FP32 value is exactly the sum of
+// three BF16 values, its 24 significant bits cut into three groups of eight
+// (x = x0 + x1 + x2, each group's exponent its own); of the nine products of
+// two such sums the six largest are taken (x0 y0, x0 y1, x1 y0, x1 y1, x0 y2,
+// x2 y0: what is left out is below 2^-24 of the product), smallest first, in
+// FP32 accumulators in TMEM. The tensor core's FP32 accumulation truncates, so
+// an accumulator takes only the 64 rows of one stage (four accumulations at
+// full magnitude) and the stages' sums are added in registers with rounding:
+// closer to the exact sum than one chain of FMAs over a slice of rows was (the
+// gradient of 5,000 rows 2.9e-7 from 64-bit arithmetic, against 8.1e-7).
+//
+// Six BF16 products are still four to five times the rate of the FP32 FMA
+// pipe, which bound the kernel before: 6.2 ms of a 1,024-ray step's two
+// networks (262,144 rows), 2.1 here. A 64-row stage takes ~6k cycles, 3,072 of
+// them MMAs; the conversion bounds it (~3.5k cycles of its eight warps; four
+// warps took 7k, a stage 12.7k with the MMAs issued by one of them).
+//
+// CTAs run as cluster pairs (tcgen05.mma.cta_group::2, M = 256): each CTA
+// converts its half of either operand's columns, the even CTA issues. Both operands
+// are MN-major (the reduction runs along the rows) in the 128-byte swizzled
+// layout (gemm_tc.cu): 64-column atoms of 64 rows x 128 bytes.
+//
+// Warp roles (16 warps): 0-7 add each stage's accumulator to the item's sums,
+// 128 registers per thread, and at the item's end add those to the gradient;
+// 8-15 convert, with rows fetched into L2 ahead of them. Thread 0 of the even
+// CTA issues a stage's MMAs before it adds the stage before. The warp groups
+// trade registers (setmaxnreg): 168 for the sums, 88 for the conversion.
+//
+// Every mbarrier wait is bounded (tc::wait_bar): on a timeout every role
+// stops, the issuer drains its MMAs, TMEM is freed and the CTA writes NaN into
+// every layer's gradient.
+#include <stdint.h>
+
+#include <mutex>
+#include <unordered_map>
+
+#include "common.cuh"
+#include "mlp_internal.cuh"
+#include "tcgen05.cuh"
+
+namespace nerfgb {
+namespace split {
+
+using namespace tc;
+
+constexpr int kRows = 64;  // rows (K) per stage
+constexpr int kAhead = 4;  // stages fetched into L2 ahead of the one converted
+constexpr int kSumWarps = 8, kConvWarps = 8, kThreads = 32 * (kSumWarps + kConvWarps);
+// Registers of the two kinds of warp group (the block is launched with 128 a thread).
+constexpr int kSumRegs = 168, kConvRegs = 88;
+static_assert(kSumRegs * kSumWarps + kConvRegs * kConvWarps <= 128 * (kSumWarps + kConvWarps), "the launch's registers");
+constexpr uint32_t kAtomBytes = 64 * 128;        // 64 columns x 64 rows
+constexpr uint32_t kPart = 2 * kAtomBytes;       // one BF16 part of 128 columns
+constexpr uint32_t kOperand = 3 * kPart;
+constexpr uint32_t kStage = 2 * kOperand;        // A, B
+constexpr uint32_t kBar0 = 2 * kStage;
+constexpr uint32_t kBarFull = kBar0;             // [2] operands of the stage written (both CTAs)
+constexpr uint32_t kBarDone = kBar0 + 16;        // [2] its MMAs are complete: stage free, accumulator full
+constexpr uint32_t kBarRead = kBar0 + 32;        // [2] its accumulator has been read (both CTAs)
+constexpr uint32_t kBarDrain = kBar0 + 48;
+constexpr uint32_t kTmemSlot = kBar0 + 56;
+constexpr uint32_t kAbort = kBar0 + 64;          // int, then the wait limit (u64) at +8
+constexpr uint32_t kErr = kBar0 + 80;            // int
+constexpr uint32_t kSmem = kBar0 + 96;
+static_assert(kSmem <= 227 * 1024, "two stages");
+
+// One product. Plain: A = the tape's columns col .. col + 255 (the layer's
+// input), B = the dZ of `slot` (N columns). Flipped (inputs of fewer than 64
+// columns, K): A = the dZ of `slot` (M columns), B = the tape's columns col ..
+// col + 127, of which the first K count; the result is transposed.
+struct Job {
+  int col, slot, K, N, flat, k_dst0;
+  bool flip, bias;
+  __host__ __device__ constexpr int n_mma() const { return flip ? 128 : N; }
+  // a stage's cost in units of a quarter of 256 columns' (the conversion bounds the narrow ones)
+  __host__ __device__ constexpr int cost() const { return n_mma() == 256 ? 4 : 3; }
+};
+constexpr int kJobs = 12;
+__host__ __device__ constexpr Job job_of(int j) {
+  return j == 0   ? Job{acts_offset(8), 9, 256, 128, 10, 0, false, true}
+         : j == 1 ? Job{kActsEncDir, 9, 27, 128, 10, 256, true, false}
+         : j == 2 ? Job{acts_offset(7), 8, 256, 256, 9, 0, false, true}
+         : j == 3 ? Job{kActsEncXyz, 5, 63, 256, 5, 256, true, false}
+         : j == 4 ? Job{kActsEncXyz, 0, 63, 256, 0, 0, true, true}
+                  : Job{acts_offset(j - 5), j - 4, 256, 256, j - 4, 0, false, true};  // dense_1 .. dense_7
+}
+static_assert(kActsEncDir + 128 <= kActsLd && kActsLd % 4 == 0, "flipped inputs stay inside the row");
+constexpr int cost_sum() {
+  int c = 0;
+  for (int j = 0; j < kJobs; ++j) c += job_of(j).cost();
+  return c;
+}
+
+// A pair's stages of job j (every job has `stages`): all jobs' stages in order,
+// each at the sum of the costs before it, are dealt evenly by cost.
+__device__ __forceinline__ void stages_of(int j, int stages, int pair, int pairs, int &b, int &e) {
+  long long at = 0;
+  for (int i = 0; i < j; ++i) at += (long long)job_of(i).cost() * stages;
+  const long long all = (long long)cost_sum() * stages, w = job_of(j).cost();
+  const long long lo = pair * all / pairs - at, hi = (pair + 1) * all / pairs - at;
+  b = lo <= 0 ? 0 : (int)((lo + w - 1) / w < stages ? (lo + w - 1) / w : stages);
+  e = hi <= 0 ? 0 : (int)((hi + w - 1) / w < stages ? (hi + w - 1) / w : stages);
+}
+
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kAtomBytes >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
+}
+
+// The upper halves of two words (BF16 by truncation) as one word.
+__device__ __forceinline__ uint32_t upper(float lo, float hi) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(d) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+  return d;
+}
+__device__ __forceinline__ float head(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+
+// Eight values of a row to the three parts' 16-byte chunks at dst.
+__device__ __forceinline__ void split_store(const float4 &u, const float4 &v, uint32_t dst) {
+  const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+  float r[8], q[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[i] = x[i] - head(x[i]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i] = r[i] - head(r[i]);
+  st_shared_v4(dst, upper(x[0], x[1]), upper(x[2], x[3]), upper(x[4], x[5]), upper(x[6], x[7]));
+  st_shared_v4(dst + kPart, upper(r[0], r[1]), upper(r[2], r[3]), upper(r[4], r[5]), upper(r[6], r[7]));
+  st_shared_v4(dst + 2 * kPart, upper(q[0], q[1]), upper(q[2], q[3]), upper(q[4], q[5]), upper(q[6], q[7]));
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+    dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, long long n, float *__restrict__ grads) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_rank();
+  const int pair = (int)cluster_id(), pairs = (int)cluster_count();
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kAbort);
+  int *err = reinterpret_cast<int *>(smem + kErr);
+  // (the swizzled stages need 1024-byte alignment: without it nothing runs)
+  const bool aligned = (sbase & 1023u) == 0;
+  const int stages = aligned ? (int)((n + kRows - 1) / kRows) : 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(sbase + kBarFull + 8 * s, 2 * kConvWarps);
+      mbar_init(sbase + kBarDone + 8 * s, 1);
+      mbar_init(sbase + kBarRead + 8 * s, 2 * kSumWarps);
+    }
+    mbar_init(sbase + kBarDrain, 1);
+    *abort_flag = aligned ? 0 : 1;
+    *err = 0;
+    set_wait_limit(abort_flag, kWaitNs);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kTmemSlot),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
+
+  if (warp >= kSumWarps) {
+    // ---------------- conversion ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kConvRegs));
+    // A lane takes 8 columns (chunk c of an atom) of the rows r + 16u: warps
+    // 0-3 the first atom's, 4-7 the second's.
+    const int w = warp - kSumWarps, c = lane & 7, r = (w & 3) * 4 + (lane >> 3);
+    const int col = (int)crank * 128 + (w >> 2) * 64 + 8 * c;  // within 256 columns
+    const uint32_t dst =
+        sbase + (uint32_t)(w >> 2) * kAtomBytes + (uint32_t)r * 128u + (uint32_t)((c ^ (r & 7)) << 4);
+    bool ok = true;
+    uint32_t q = 0;  // stages so far
+    float4 v[4][2];  // A's four units, each replaced by B's once stored, B's by the next stage's A
+    // The stage's values of operand A and B: this lane's columns start at pa
+    // and pb (nullptr: not needed), `rows` rows from there.
+    const float *pa = nullptr, *pb = nullptr;
+    int rows = 0;
+    auto load = [&](const float *p, int ld, int u) {
+      v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p && r + 16 * u < rows) {
+        const float4 *s = reinterpret_cast<const float4 *>(p + (long long)u * 16 * ld);
+        v[u][0] = __ldg(s);
+        v[u][1] = __ldg(s + 1);
+      }
+    };
+    auto place = [&](const Job &job, int st) {
+      const long long m = (long long)st * kRows + r;
+      const long long left = n - (long long)st * kRows;
+      rows = left < kRows ? (int)left : kRows;
+      const float *z = dz + ((long long)job.slot * n + m) * 256, *t = acts + m * kActsLd + job.col;
+      // B has N / 2 columns in each CTA
+      const int half = job.n_mma() / 2, bc = (w >> 2) * 64 + 8 * c;
+      if (job.flip) {
+        pa = col < job.N ? z + col : nullptr;
+        pb = crank == 0 && bc < 64 ? t + bc : nullptr;
+      } else {
+        pa = t + col;
+        pb = bc < half ? z + (int)crank * half + bc : nullptr;
+      }
+    };
+    // A stage's rows into L2: a lane fetches this CTA's columns of one row of
+    // either operand.
+    auto prefetch = [&](const Job &job, int st) {
+      const int i = w * 32 + lane;
+      if (i >= 128) return;
+      const bool tape = (i < 64) != job.flip;
+      const long long m = (long long)st * kRows + (i & 63);
+      // columns of A in this CTA, then of B
+      const int first = (int)crank * (i < 64 ? 128 : job.flip ? 64 : job.N / 2);
+      const int count = i < 64 ? 128 : job.flip ? 64 : job.N / 2;
+      if (m >= n || (job.flip && (i < 64 ? first >= job.N : crank == 1))) return;
+      const float *src = tape ? acts + m * kActsLd + job.col : dz + ((long long)job.slot * n + m) * 256;
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + first), "r"(count * 4) : "memory");
+    };
+#pragma unroll 1
+    for (int j = 0; j < kJobs && ok; ++j) {
+      const Job job = job_of(j);
+      int sb, se;
+      stages_of(j, stages, pair, pairs, sb, se);
+      if (sb >= se) continue;
+#pragma unroll 1
+      for (int st = sb + 1; st < se && st < sb + kAhead; ++st) prefetch(job, st);
+      const int lda = job.flip ? 256 : kActsLd, ldb = job.flip ? kActsLd : 256;
+      place(job, sb);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) load(pa, lda, u);
+      float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int st = sb; st < se; ++st, ++q) {
+        const int k = (int)(q & 1);
+        if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, (uint32_t)((q >> 1) & 1) ^ 1u, abort_flag, err))) {
+          ok = false;
+          break;
+        }
+        const uint32_t at = dst + (uint32_t)k * kStage;
+        if (st + kAhead < se) prefetch(job, st + kAhead);
+        auto add = [&](int u) {
+          const float4 x = v[u][0], y = v[u][1];
+          sum[0] += x.x; sum[1] += x.y; sum[2] += x.z; sum[3] += x.w;
+          sum[4] += y.x; sum[5] += y.y; sum[6] += y.z; sum[7] += y.w;
+        };
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (pa) {
+            if (job.bias && job.flip) add(u);
+            split_store(v[u][0], v[u][1], at + 2048u * u);
+          }
+          load(pb, ldb, u);
+        }
+        const bool use_b = pb != nullptr;
+        if (st + 1 < se)
+          place(job, st + 1);
+        else
+          pa = nullptr;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (use_b) {
+            if (job.bias && !job.flip) add(u);
+            split_store(v[u][0], v[u][1], at + kOperand + 2048u * u);
+          }
+          load(pa, lda, u);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarFull + 8 * k, 0));
+      }
+      if (job.bias) {
+        // the lanes of a chunk, then the warps (and pairs) by atomics
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 8);
+          sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 16);
+        }
+        const int half = job.n_mma() / 2, bc = (w >> 2) * 64 + 8 * c;
+        if (lane < 8 && (job.flip || bc < half)) {
+          float *db = grads + flat_offset(job.flat) + (long long)flat_in(job.flat) * job.N +
+                      (job.flip ? col : (int)crank * half + bc);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) atomicAdd(db + i, sum[i]);
+        }
+      }
+    }
+  } else {
+    // ---------------- the stages' sums (and the issuer) ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSumRegs));
+    // Warp w: TMEM lane quadrant w % 4 (rows of D), half w / 4 of the columns
+    // that count, as 16 x 32 fragments (tcgen05.cuh).
+    const int qd = warp & 3, h = warp >> 2;
+    const uint32_t tl = tmem + ((uint32_t)(32 * qd) << 16);
+    // The issuer: one thread of the even CTA, a stage ahead of the sums.
+    const bool issuer = crank == 0 && threadIdx.x == 0;
+    int ij = -1, ileft = 0;  // its job, the job's stages left
+    uint32_t iq = 0;
+    if (issuer) {
+      // both CTAs must hold the same TMEM columns (the collective allocation gives them)
+      uint32_t peer_tmem;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(peer_tmem) : "r"(peer_addr(sbase + kTmemSlot, 1))
+                   : "memory");
+      if (peer_tmem != tmem) *abort_flag = 1;
+    }
+    auto issue_next = [&]() {
+      while (ileft == 0) {
+        if (++ij >= kJobs) {
+          ij = kJobs;
+          return;
+        }
+        int b, e;
+        stages_of(ij, stages, pair, pairs, b, e);
+        ileft = e > b ? e - b : 0;
+      }
+      const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
+      --ileft;
+      ++iq;
+      if (!wait_bar(sbase + kBarFull + 8 * k, ph, abort_flag, err) ||
+          !wait_bar(sbase + kBarRead + 8 * k, ph ^ 1u, abort_flag, err))
+        return;
+      tc_fence_after();
+      const uint32_t idesc = idesc_bf16(256, 0) | (1u << 15) | (1u << 16) | ((uint32_t)(job_of(ij).n_mma() >> 3) << 17);
+      const uint32_t sa = sbase + k * kStage, acc = tmem + 256u * k;
+      // the six products, smallest first
+      constexpr int px[6] = {0, 2, 1, 0, 1, 0}, py[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int s = 0; s < kRows / 16; ++s)
+          tc_mma_pair(acc, desc_mn_sw128(sa + px[i] * kPart + 2048u * s),
+                      desc_mn_sw128(sa + kOperand + py[i] * kPart + 2048u * s), idesc, i + s > 0 ? 1u : 0u);
+      tc_commit_pair(sbase + kBarDone + 8 * k);
+    };
+    if (issuer) issue_next();
+    __syncwarp();
+    bool ok = true;
+    uint32_t q = 0;
+#pragma unroll 1
+    for (int j = 0; j < kJobs && ok; ++j) {
+      const Job job = job_of(j);
+      int sb, se;
+      stages_of(j, stages, pair, pairs, sb, se);
+      if (sb >= se) continue;
+      const int cols = (job.flip ? 64 : job.N) / 2, c0 = h * cols;  // 128, 64 or 32
+      float sum[4][2][16];
+#pragma unroll
+      for (int f = 0; f < 8; ++f)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[f / 2][f % 2][i] = 0.0f;
+#pragma unroll 1
+      for (int st = sb; st < se; ++st, ++q) {
+        const int k = (int)(q & 1);
+        if (issuer) issue_next();
+        if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, (uint32_t)((q >> 1) & 1), abort_flag, err))) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int f = 0; f < 8; ++f) {
+          if (32 * (f / 2) < cols) {
+            uint32_t raw[16];
+            tmem_ld_frag32(tl + ((uint32_t)(16 * (f % 2)) << 16) + 256u * k + c0 + 32 * (f / 2), raw);
+            tmem_wait16(raw);
+            float *s = sum[f / 2][f % 2];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2)
+              add_f32x2(s[i], s[i + 1], s[i], s[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarRead + 8 * k, 0));
+      }
+      if (!ok) break;
+      // D's rows are the layer's inputs (flipped: outputs), its columns the outputs (inputs)
+      float *dW = grads + flat_offset(job.flat) + (long long)job.k_dst0 * job.N;
+#pragma unroll
+      for (int f = 0; f < 8; ++f) {
+        if (32 * (f / 2) >= cols) continue;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int row = (int)crank * 128 + 32 * qd + 16 * (f % 2) + lane / 4 + 8 * ((i >> 1) & 1);
+          const int cl = c0 + 32 * (f / 2) + 8 * (i / 4) + 2 * (lane % 4) + (i & 1);
+          if (!job.flip)
+            atomicAdd(dW + (long long)row * job.N + cl, sum[f / 2][f % 2][i]);
+          else if (cl < job.K && row < job.N)
+            atomicAdd(dW + (long long)cl * job.N + row, sum[f / 2][f % 2][i]);
+        }
+      }
+    }
+    if (issuer && stages > 0) {
+      // Drain every MMA issued before TMEM is released (in both CTAs).
+      tc_commit_pair(sbase + kBarDrain);
+      const uint64_t t0 = globaltimer();
+      while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x < 11) grads[flat_offset(threadIdx.x)] = __int_as_float(0x7fffffff);
+  if (crank == 1 && threadIdx.x == 0 && stages > 0) {
+    // the even CTA's MMAs read this CTA's stages: its last commit (after a
+    // timeout of either CTA: for a bounded time)
+    const uint64_t t0 = globaltimer();
+    while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+}  // namespace split
+
+int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t st) {
+  using namespace split;
+  if (n == 0) return NERFGB_OK;
+  if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
+    return NERFGB_E_CUDA;
+  const int sms = num_sms();
+  if (sms <= 0) return NERFGB_E_DEVICE;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  // co-resident pairs, asked once per device (as mlp_tc.cu)
+  static std::mutex mu;
+  static std::unordered_map<int, int> pairs_of_device;
+  int dev = -1, max_pairs;
+  if (cudaGetDevice(&dev) != cudaSuccess) return NERFGB_E_DEVICE;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto hit = pairs_of_device.find(dev);
+    if (hit == pairs_of_device.end()) {
+      cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
+      int m = 0;
+      if (cudaOccupancyMaxActiveClusters(&m, dw_kernel, &cfg) != cudaSuccess) return NERFGB_E_CUDA;
+      hit = pairs_of_device.emplace(dev, m).first;
+    }
+    max_pairs = hit->second;
+  }
+  if (max_pairs < 1) return NERFGB_E_UNSUPPORTED;
+  const long long work = kJobs * ((n + kRows - 1) / kRows), pairs = work < max_pairs ? work : max_pairs;
+  cfg.gridDim = dim3((unsigned)(2 * pairs));
+  if (cudaLaunchKernelEx(&cfg, dw_kernel, acts, dz, n, grads) != cudaSuccess) return NERFGB_E_CUDA;
+  return launch_status();
+}
+
+}  // namespace nerfgb

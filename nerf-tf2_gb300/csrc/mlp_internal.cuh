@@ -62,6 +62,11 @@ int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t st
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
                      __nv_bfloat16 *dz, float *grads, int *err, cudaStream_t stream);
 
+// Weight and bias gradients of dense_0 .. dense_9 in the FP32 backward
+// (gemm_fp32_tc.cu): every layer's In^T dZ and column sums of dZ over n rows
+// added to the flat gradient blob, In from the FP32 tape, dz [10][n][256].
+int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t stream);
+
 // Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
 // layer's In^T dZ over M rows added to the flat gradient blob, In from the
 // BF16 tape, dz [10][M][256] BF16; part: gemm_dw_partial_floats(M) floats.

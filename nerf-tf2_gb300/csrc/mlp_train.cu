@@ -11,7 +11,8 @@
 //                 in shared memory:
 //                 dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
 //                                 * [h_prev[m][k] > 0]
-//   dW kernel     for every layer: dW[k][n] += sum_m In[m][k] dZ[m][n]
+//   dW kernel     for every layer: dW[k][n] += sum_m In[m][k] dZ[m][n], db[n]
+//                 += sum_m dZ[m][n], on the tensor cores (gemm_fp32_tc.cu)
 // Gradients land in the flat Keras layout of the parameter blob.
 #include <cuda_bf16.h>
 
@@ -288,115 +289,6 @@ __global__ void __launch_bounds__(fp32::kThreads, 2)
   }
 }
 
-// ---------------------------------------------------------------------------
-// dW: dW[(k_dst0 + k) * out + n] += sum_m In[m][k] dZ[m][n]; db[n] += sum dZ.
-// ---------------------------------------------------------------------------
-// All layers in one launch: grid (128 x 128 tiles of all the jobs, m-slices).
-// A thread holds 8 x 8 outputs as paired FMAs along n (fp32_tile.cuh gives
-// the reason); the rows stream through two 16-row stages of cp.async. A 4 x 4
-// tile per thread with guarded 4-byte loads was bound by its loads: 33 of the
-// 39 ms of a 1,024-ray step, 6.2 of 17.6 here.
-constexpr int kMC = 16, kTN = 128;
-
-struct DwJob {
-  int in_off, K, slot, flat, k_dst0;  // tape columns, dZ buffer, destination layer and rows
-};
-constexpr int kJobs = 12;
-__host__ __device__ constexpr DwJob dw_job(int j) {
-  return j == 0   ? DwJob{acts_offset(8), 256, 9, 10, 0}
-         : j == 1 ? DwJob{kActsEncDir, 27, 9, 10, 256}
-         : j == 2 ? DwJob{acts_offset(7), 256, 8, 9, 0}
-         : j == 3 ? DwJob{kActsEncXyz, 63, 5, 5, 256}
-         : j == 4 ? DwJob{kActsEncXyz, 63, 0, 0, 0}
-                  : DwJob{acts_offset(j - 5), 256, j - 4, j - 4, 0};  // dense_1 .. dense_7
-}
-__host__ __device__ constexpr int dw_tiles(int j) {
-  return ((dw_job(j).K + kTN - 1) / kTN) * (flat_out(dw_job(j).flat) / kTN);
-}
-__host__ __device__ constexpr int dw_first(int j) {
-  int t = 0;
-  for (int i = 0; i < j; ++i) t += dw_tiles(i);
-  return t;
-}
-constexpr int kDwTiles = dw_first(kJobs);
-static_assert(kActsEncDir + kTN <= kActsLd, "a tile's columns stay inside the row");
-
-__device__ __forceinline__ void cp_async16z(float *smem, const float *gmem, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(valid ? 16u : 0u));
-}
-
-__global__ void __launch_bounds__(256, 2)
-    dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, long long n, long long slice,
-              float *__restrict__ grads) {
-  __shared__ __align__(16) float sA[2][kMC][kTN];
-  __shared__ __align__(16) float sB[2][kMC][kTN];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int j = 0;
-  while (j + 1 < kJobs && (int)blockIdx.x >= dw_first(j + 1)) ++j;
-  const DwJob job = dw_job(j);
-  const int N = flat_out(job.flat), t = blockIdx.x - dw_first(j), ntn = N / kTN;
-  const int n0 = (t % ntn) * kTN, k0 = (t / ntn) * kTN;
-  const long long m_begin = blockIdx.y * slice, m_end = m_begin + slice < n ? m_begin + slice : n;
-  const float *A = acts + job.in_off + k0, *B = dz + job.slot * n * kDzLd + n0;
-  auto load = [&](long long m0, int st) {
-#pragma unroll
-    for (int p = tid; p < kMC * kTN / 4; p += 256) {
-      const int mm = p / (kTN / 4), q = p % (kTN / 4);
-      const bool v = m0 + mm < m_end;
-      const long long m = v ? m0 + mm : m_begin;
-      cp_async16z(&sA[st][mm][4 * q], A + m * kActsLd + 4 * q, v);
-      cp_async16z(&sB[st][mm][4 * q], B + m * kDzLd + 4 * q, v);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[i][q] = 0.0f;
-  float bacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const bool do_bias = job.k_dst0 == 0 && k0 == 0 && tid < 32;  // a warp holding the tile's columns (twice)
-  load(m_begin, 0);
-  int st = 0;
-#pragma unroll 1
-  for (long long m0 = m_begin; m0 < m_end; m0 += kMC, st ^= 1) {
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();  // the stage is there, the other one used up
-    if (m0 + kMC < m_end) load(m0 + kMC, st ^ 1);
-#pragma unroll
-    for (int mm = 0; mm < kMC; ++mm) {
-      float a[8], b[8];
-      *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(&sA[st][mm][4 * ty]);
-      *reinterpret_cast<float4 *>(a + 4) = *reinterpret_cast<const float4 *>(&sA[st][mm][64 + 4 * ty]);
-      *reinterpret_cast<float4 *>(b) = *reinterpret_cast<const float4 *>(&sB[st][mm][4 * tx]);
-      *reinterpret_cast<float4 *>(b + 4) = *reinterpret_cast<const float4 *>(&sB[st][mm][64 + 4 * tx]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int q = 0; q < 8; q += 2)
-          fma_f32x2(acc[i][q], acc[i][q + 1], a[i], a[i], b[q], b[q + 1], acc[i][q], acc[i][q + 1]);
-      if (do_bias) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) bacc[q] += b[q];
-      }
-    }
-  }
-  float *dW = grads + flat_offset(job.flat), *db = dW + (long long)flat_in(job.flat) * N;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int k = k0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
-    if (k >= job.K) continue;
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      atomicAdd(dW + (long long)(job.k_dst0 + k) * N + n0 + (q < 4 ? 4 * tx + q : 64 + 4 * tx + q - 4), acc[i][q]);
-  }
-  if (do_bias && ty == 0) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) atomicAdd(db + n0 + (q < 4 ? 4 * tx + q : 64 + 4 * tx + q - 4), bacc[q]);
-  }
-}
-
 }  // namespace train
 
 template <typename T, typename TZ>
@@ -490,12 +382,7 @@ extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long l
     chain_kernel<<<(unsigned)(tiles < 2 * sms ? tiles : 2 * sms), fp32::kThreads, fp32::kSmem, st>>>(w.wt, table, a, n,
                                                                                                 w.dsp, w.dz);
     if ((rc = launch_status()) != NERFGB_OK) return rc;
-    // slices of at least 256 rows, enough of them for eight waves of two CTAs per SM
-    const long long want = (16LL * sms + kDwTiles - 1) / kDwTiles, most = (n + 255) / 256;
-    const long long slices = want < most ? want : most;
-    const long long slice = ((n + slices - 1) / slices + kMC - 1) / kMC * kMC;
-    dw_kernel<<<dim3(kDwTiles, (unsigned)((n + slice - 1) / slice)), 256, 0, st>>>(a, w.dz, n, slice, grad_params);
-    if ((rc = launch_status()) != NERFGB_OK) return rc;
+    if ((rc = launch_fp32_dw(a, w.dz, n, grad_params, st)) != NERFGB_OK) return rc;
   }
   return NERFGB_OK;
 }
