@@ -1,25 +1,32 @@
-// FP32 weight gradients of the MLP backward on the tensor cores (the gradient
+// The products of the FP32 MLP backward on the tensor cores (the gradient
 // tf.GradientTape takes at nerf/core/model.py:148-170 through the Dense
 // layers of model.py:366-387): for every layer
 //
-//   dW[k][n] += sum_m In[m][k] dZ[m][n],   db[n] += sum_m dZ[m][n]
+//   dW[k][n] += sum_m In[m][k] dZ[m][n],   db[n] += sum_m dZ[m][n]    (dw_kernel)
+//   dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
+//                   * [h_prev[m][k] > 0]                             (chain_kernel)
 //
 // in FP32 accuracy from BF16 products. An FP32 value is exactly the sum of
-// three BF16 values, its 24 significant bits cut into three groups of eight
-// (x = x0 + x1 + x2, each group's exponent its own); of the nine products of
-// two such sums the six largest are taken (x0 y0, x0 y1, x1 y0, x1 y1, x0 y2,
-// x2 y0: what is left out is below 2^-24 of the product), smallest first, in
-// FP32 accumulators in TMEM. The tensor core's FP32 accumulation truncates, so
-// an accumulator takes only the 64 rows of one stage (four accumulations at
-// full magnitude) and the stages' sums are added in registers with rounding:
-// closer to the exact sum than one chain of FMAs over a slice of rows was (the
-// gradient of 5,000 rows 2.9e-7 from 64-bit arithmetic, against 8.1e-7).
+// three BF16 values (x rounded, what that leaves rounded, and the rest: 24
+// significant bits in three groups of eight); of the nine products of two such
+// sums the six largest are taken (x0 y0, x0 y1, x1 y0, x1 y1, x0 y2, x2 y0: what
+// is left out is below 2^-24 of the product and of either sign; parts cut off
+// instead of rounded left a bias of 6e-8 per layer), smallest first, in FP32
+// accumulators in TMEM. The tensor core's FP32 accumulation truncates, so an
+// accumulator takes only the 64 terms of one stage (four accumulations at full
+// magnitude) and the stages' sums are added in registers with rounding. The
+// gradient is closer to 64-bit arithmetic than from the chains of FMAs before:
+// 1.7e-7 of its norm for 1,000 rows (5.0e-7), 3.5e-7 for 100,000 (1.1e-6), and
+// for every layer. What is not finite becomes NaN.
 //
 // Six BF16 products are still four to five times the rate of the FP32 FMA
-// pipe, which bound the kernel before: 6.2 ms of a 1,024-ray step's two
-// networks (262,144 rows), 2.1 here. A 64-row stage takes ~6k cycles, 3,072 of
-// them MMAs; the conversion bounds it (~3.5k cycles of its eight warps; four
-// warps took 7k, a stage 12.7k with the MMAs issued by one of them).
+// pipe, which bound the kernels before: of a 1,024-ray step's two networks
+// (262,144 rows) dW took 6.2 ms, 2.0 here, and the chain 5.5, 2.1 here. A stage
+// is 3,072 cycles of MMAs. In dw_kernel, which converts both operands, it takes
+// ~6k: the conversion bounds it (~3.5k cycles of its eight warps; four warps
+// took 7k, a stage 12.7k with the MMAs issued by one of them). In chain_kernel
+// ~5.5k: the conversion is half, but the sums' warps also write dZ (~2k per
+// stage, the store path), during which no accumulator is free.
 //
 // CTAs run as cluster pairs (tcgen05.mma.cta_group::2, M = 256): each CTA
 // converts its half of either operand's columns, the even CTA issues. Both operands
@@ -42,6 +49,7 @@
 
 #include "common.cuh"
 #include "mlp_internal.cuh"
+#include "pair_tc.cuh"
 #include "tcgen05.cuh"
 
 namespace nerfgb {
@@ -63,11 +71,15 @@ constexpr uint32_t kBar0 = 2 * kStage;
 constexpr uint32_t kBarFull = kBar0;             // [2] operands of the stage written (both CTAs)
 constexpr uint32_t kBarDone = kBar0 + 16;        // [2] its MMAs are complete: stage free, accumulator full
 constexpr uint32_t kBarRead = kBar0 + 32;        // [2] its accumulator has been read (both CTAs)
-constexpr uint32_t kBarDrain = kBar0 + 48;
-constexpr uint32_t kTmemSlot = kBar0 + 56;
-constexpr uint32_t kAbort = kBar0 + 64;          // int, then the wait limit (u64) at +8
-constexpr uint32_t kErr = kBar0 + 80;            // int
-constexpr uint32_t kSmem = kBar0 + 96;
+constexpr uint32_t kBarB = kBar0 + 48;           // [2] chain: its weights have arrived (both CTAs')
+constexpr uint32_t kBarZ = kBar0 + 64;           // [2] chain: a tile's dZ of the layer is written
+constexpr uint32_t kBarMask = kBar0 + 80;        // [2] chain: a tile's mask of the layer is written
+constexpr uint32_t kBarDrain = kBar0 + 96;
+constexpr uint32_t kTmemSlot = kBar0 + 104;
+constexpr uint32_t kAbort = kBar0 + 112;         // int, then the wait limit (u64) at +8
+constexpr uint32_t kErr = kBar0 + 128;           // int
+constexpr uint32_t kMask = kBar0 + 144;          // [2][256 threads] chain: mask bits, 16 bytes each
+constexpr uint32_t kSmem = kMask + 2 * 4096;
 static_assert(kSmem <= 227 * 1024, "two stages");
 
 // One product. Plain: A = the tape's columns col .. col + 255 (the layer's
@@ -113,25 +125,110 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
          (1ull << 46) | (2ull << 61);
 }
 
-// The upper halves of two words (BF16 by truncation) as one word.
-__device__ __forceinline__ uint32_t upper(float lo, float hi) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(d) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
-  return d;
+// Barriers, TMEM (all 512 columns of both CTAs; its address) and the pair's start.
+__device__ __forceinline__ uint32_t begin(uint8_t *smem, uint32_t sbase, volatile int *abort_flag, int *err,
+                                          bool aligned) {
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(sbase + kBarFull + 8 * s, 2 * kConvWarps);
+      mbar_init(sbase + kBarDone + 8 * s, 1);
+      mbar_init(sbase + kBarRead + 8 * s, 2 * kSumWarps);
+      mbar_init(sbase + kBarB + 8 * s, 1);
+      mbar_init(sbase + kBarZ + 8 * s, kSumWarps);
+      mbar_init(sbase + kBarMask + 8 * s, kConvWarps);
+    }
+    mbar_init(sbase + kBarDrain, 1);
+    *abort_flag = aligned ? 0 : 1;
+    *err = 0;
+    set_wait_limit(abort_flag, kWaitNs);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kTmemSlot),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  return *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
 }
-__device__ __forceinline__ float head(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+
+// The MMAs of a stage: the six products, smallest first, of K-steps `step`
+// descriptor units apart.
+__device__ __forceinline__ void issue_stage(uint32_t acc, uint64_t a, uint64_t b, uint32_t step, uint32_t idesc) {
+  constexpr int px[6] = {0, 2, 1, 0, 1, 0}, py[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int s = 0; s < kRows / 16; ++s)
+      tc_mma_pair(acc, a + px[i] * (kPart >> 4) + s * step, b + py[i] * (kPart >> 4) + s * step, idesc,
+                  i + s > 0 ? 1u : 0u);
+}
+
+// Both CTAs must hold the same TMEM columns (the collective allocation gives them).
+__device__ __forceinline__ void check_tmem(uint32_t sbase, uint32_t tmem, volatile int *abort_flag) {
+  uint32_t peer_tmem;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(peer_tmem) : "r"(peer_addr(sbase + kTmemSlot, 1)) : "memory");
+  if (peer_tmem != tmem) *abort_flag = 1;
+}
+
+// By the issuer: every MMA is complete (in both CTAs).
+__device__ __forceinline__ void drain(uint32_t sbase) {
+  tc_commit_pair(sbase + kBarDrain);
+  const uint64_t t0 = globaltimer();
+  while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
+  }
+}
+
+// The pair's end. After a timeout the gradient is not a number. `ran`: the issuer drains.
+__device__ __forceinline__ void finish(uint32_t sbase, uint32_t tmem, volatile int *abort_flag, float *grads, bool ran) {
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x < 11) grads[flat_offset(threadIdx.x)] = __int_as_float(0x7fffffff);
+  if (cluster_rank() == 1 && threadIdx.x == 0 && ran) {
+    // the even CTA's MMAs read this CTA's stages: its last commit
+    uint64_t t0 = globaltimer();
+    while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
+    }
+    // after a timeout (in either CTA) copies that complete on the even CTA's
+    // barriers may be in flight: give them 100 us (mlp_tc.cu)
+    uint32_t peer_abort;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(peer_abort) : "r"(peer_addr(sbase + kAbort, 0)) : "memory");
+    if (*abort_flag || peer_abort) {
+      t0 = globaltimer();
+      while (globaltimer() - t0 < 100000ull) {
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (threadIdx.x < 32) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+// The BF16 parts of two values, packed: what the rounding leaves of a 24-bit
+// value has at most 16 bits, of those at most 8, each exactly subtracted.
+__device__ __forceinline__ uint32_t next_part(float &x, float &y) {
+  const uint32_t p = pack_bf16(x, y);
+  x -= __uint_as_float(p << 16);
+  y -= __uint_as_float(p & 0xffff0000u);
+  return p;
+}
 
 // Eight values of a row to the three parts' 16-byte chunks at dst.
 __device__ __forceinline__ void split_store(const float4 &u, const float4 &v, uint32_t dst) {
-  const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-  float r[8], q[8];
+  float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) r[i] = x[i] - head(x[i]);
+  for (int i = 0; i < 3; ++i) {
+    uint32_t p[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] = r[i] - head(r[i]);
-  st_shared_v4(dst, upper(x[0], x[1]), upper(x[2], x[3]), upper(x[4], x[5]), upper(x[6], x[7]));
-  st_shared_v4(dst + kPart, upper(r[0], r[1]), upper(r[2], r[3]), upper(r[4], r[5]), upper(r[6], r[7]));
-  st_shared_v4(dst + 2 * kPart, upper(q[0], q[1]), upper(q[2], q[3]), upper(q[4], q[5]), upper(q[6], q[7]));
+    for (int j = 0; j < 4; ++j) p[j] = next_part(x[2 * j], x[2 * j + 1]);
+    st_shared_v4(dst + i * kPart, p[0], p[1], p[2], p[3]);
+  }
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -147,28 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const bool aligned = (sbase & 1023u) == 0;
   const int stages = aligned ? (int)((n + kRows - 1) / kRows) : 0;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(sbase + kBarFull + 8 * s, 2 * kConvWarps);
-      mbar_init(sbase + kBarDone + 8 * s, 1);
-      mbar_init(sbase + kBarRead + 8 * s, 2 * kSumWarps);
-    }
-    mbar_init(sbase + kBarDrain, 1);
-    *abort_flag = aligned ? 0 : 1;
-    *err = 0;
-    set_wait_limit(abort_flag, kWaitNs);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kTmemSlot),
-                 "r"(512));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();
-  tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
+  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned);
 
   if (warp >= kSumWarps) {
     // ---------------- conversion ----------------
@@ -302,13 +378,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool issuer = crank == 0 && threadIdx.x == 0;
     int ij = -1, ileft = 0;  // its job, the job's stages left
     uint32_t iq = 0;
-    if (issuer) {
-      // both CTAs must hold the same TMEM columns (the collective allocation gives them)
-      uint32_t peer_tmem;
-      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(peer_tmem) : "r"(peer_addr(sbase + kTmemSlot, 1))
-                   : "memory");
-      if (peer_tmem != tmem) *abort_flag = 1;
-    }
+    if (issuer) check_tmem(sbase, tmem, abort_flag);
     auto issue_next = [&]() {
       while (ileft == 0) {
         if (++ij >= kJobs) {
@@ -328,14 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc_fence_after();
       const uint32_t idesc = idesc_bf16(256, 0) | (1u << 15) | (1u << 16) | ((uint32_t)(job_of(ij).n_mma() >> 3) << 17);
       const uint32_t sa = sbase + k * kStage, acc = tmem + 256u * k;
-      // the six products, smallest first
-      constexpr int px[6] = {0, 2, 1, 0, 1, 0}, py[6] = {2, 0, 1, 1, 0, 0};
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-#pragma unroll
-        for (int s = 0; s < kRows / 16; ++s)
-          tc_mma_pair(acc, desc_mn_sw128(sa + px[i] * kPart + 2048u * s),
-                      desc_mn_sw128(sa + kOperand + py[i] * kPart + 2048u * s), idesc, i + s > 0 ? 1u : 0u);
+      issue_stage(acc, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc);
       tc_commit_pair(sbase + kBarDone + 8 * k);
     };
     if (issuer) issue_next();
@@ -396,39 +459,281 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
-    if (issuer && stages > 0) {
-      // Drain every MMA issued before TMEM is released (in both CTAs).
-      tc_commit_pair(sbase + kBarDrain);
-      const uint64_t t0 = globaltimer();
-      while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
-      }
-    }
+    if (issuer && stages > 0) drain(sbase);
   }
 
-  tc_fence_before();
-  __syncthreads();
-  if (*abort_flag && threadIdx.x < 11) grads[flat_offset(threadIdx.x)] = __int_as_float(0x7fffffff);
-  if (crank == 1 && threadIdx.x == 0 && stages > 0) {
-    // the even CTA's MMAs read this CTA's stages: its last commit (after a
-    // timeout of either CTA: for a bounded time)
-    const uint64_t t0 = globaltimer();
-    while (!mbar_try(sbase + kBarDrain, 0) && globaltimer() - t0 < 100000000ull) {
+  finish(sbase, tmem, abort_flag, grads, stages > 0);
+}
+
+// ---------------------------------------------------------------------------
+// Chain
+// ---------------------------------------------------------------------------
+// Weights of GEMM layer g as the B operand of dX: 64 n at a time, for either
+// CTA (128 k) the three parts, K-major in the 128-byte swizzled layout: row k
+// at k * 128 bytes, its 16-byte chunk c at (c ^ (k & 7)) * 16. Layers from
+// dense_9 down.
+__host__ __device__ constexpr int first_chunk(int g) { return g == 9 ? 0 : 2 + (8 - g) * 4; }
+constexpr long long kPackBytes = (long long)first_chunk(0) * 2 * kOperand;
+
+__global__ void pack_kernel(const float *__restrict__ W, uint8_t *__restrict__ out) {
+  const int g = 9 - blockIdx.y, N = gemm_n(g), e = blockIdx.x * blockDim.x + threadIdx.x;  // k * N + n
+  if (e >= 256 * N) return;
+  const int k = e / N, n = e % N;
+  float x = W[gemm_w_offset(g) + e], none = 0.0f;
+  uint8_t *dst = out + ((long long)(first_chunk(g) + n / 64) * 2 + k / 128) * kOperand + (k % 128) * 128 +
+                 ((((n % 64) / 8) ^ (k & 7)) << 4) + (n % 8) * 2;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint16_t *>(dst + i * kPart) = (uint16_t)next_part(x, none);
+}
+
+// dz [10][n][256]: dz[9] (128 columns) in, dz[8] .. dz[0] out. A pair takes
+// tiles of 256 rows (128 per CTA) through all layers, two tiles in turn, so
+// that one's sums and dZ are finished under the other's MMAs (with a tile
+// alone a layer's first stage waits for the layer before); a tile's dZ goes
+// through L2 to the conversion of the next layer (the three parts of a tile
+// would fill shared memory). K runs in stages of 64 n: the dZ converted as in
+// dw_kernel, K-major, the weights split once (pack_kernel) and copied by TMA.
+// The ReLU masks are read as bits by the conversion's warps, a layer after
+// their rows were fetched into L2: read by the sums' warps at the end of a
+// layer, the loads' latencies were four fifths of the time (1,094 us for 65,536
+// rows; in their waits for the stages 550; 490 - 526 here).
+__global__ void __launch_bounds__(kThreads, 1)
+    chain_kernel(const float *__restrict__ sigma_w, const float *__restrict__ acts, const float *__restrict__ dsp,
+                 long long n, float *dz, float *__restrict__ grads, const __grid_constant__ CUtensorMap weights) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_rank();
+  const int pair = (int)cluster_id(), pairs = (int)cluster_count();
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kAbort);
+  int *err = reinterpret_cast<int *>(smem + kErr);
+  // (the swizzled stages need 1024-byte alignment: without it nothing runs)
+  const bool aligned = (sbase & 1023u) == 0;
+  const int tiles = aligned ? (int)((n + 255) / 256) : 0;
+  // the tiles dealt evenly and contiguously
+  const int first = (int)((long long)pair * tiles / pairs), count = (int)((long long)(pair + 1) * tiles / pairs) - first;
+  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned);
+
+  if (warp >= kSumWarps) {
+    // ---------------- conversion, weight copies ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kConvRegs));
+    // A lane takes 8 of a stage's 64 n (chunk c) of the rows r + 32u.
+    const int w = warp - kSumWarps, c = lane & 7, r = w * 4 + (lane >> 3);
+    const uint32_t dst = sbase + (uint32_t)r * 128u + (uint32_t)((c ^ (r & 7)) << 4);
+    bool ok = true;
+    uint32_t q = 0;
+#pragma unroll 1
+    for (int t = 0; t < count && ok; t += 2) {
+      const int subs = min(2, count - t);
+#pragma unroll 1
+      for (int g = 9; g >= 1 && ok; --g) {
+        const int chunks = gemm_n(g) / 64;
+#pragma unroll 1
+        for (int s = 0; s < subs && ok; ++s) {
+          if (g < 9 && !__all_sync(0xffffffffu, wait_bar(sbase + kBarZ + 8 * s, (uint32_t)(g & 1), abort_flag, err))) {
+            ok = false;
+            break;
+          }
+          const long long tile0 = (long long)(first + t + s) * 256 + crank * 128, row = tile0 + r;
+          // the next layer's mask into L2, a row per lane
+          if (g > 1 && w < 4 && tile0 + w * 32 + lane < n)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(acts + (tile0 + w * 32 + lane) * kActsLd +
+                                                                             acts_offset(g - 2)),
+                         "r"(1024)
+                         : "memory");
+          // This layer's mask for lane `lane` of sum warp w: its columns of the
+          // rows mrow + 8 rr (a bit each), one rr per stage.
+          const long long mrow = tile0 + 32 * (w & 3) + lane / 4;
+          const float *mask = acts + mrow * kActsLd + acts_offset(g - 1) + 128 * (w >> 2) + 2 * (lane % 4);
+          uint32_t bits[4] = {0u, 0u, 0u, 0u};
+          float2 m[8];
+          auto load_mask = [&](int rr, int half) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              m[i] = make_float2(0.f, 0.f);
+              if (g != 9 && mrow + 8 * rr < n)
+                m[i] = __ldcs(reinterpret_cast<const float2 *>(mask + (long long)8 * rr * kActsLd + 8 * (8 * half + i)));
+            }
+          };
+          auto mask_bits = [&](int half) {
+            uint32_t v = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              v |= (m[i].x > 0.0f ? 1u : 0u) << (2 * (8 * half + i)) | (m[i].y > 0.0f ? 2u : 0u) << (2 * (8 * half + i));
+            return v;
+          };
+          const float *src = dz + ((long long)g * n + row) * 256 + 8 * c;
+          float4 v[4][2];
+          auto load = [&](int ch, int u) {
+            v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ch < chunks && row + 32 * u < n) {
+              // (written in this launch: not through the read-only path)
+              const float4 *p = reinterpret_cast<const float4 *>(src + 32 * 256 * u + 64 * ch);
+              v[u][0] = __ldcg(p);
+              v[u][1] = __ldcg(p + 1);
+            }
+          };
+#pragma unroll
+          for (int u = 0; u < 4; ++u) load(0, u);
+#pragma unroll 1
+          for (int ch = 0; ch < chunks; ++ch, ++q) {
+            const uint32_t k = q & 1u;
+            load_mask(ch, 0);
+            if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, ((q >> 1) & 1u) ^ 1u, abort_flag, err))) {
+              ok = false;
+              break;
+            }
+            if (w == 0 && lane == 0) {
+              const uint32_t bar = sbase + kBarB + 8 * k, to = sbase + k * kStage + kOperand;
+              if (crank == 0) mbar_expect_tx(bar, 2 * kOperand);
+              const int y = ((first_chunk(g) + ch) * 2 + (int)crank) * (int)(kOperand / 256);
+#pragma unroll
+              for (int i = 0; i < 3; ++i)
+                tma_2d_pair(to + i * kPart, &weights, 0, y + i * (int)(kPart / 256), crank == 0 ? bar : peer_addr(bar, 0));
+            }
+            __syncwarp();
+            uint32_t mb = mask_bits(0);
+            load_mask(ch, 1);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              split_store(v[u][0], v[u][1], dst + k * kStage + 4096u * u);
+              load(ch + 1, u);
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarFull + 8 * k, 0));
+            mb |= mask_bits(1);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bits[i] = ch == i ? mb : bits[i];
+          }
+          if (g != 9) {
+            st_shared_v4(sbase + kMask + s * 4096 + (w * 32 + lane) * 16, bits[0], bits[1], bits[2], bits[3]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sbase + kBarMask + 8 * s);
+          }
+        }
+      }
     }
+  } else {
+    // ---------------- the stages' sums, dZ (and the issuer) ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSumRegs));
+    const int qd = warp & 3, h = warp >> 2;
+    const uint32_t tl = tmem + ((uint32_t)(32 * qd) << 16) + 128u * h;
+    const bool issuer = crank == 0 && threadIdx.x == 0;
+    const uint32_t total = (uint32_t)count * first_chunk(0);
+    if (issuer) check_tmem(sbase, tmem, abort_flag);
+    uint32_t iq = 0;  // stages issued
+    auto issue = [&]() {
+      if (iq >= total) return;
+      const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
+      ++iq;
+      if (!wait_bar(sbase + kBarFull + 8 * k, ph, abort_flag, err) ||
+          !wait_bar(sbase + kBarB + 8 * k, ph, abort_flag, err) ||
+          !wait_bar(sbase + kBarRead + 8 * k, ph ^ 1u, abort_flag, err))
+        return;
+      tc_fence_after();
+      const uint32_t sa = (sbase + k * kStage) & 0x3FFFFu;
+      const uint64_t hi = (uint64_t)kDescHiA << 32;
+      issue_stage(tmem + 256u * k, hi | (sa >> 4) | (1u << 16), hi | ((sa + kOperand) >> 4) | (1u << 16), 32 >> 4,
+                  idesc_bf16(256, 256));
+      tc_commit_pair(sbase + kBarDone + 8 * k);
+    };
+    bool ok = true;
+    uint32_t q = 0;
+#pragma unroll 1
+    for (int t = 0; t < count && ok; t += 2) {
+      const int subs = min(2, count - t);
+#pragma unroll 1
+      for (int g = 9; g >= 1 && ok; --g) {
+        const int chunks = gemm_n(g) / 64;
+#pragma unroll 1
+        for (int s = 0; s < subs; ++s) {
+          const long long row0 = (long long)(first + t + s) * 256 + crank * 128 + 32 * qd + lane / 4;
+          const int col0 = 128 * h + 2 * (lane % 4);
+          float sum[4][2][16];
+#pragma unroll
+          for (int f = 0; f < 8; ++f)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sum[f / 2][f % 2][i] = 0.0f;
+#pragma unroll 1
+          for (int ch = 0; ch < chunks; ++ch, ++q) {
+            const uint32_t k = q & 1u;
+            if (issuer) {
+              if (iq == q) issue();
+              // a stage ahead, unless that waits for the dZ of this one (a tile alone)
+              if (iq == q + 1 && (subs == 2 || ch + 1 < chunks)) issue();
+            }
+            if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, (q >> 1) & 1u, abort_flag, err))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+#pragma unroll
+            for (int f = 0; f < 8; ++f) {
+              uint32_t raw[16];
+              tmem_ld_frag32(tl + ((uint32_t)(16 * (f % 2)) << 16) + 256u * k + 32 * (f / 2), raw);
+              tmem_wait16(raw);
+              float *a = sum[f / 2][f % 2];
+#pragma unroll
+              for (int i = 0; i < 16; i += 2)
+                add_f32x2(a[i], a[i + 1], a[i], a[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarRead + 8 * k, 0));
+          }
+          if (!ok) break;
+          // dense_9's input, the bottleneck, is linear: no mask
+          uint32_t bits[4] = {~0u, ~0u, ~0u, ~0u};
+          if (g != 9) {
+            if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarMask + 8 * s, (uint32_t)(g & 1), abort_flag, err))) {
+              ok = false;
+              break;
+            }
+            ld_shared_v4(sbase + kMask + s * 4096 + threadIdx.x * 16, bits[0], bits[1], bits[2], bits[3]);
+          }
+          float *out = dz + ((long long)(g - 1) * n + row0) * 256 + col0;
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr) {  // rows row0 + 8 rr
+            if (row0 + 8 * rr >= n) continue;
+            const float ds = g == 8 ? dsp[row0 + 8 * rr] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {  // columns col0 + 8 j, + 1
+              const float *a = sum[j / 4][rr / 2] + 4 * (j % 4) + 2 * (rr % 2);
+              float2 z = make_float2(a[0], a[1]);
+              if (g == 8) {  // dense_8's input h7 also feeds the sigma head
+                const float2 ws = *reinterpret_cast<const float2 *>(sigma_w + col0 + 8 * j);
+                z.x = fmaf(ds, ws.x, z.x);
+                z.y = fmaf(ds, ws.y, z.y);
+              }
+              z.x = bits[rr] >> (2 * j) & 1u ? z.x : 0.0f;
+              z.y = bits[rr] >> (2 * j) & 2u ? z.y : 0.0f;
+              *reinterpret_cast<float2 *>(out + 8 * rr * 256 + 8 * j) = z;
+            }
+          }
+          __syncwarp();
+          if (g > 1 && lane == 0) mbar_arrive(sbase + kBarZ + 8 * s);
+        }
+      }
+    }
+    if (issuer && tiles > 0) drain(sbase);
   }
-  __syncwarp();
-  cluster_sync_all();
-  if (warp == 0) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
-  }
+
+  finish(sbase, tmem, abort_flag, grads, tiles > 0);
 }
 
 }  // namespace split
 
-int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t st) {
-  using namespace split;
-  if (n == 0) return NERFGB_OK;
-  if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
+// Launches a pair kernel on at most `work` pairs, as many as are co-resident
+// (asked once per device, as mlp_tc.cu).
+namespace split {
+struct Pairs {
+  std::mutex mu;
+  std::unordered_map<int, int> of_device;
+};
+template <typename... P, typename... A>
+static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cudaStream_t st, A... args) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
     return NERFGB_E_CUDA;
   const int sms = num_sms();
   if (sms <= 0) return NERFGB_E_DEVICE;
@@ -443,27 +748,51 @@ int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // co-resident pairs, asked once per device (as mlp_tc.cu)
-  static std::mutex mu;
-  static std::unordered_map<int, int> pairs_of_device;
-  int dev = -1, max_pairs;
+  int dev = -1, most;
   if (cudaGetDevice(&dev) != cudaSuccess) return NERFGB_E_DEVICE;
   {
-    std::lock_guard<std::mutex> lock(mu);
-    auto hit = pairs_of_device.find(dev);
-    if (hit == pairs_of_device.end()) {
+    std::lock_guard<std::mutex> lock(pairs.mu);
+    auto hit = pairs.of_device.find(dev);
+    if (hit == pairs.of_device.end()) {
       cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
       int m = 0;
-      if (cudaOccupancyMaxActiveClusters(&m, dw_kernel, &cfg) != cudaSuccess) return NERFGB_E_CUDA;
-      hit = pairs_of_device.emplace(dev, m).first;
+      if (cudaOccupancyMaxActiveClusters(&m, kernel, &cfg) != cudaSuccess) return NERFGB_E_CUDA;
+      hit = pairs.of_device.emplace(dev, m).first;
     }
-    max_pairs = hit->second;
+    most = hit->second;
   }
-  if (max_pairs < 1) return NERFGB_E_UNSUPPORTED;
-  const long long work = kJobs * ((n + kRows - 1) / kRows), pairs = work < max_pairs ? work : max_pairs;
-  cfg.gridDim = dim3((unsigned)(2 * pairs));
-  if (cudaLaunchKernelEx(&cfg, dw_kernel, acts, dz, n, grads) != cudaSuccess) return NERFGB_E_CUDA;
+  if (most < 1) return NERFGB_E_UNSUPPORTED;
+  cfg.gridDim = dim3((unsigned)(2 * (work < most ? work : most)));
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return NERFGB_E_CUDA;
   return launch_status();
+}
+}  // namespace split
+
+int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t st) {
+  using namespace split;
+  if (n == 0) return NERFGB_OK;
+  static Pairs pairs;
+  return launch_pairs(dw_kernel, pairs, kJobs * ((n + kRows - 1) / kRows), st, acts, dz, n, grads);
+}
+
+long long fp32_chain_pack_bytes() { return split::kPackBytes; }
+
+int launch_fp32_chain_pack(const float *packed, void *wpack, cudaStream_t st) {
+  split::pack_kernel<<<dim3(256, 9), 256, 0, st>>>(packed, reinterpret_cast<uint8_t *>(wpack));
+  return launch_status();
+}
+
+int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts, const float *dsp, long long n,
+                      float *dz, float *grads, cudaStream_t st) {
+  using namespace split;
+  if (n == 0) return NERFGB_OK;
+  static Pairs pairs;
+  CUtensorMap weights;
+  const unsigned long long dims[2] = {128, (unsigned long long)(kPackBytes / 256)}, strides[1] = {256};
+  const unsigned box[2] = {128, kPart / 256};
+  const int rc = encode_tensor_map_u16(&weights, wpack, 2, dims, strides, box);
+  if (rc != NERFGB_OK) return rc;
+  return launch_pairs(chain_kernel, pairs, (n + 255) / 256, st, sigma_w, acts, dsp, n, dz, grads, weights);
 }
 
 }  // namespace nerfgb

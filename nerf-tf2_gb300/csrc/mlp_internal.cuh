@@ -62,6 +62,15 @@ int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t st
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
                      __nv_bfloat16 *dz, float *grads, int *err, cudaStream_t stream);
 
+// The dX products of the FP32 backward (gemm_fp32_tc.cu): dz [10][n][256],
+// dz[9] in (128 columns), dz[8] .. dz[0] out. wpack (fp32_chain_pack_bytes,
+// 16-byte aligned) from the FP32 pack's weights by launch_fp32_chain_pack;
+// sigma_w: the sigma head's weights; grads: not a number after a timeout.
+long long fp32_chain_pack_bytes();
+int launch_fp32_chain_pack(const float *packed, void *wpack, cudaStream_t stream);
+int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts, const float *dsp, long long n,
+                      float *dz, float *grads, cudaStream_t stream);
+
 // Weight and bias gradients of dense_0 .. dense_9 in the FP32 backward
 // (gemm_fp32_tc.cu): every layer's In^T dZ and column sums of dZ over n rows
 // added to the flat gradient blob, In from the FP32 tape, dz [10][n][256].

@@ -7,19 +7,18 @@
 // chunks of kChunkRows; per chunk
 //   head kernel   rgb = sigmoid(h9 Wr + br), sigma = ReLU(h7 ws + bs):
 //                 dZ9 = (dpre_rgb Wr^T) * [h9 > 0], dpre_sigma, head grads
-//   chain kernel  for every layer from dense_9 down, a tile of rows staying
-//                 in shared memory:
+//   chain kernel  for every layer from dense_9 down:
 //                 dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
 //                                 * [h_prev[m][k] > 0]
 //   dW kernel     for every layer: dW[k][n] += sum_m In[m][k] dZ[m][n], db[n]
-//                 += sum_m dZ[m][n], on the tensor cores (gemm_fp32_tc.cu)
+//                 += sum_m dZ[m][n]
+// the last two on the tensor cores in FP32 accuracy (gemm_fp32_tc.cu).
 // Gradients land in the flat Keras layout of the parameter blob.
 #include <cuda_bf16.h>
 
 #include <type_traits>
 
 #include "common.cuh"
-#include "fp32_tile.cuh"
 #include "mlp_internal.cuh"
 
 namespace nerfgb {
@@ -27,8 +26,8 @@ namespace train {
 
 constexpr int kDzLd = 256;  // row stride of the dZ buffers
 // Rows per chunk: the workspace holds every layer's dZ of one chunk (four
-// 64-row tiles per CTA of the chain kernel, two CTAs per SM, 152 SMs).
-constexpr long long kChunkRows = 4LL * 2 * 152 * 64;
+// 256-row tiles per pair of the chain kernel, 76 pairs).
+constexpr long long kChunkRows = 4LL * 76 * 256;
 
 // ---------------------------------------------------------------------------
 // Heads
@@ -202,93 +201,6 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
   }
 }
 
-// ---------------------------------------------------------------------------
-// Chain
-// ---------------------------------------------------------------------------
-// Transposed weights of GEMM layer g >= 1, [n][k < 256], for the chain.
-__host__ __device__ constexpr long long wt_offset(int g) {
-  long long off = 0;
-  for (int i = 1; i < g; ++i) off += (long long)gemm_n(i) * 256;
-  return off;
-}
-constexpr long long kWtElems = wt_offset(kNumGemm);
-
-__global__ void transpose_kernel(const float *__restrict__ W, float *__restrict__ wt) {
-  __shared__ float t[32][33];
-  const int g = blockIdx.z + 1, N = gemm_n(g), n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  if (n0 >= N) return;
-  const float *src = W + gemm_w_offset(g);
-  for (int i = threadIdx.y; i < 32; i += 8) t[i][threadIdx.x] = src[(long long)(k0 + i) * N + n0 + threadIdx.x];
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) wt[wt_offset(g) + (long long)(n0 + i) * 256 + k0 + threadIdx.x] = t[threadIdx.x][i];
-}
-
-// dz [10][rows][kDzLd]: dz[9] (128 columns, from the heads) in, dz[8] .. dz[0]
-// out. The layers' products are the forward's (fp32_tile.cuh: X the tile's
-// dZ, the transposed weights streamed); every output is one chain of FMAs
-// over n in order. Taking the layers one kernel at a time re-read and
-// re-staged dZ and gathered W transposed for every 64-row tile (8.4 ms of a
-// 1,024-ray step's two networks, against 5.5 here).
-__global__ void __launch_bounds__(fp32::kThreads, 2)
-    chain_kernel(const float *__restrict__ wt, const float *__restrict__ table, const float *__restrict__ acts,
-                 long long n, const float *__restrict__ dsp, float *__restrict__ dz) {
-  using fp32::kTM;
-  using fp32::kXLD;
-  extern __shared__ __align__(16) float sm[];
-  float *X = sm, *Wb = sm + kTM * kXLD;
-  const int tid = threadIdx.x;
-  const fp32::Place pl(tid, 256);
-  const long long ntiles = (n + kTM - 1) / kTM;
-  int buf = 0;
-  if ((long long)blockIdx.x < ntiles) fp32::load_chunk<256>(wt + wt_offset(9), Wb, tid);
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long row0 = tile * kTM;
-    for (int e = tid; e < kTM * 32; e += fp32::kThreads) {
-      const int r = e >> 5, q = e & 31;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row0 + r < n) v = *reinterpret_cast<const float4 *>(dz + (9 * n + row0 + r) * kDzLd + 4 * q);
-      *reinterpret_cast<float4 *>(X + r * kXLD + 4 * q) = v;
-    }
-#pragma unroll 1
-    for (int g = 9; g >= 1; --g) {
-      const bool more = g > 1 || tile + gridDim.x < ntiles;
-      float acc[8][8];
-      fp32::layer<256>(X, Wb, buf, wt + wt_offset(g), gemm_n(g), 0, wt + wt_offset(g > 1 ? g - 1 : 9), more ? 256 : 0,
-                       tid, pl, acc);
-      // dense_9's input, the bottleneck, is linear: no mask; dense_8's input h7 also feeds the sigma head
-      const int mask_off = g == 9 ? -1 : acts_offset(g - 1);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const long long m = row0 + pl.row(i);
-        const bool valid = m < n;
-        const float ds = g == 8 && valid ? dsp[m] : 0.0f;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = pl.col(h);
-          float4 v = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
-          if (g == 8) {
-            const float4 ws = *reinterpret_cast<const float4 *>(table + kSigmaWOff + k);
-            v.x = fmaf(ds, ws.x, v.x);
-            v.y = fmaf(ds, ws.y, v.y);
-            v.z = fmaf(ds, ws.z, v.z);
-            v.w = fmaf(ds, ws.w, v.w);
-          }
-          if (mask_off >= 0 && valid) {
-            const float4 hm = *reinterpret_cast<const float4 *>(acts + m * kActsLd + mask_off + k);
-            v.x = hm.x > 0.0f ? v.x : 0.0f;
-            v.y = hm.y > 0.0f ? v.y : 0.0f;
-            v.z = hm.z > 0.0f ? v.z : 0.0f;
-            v.w = hm.w > 0.0f ? v.w : 0.0f;
-          }
-          *reinterpret_cast<float4 *>(X + pl.row(i) * kXLD + k) = v;
-          if (valid) *reinterpret_cast<float4 *>(dz + ((g - 1) * n + m) * kDzLd + k) = v;
-        }
-      }
-    }
-    __syncthreads();  // X is rewritten
-  }
-}
-
 }  // namespace train
 
 template <typename T, typename TZ>
@@ -318,17 +230,18 @@ int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const
 namespace train {
 
 struct Ws {
-  float *wt, *dsp, *dz;
+  float *wpack, *dsp, *dz;
   long long rows, bytes;
 };
 static Ws carve(void *base, long long n) {
   Ws w{};
   float *p = reinterpret_cast<float *>(base);
   w.rows = n < kChunkRows ? n : kChunkRows;
-  w.wt = p;
-  w.dz = p + kWtElems;
+  const long long pack = fp32_chain_pack_bytes() / (long long)sizeof(float);
+  w.wpack = p;
+  w.dz = p + pack;
   w.dsp = w.dz + kNumGemm * w.rows * kDzLd;
-  w.bytes = (kWtElems + w.rows * (kNumGemm * kDzLd + 1)) * (long long)sizeof(float);
+  w.bytes = (pack + w.rows * (kNumGemm * kDzLd + 1)) * (long long)sizeof(float);
   return w;
 }
 
@@ -365,23 +278,16 @@ extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long l
   const float *W = reinterpret_cast<const float *>(packed);  // FP32 pack: padded [Kp][N] blocks
   const float *table = W + kFp32TableOff;
   const Ws w = carve(workspace, n_rows);
-  const int sms = num_sms();
-  if (sms <= 0) return NERFGB_E_DEVICE;
-  if (cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) != cudaSuccess)
-    return NERFGB_E_CUDA;
-  transpose_kernel<<<dim3(8, 8, kNumGemm - 1), dim3(32, 8), 0, st>>>(W, w.wt);
   int rc;
-  if ((rc = launch_status()) != NERFGB_OK) return rc;
+  if ((rc = launch_fp32_chain_pack(W, w.wpack, st)) != NERFGB_OK) return rc;
   for (long long r0 = 0; r0 < n_rows; r0 += kChunkRows) {
     const long long n = n_rows - r0 < kChunkRows ? n_rows - r0 : kChunkRows;
     const float *a = acts + r0 * kActsLd;
     if ((rc = launch_head_bwd(table, a, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * kDzLd,
                               w.dsp, grad_params, st)) != NERFGB_OK)
       return rc;
-    const long long tiles = (n + fp32::kTM - 1) / fp32::kTM;
-    chain_kernel<<<(unsigned)(tiles < 2 * sms ? tiles : 2 * sms), fp32::kThreads, fp32::kSmem, st>>>(w.wt, table, a, n,
-                                                                                                w.dsp, w.dz);
-    if ((rc = launch_status()) != NERFGB_OK) return rc;
+    if ((rc = launch_fp32_chain(w.wpack, table + kSigmaWOff, a, w.dsp, n, w.dz, grad_params, st)) != NERFGB_OK)
+      return rc;
     if ((rc = launch_fp32_dw(a, w.dz, n, grad_params, st)) != NERFGB_OK) return rc;
   }
   return NERFGB_OK;
