@@ -21,12 +21,12 @@
 //
 // Six BF16 products are still four to five times the rate of the FP32 FMA
 // pipe, which bound the kernels before: of a 1,024-ray step's two networks
-// (262,144 rows) dW took 6.2 ms, 2.0 here, and the chain 5.5, 2.1 here. A stage
-// is 3,072 cycles of MMAs. In dw_kernel, which converts both operands, it takes
-// ~6k: the conversion bounds it (~3.5k cycles of its eight warps; four warps
-// took 7k, a stage 12.7k with the MMAs issued by one of them). In chain_kernel
-// ~5.5k: the conversion is half, but the sums' warps also write dZ (~2k per
-// stage, the store path), during which no accumulator is free.
+// (262,144 rows) dW took 6.2 ms, 1.6 here, and the chain 5.5, 2.1 here. A stage
+// is 3,072 cycles of MMAs. In dw_kernel, which converts both operands with
+// eight warps, it takes ~4.3k (with four of them 7k for the conversion alone,
+// and 12.7k with the MMAs issued by one of them). In chain_kernel ~5.5k: the
+// sums' warps also write dZ (~2k per stage, the store path), during which no
+// accumulator is free.
 //
 // CTAs run as cluster pairs (tcgen05.mma.cta_group::2, M = 256): each CTA
 // converts its half of either operand's columns, the even CTA issues. Both operands
@@ -219,6 +219,8 @@ __device__ __forceinline__ uint32_t next_part(float &x, float &y) {
   return p;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Eight values of a row to the three parts' 16-byte chunks at dst.
 __device__ __forceinline__ void split_store(const float4 &u, const float4 &v, uint32_t dst) {
   float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
@@ -285,19 +287,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         pb = bc < half ? z + (int)crank * half + bc : nullptr;
       }
     };
-    // A stage's rows into L2: a lane fetches this CTA's columns of one row of
-    // either operand.
+    // A stage's rows into L2: a lane fetches half of this CTA's columns of one
+    // row of either operand (lines of 128 bytes; a bulk prefetch per row took
+    // its warp 2k cycles a stage).
     auto prefetch = [&](const Job &job, int st) {
-      const int i = w * 32 + lane;
-      if (i >= 128) return;
-      const bool tape = (i < 64) != job.flip;
-      const long long m = (long long)st * kRows + (i & 63);
-      // columns of A in this CTA, then of B
-      const int first = (int)crank * (i < 64 ? 128 : job.flip ? 64 : job.N / 2);
-      const int count = i < 64 ? 128 : job.flip ? 64 : job.N / 2;
-      if (m >= n || (job.flip && (i < 64 ? first >= job.N : crank == 1))) return;
-      const float *src = tape ? acts + m * kActsLd + job.col : dz + ((long long)job.slot * n + m) * 256;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + first), "r"(count * 4) : "memory");
+      const int i = w * 32 + lane, is_b = i >> 7;
+      const bool tape = (is_b != 0) == job.flip;
+      const long long m = (long long)st * kRows + ((i >> 1) & 63);
+      const int cols = !is_b ? 128 : job.flip ? 64 : job.N / 2;  // of this CTA
+      const int first = (int)crank * cols + (i & 1) * (cols / 2);
+      if (m >= n || (job.flip && (is_b ? crank == 1 : first >= job.N))) return;
+      const float *src = (tape ? acts + m * kActsLd + job.col : dz + ((long long)job.slot * n + m) * 256) + first;
+      prefetch_l2(src);
+      if (cols == 128) prefetch_l2(src + 32);
     };
 #pragma unroll 1
     for (int j = 0; j < kJobs && ok; ++j) {
@@ -535,12 +537,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           const long long tile0 = (long long)(first + t + s) * 256 + crank * 128, row = tile0 + r;
-          // the next layer's mask into L2, a row per lane
-          if (g > 1 && w < 4 && tile0 + w * 32 + lane < n)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(acts + (tile0 + w * 32 + lane) * kActsLd +
-                                                                             acts_offset(g - 2)),
-                         "r"(1024)
-                         : "memory");
+          // the next layer's mask into L2, half a row per lane
+          if (g > 1 && tile0 + w * 16 + lane / 2 < n) {
+            const float *next = acts + (tile0 + w * 16 + lane / 2) * kActsLd + acts_offset(g - 2) + 128 * (lane & 1);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) prefetch_l2(next + 32 * i);
+          }
           // This layer's mask for lane `lane` of sum warp w: its columns of the
           // rows mrow + 8 rr (a bit each), one rr per stage.
           const long long mrow = tile0 + 32 * (w & 3) + lane / 4;
