@@ -1,12 +1,15 @@
 // NeRF MLP (nerf/core/model.py:334-394): weight packing, the FP32 SIMT
 // forward (the plain path) and the precision dispatcher.
 //
-// FP32 SIMT forward: one CTA of 256 threads owns a 64-row tile, two CTAs per
-// SM. The tile's activations stay in shared memory for all ten GEMM layers
-// (X[64][320]: hidden state in columns 0..255, enc_xyz in 256..319, later
-// enc_dir in 256..287); the product and its tiling are fp32_tile.cuh's. 100,003
-// rows: 2.21 ms, 54 TFLOP/s (3.18 ms with one CTA per SM, scalar FMAs and
-// warps of 8 rows x 256 columns), the same outputs bit for bit.
+// FP32 SIMT forward: one CTA of 256 threads owns a tile of 64 rows (or fewer:
+// launch_fp32), two CTAs per SM. The tile's activations stay in shared memory
+// for all ten GEMM layers (X[rows][320]: hidden state in columns 0..255, enc_xyz
+// in 256..319, later enc_dir in 256..287); the product and its tiling are
+// fp32_tile.cuh's. 100,003 rows: 2.12 ms, 56 TFLOP/s (3.18 ms with one CTA per
+// SM, scalar FMAs and warps of 8 rows x 256 columns), the same outputs bit for
+// bit. (The split products of gemm_fp32_tc.cu would be several times faster, but
+// not the same bits: the training forward's ReLU masks decide the gradient, and
+// the forward and the training forward give the same values.)
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -79,10 +82,10 @@ __global__ void fp8_scale_kernel(const float *__restrict__ flat, unsigned char *
 // ---------------------------------------------------------------------------
 // FP32 SIMT forward
 // ---------------------------------------------------------------------------
-using fp32::kTM;
 using fp32::kXLD;
 
-// Copies columns [c0, c0 + nc) of the tile's X rows to acts[row][off ..].
+// Copies columns [c0, c0 + nc) of the tile's kTM X rows to acts[row][off ..].
+template <int kTM>
 __device__ __forceinline__ void store_cols(float *__restrict__ acts, long long row0, long long n, const float *X,
                                            int c0, int nc, int off, int tid) {
   const int per_row = nc / 4;
@@ -97,17 +100,18 @@ __device__ __forceinline__ void store_cols(float *__restrict__ acts, long long r
 // STORE: also write every layer's post-activation rows to `acts` (training).
 // rm: optional row map (logical row k reads and writes physical row
 // rm.map[k]) and device row count; not used with STORE.
-template <bool STORE>
+template <bool STORE, int RI>
 __global__ void __launch_bounds__(fp32::kThreads, 2)
     mlp_fp32_kernel(const float *__restrict__ pk, const float *__restrict__ xyz,
                     const float *__restrict__ dirs, long long n_max, int rpd, float *__restrict__ rgb,
                     float *__restrict__ sigma, float *__restrict__ acts, RowMap rm) {
+  constexpr int kTM = 8 * RI;  // rows per tile
   extern __shared__ __align__(16) float sm[];
   float *X = sm;
   float *Wb = sm + kTM * kXLD;
   const float *table = pk + kFp32TableOff;
   const int tid = threadIdx.x;
-  const fp32::Place p256(tid, 256), p128(tid, 128);
+  const fp32::Place<RI> p256(tid, 256), p128(tid, 128);
   const long long n = rm.n_dev ? min((long long)*rm.n_dev, n_max) : n_max;
   const long long ntiles = (n + kTM - 1) / kTM;
   auto phys = [&](long long k) -> long long {
@@ -146,13 +150,13 @@ __global__ void __launch_bounds__(fp32::kThreads, 2)
       const int gn = g + 1 < kNumGemm ? g + 1 : 0;
       const float *W = pk + gemm_w_offset(g), *Wn = pk + gemm_w_offset(gn);
       const int next_n = more ? gemm_n(gn) : 0;
-      float acc[8][8];
+      float acc[RI][8];
       if (N == 256)
-        fp32::layer<256>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p256, acc);
+        fp32::layer<256, RI>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p256, acc);
       else
-        fp32::layer<128>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p128, acc);
+        fp32::layer<128, RI>(X, Wb, buf, W, gemm_kp(g), kin, Wn, next_n, tid, p128, acc);
       // Epilogue: bias (+ReLU) into X[:, 0..N).
-      const fp32::Place &pl = N == 256 ? p256 : p128;
+      const fp32::Place<RI> &pl = N == 256 ? p256 : p128;
       const float *bias = table + bias_offset(g);
       const bool relu = gemm_relu(g);
 #pragma unroll
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(fp32::kThreads, 2)
         const int col = pl.col(h);
         float4 bv = *reinterpret_cast<const float4 *>(bias + col);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < RI; ++i) {
           float4 v = make_float4(acc[i][4 * h] + bv.x, acc[i][4 * h + 1] + bv.y, acc[i][4 * h + 2] + bv.z,
                                  acc[i][4 * h + 3] + bv.w);
           if (relu) {
@@ -194,19 +198,19 @@ __global__ void __launch_bounds__(fp32::kThreads, 2)
       }
       __syncthreads();
       if (STORE) {
-        store_cols(acts, row0, n, X, 0, N, acts_offset(g), tid);
-        if (g == 0) store_cols(acts, row0, n, X, 256, 64, kActsEncXyz, tid);
-        if (g == 8) store_cols(acts, row0, n, X, 256, 32, kActsEncDir, tid);
+        store_cols<kTM>(acts, row0, n, X, 0, N, acts_offset(g), tid);
+        if (g == 0) store_cols<kTM>(acts, row0, n, X, 256, 64, kActsEncXyz, tid);
+        if (g == 8) store_cols<kTM>(acts, row0, n, X, 256, 32, kActsEncDir, tid);
       }
       if (g == 7) {
         // sigma = ReLU(h7 . w + b) (model.py:374-375).
-        int r = tid >> 2, part = tid & 3;
+        int r = tid >> 2, part = tid & 3;  // (r < kTM by whole warps)
         const float *sw = table + kSigmaWOff;
         float s = 0.0f;
-        for (int k = part * 64; k < part * 64 + 64; ++k) s = fmaf(X[r * kXLD + k], sw[k], s);
+        for (int k = part * 64; r < kTM && k < part * 64 + 64; ++k) s = fmaf(X[r * kXLD + k], sw[k], s);
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (part == 0 && row0 + r < n) sigma[phys(row0 + r)] = fmaxf(s + table[kSigmaBOff], 0.0f);
+        if (part == 0 && r < kTM && row0 + r < n) sigma[phys(row0 + r)] = fmaxf(s + table[kSigmaBOff], 0.0f);
         __syncthreads();
       }
     }
@@ -252,32 +256,64 @@ extern "C" int nerfgb_mlp_pack(const float *params, int precision, void *packed,
 }
 
 namespace nerfgb {
-int launch_mlp_fp32(const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
-                    float *rgb, float *sigma, cudaStream_t stream, const RowMap &rm) {
-  if (cudaFuncSetAttribute(mlp_fp32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) !=
+// Rows per tile, 8 RI. A wave of two CTAs per SM takes 406, 355, 317, 234, 195
+// us for RI = 8, 7, 6, 4, 2 (about RI + 3 units), and about half where an SM has
+// one CTA: up to one tile per SM, or up to half as many tiles left for the last
+// wave (the first CTAs; more of them share SMs). The RI with the least half
+// waves * (RI + 3) is taken: a last wave that 64-row tiles would leave nearly
+// empty then costs less, and a small batch spreads over more SMs (100,003 rows
+// 2.21 -> 2.12 ms, 20,000: 0.59 -> 0.52, 1,000: 229 -> 118 us). Every output is
+// the same chain of FMAs whatever RI.
+static long long half_waves(long long tiles, int sms) {
+  const long long rest = tiles % (2 * sms);
+  return tiles / (2 * sms) * 2 + (rest == 0 ? 0 : tiles <= sms || rest <= sms / 2 ? 1 : 2);
+}
+
+template <bool STORE, int RI>
+static int launch_fp32_tiles(int sms, const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
+                             float *rgb, float *sigma, float *acts, cudaStream_t stream, const RowMap &rm) {
+  constexpr size_t smem = fp32::smem_of(RI);
+  if (cudaFuncSetAttribute(mlp_fp32_kernel<STORE, RI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return NERFGB_E_CUDA;
-  long long ntiles = (n + kTM - 1) / kTM;
-  int sms = num_sms();
-  if (sms <= 0) return NERFGB_E_DEVICE;
-  const int grid = (int)(ntiles < 2 * sms ? ntiles : 2 * sms);  // two CTAs per SM
-  mlp_fp32_kernel<false><<<grid, 256, fp32::kSmem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs,
-                                                            n, rpd, rgb, sigma, nullptr, rm);
+  const long long tiles = (n + 8 * RI - 1) / (8 * RI);
+  mlp_fp32_kernel<STORE, RI><<<(int)(tiles < 2 * sms ? tiles : 2 * sms), fp32::kThreads, smem, stream>>>(
+      reinterpret_cast<const float *>(packed), xyz, dirs, n, rpd, rgb, sigma, acts, rm);
   return launch_status();
+}
+
+template <bool STORE>
+static int launch_fp32(const void *packed, const float *xyz, const float *dirs, long long n, int rpd, float *rgb,
+                       float *sigma, float *acts, cudaStream_t stream, const RowMap &rm) {
+  const int sms = num_sms();
+  if (sms <= 0) return NERFGB_E_DEVICE;
+  constexpr int sizes[5] = {8, 7, 6, 4, 2};
+  int best = 8;
+  long long least = 0;
+  for (int ri : sizes) {
+    const long long cost = half_waves((n + 8 * ri - 1) / (8 * ri), sms) * (ri + 3);
+    if (least == 0 || cost < least) {
+      least = cost;
+      best = ri;
+    }
+  }
+  switch (best) {
+    case 7: return launch_fp32_tiles<STORE, 7>(sms, packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, rm);
+    case 6: return launch_fp32_tiles<STORE, 6>(sms, packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, rm);
+    case 4: return launch_fp32_tiles<STORE, 4>(sms, packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, rm);
+    case 2: return launch_fp32_tiles<STORE, 2>(sms, packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, rm);
+    default: return launch_fp32_tiles<STORE, 8>(sms, packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, rm);
+  }
+}
+
+int launch_mlp_fp32(const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
+                    float *rgb, float *sigma, cudaStream_t stream, const RowMap &rm) {
+  return launch_fp32<false>(packed, xyz, dirs, n, rpd, rgb, sigma, nullptr, stream, rm);
 }
 
 int launch_mlp_fp32_store(const void *packed, const float *xyz, const float *dirs, long long n, int rpd,
                           float *rgb, float *sigma, float *acts, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(mlp_fp32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp32::kSmem) !=
-      cudaSuccess)
-    return NERFGB_E_CUDA;
-  long long ntiles = (n + kTM - 1) / kTM;
-  int sms = num_sms();
-  if (sms <= 0) return NERFGB_E_DEVICE;
-  const int grid = (int)(ntiles < 2 * sms ? ntiles : 2 * sms);
-  mlp_fp32_kernel<true><<<grid, 256, fp32::kSmem, stream>>>(reinterpret_cast<const float *>(packed), xyz, dirs, n,
-                                                           rpd, rgb, sigma, acts, RowMap());
-  return launch_status();
+  return launch_fp32<true>(packed, xyz, dirs, n, rpd, rgb, sigma, acts, stream, RowMap());
 }
 }  // namespace nerfgb
 
