@@ -92,22 +92,6 @@ __global__ void pack_kernel(const float *__restrict__ W, uint8_t *__restrict__ o
   *reinterpret_cast<__nv_bfloat16 *>(out + byte) = __float2bfloat16_rn(W[gemm_w_offset(g) + e]);
 }
 
-// A 3-D box (tma_store_3d's coordinates) into this CTA's shared memory,
-// completing on its own barrier, or on the pair's even CTA's.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *map, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
-          "r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void *map, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-      "%4}], [%5];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&m)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(m[0]), "=r"(m[1]), "=r"(m[2]), "=r"(m[3])

@@ -77,11 +77,11 @@ int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts
 int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t stream);
 
 // Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
-// layer's In^T dZ over M rows added to the flat gradient blob, In from the
-// BF16 tape, dz [10][M][256] BF16; part: gemm_dw_partial_floats(M) floats.
-int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long M, float *grads, float *part, int *err,
+// layer's In^T dZ over n rows added to the flat gradient blob, In from the
+// BF16 tape, dz [10][n][256] BF16; part: gemm_dw_partial_floats() floats.
+int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part, int *err,
                    cudaStream_t stream);
-long long gemm_dw_partial_floats(long long M);
+long long gemm_dw_partial_floats();
 // The BF16 (pair) or FP8 tensor-core forward with a chosen limit on every
 // bounded wait (ns) and the weight chunk at position `withhold` of the load
 // sequence of the (even) CTA left unloaded, so that a wait runs out: the

@@ -22,7 +22,7 @@ namespace train16 {
 constexpr long long kChunkRows = 1LL << 20;
 
 struct Ws {
-  float *dsp, *part;    // dpre_sigma, dW split partials
+  float *dsp, *part;    // dpre_sigma, the dW kernel's partial sums
   __nv_bfloat16 *dz;    // [10][rows][256]
   void *wpack;          // the chain's BF16 weights
   long long bytes;
@@ -42,7 +42,7 @@ static Ws carve(void *base, long long n) {
   w.dz = reinterpret_cast<__nv_bfloat16 *>(take(kNumGemm * rows * 256 * 2));
   w.dsp = reinterpret_cast<float *>(take(rows * 4));
   w.wpack = take(mlp_chain_pack_bytes());
-  w.part = reinterpret_cast<float *>(take(gemm_dw_partial_floats(rows) * 4));
+  w.part = reinterpret_cast<float *>(take(gemm_dw_partial_floats() * 4));
   w.bytes = off;
   return w;
 }

@@ -92,6 +92,22 @@ __device__ __forceinline__ void tma_2d_pair(uint32_t dst, const void *map, int x
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// A 3-D box (coordinates 0, c1, c2) into this CTA's shared memory, completing
+// on its own barrier, or on the pair's even CTA's.
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *map, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+          "r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void *map, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+      "%4}], [%5];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
 // A 3-D box from shared memory at src to global memory by a tensor store
 // (the box's image in shared memory: innermost dimension first), in the
 // thread's bulk async-group. Writes to src by other threads must have been
