@@ -64,10 +64,14 @@
 // - dense_0's operand is written as soon as dense_9 is done, before the rgb
 //   head, and its MMAs wait only for the head's reads of the accumulator.
 // - E4M3's ReLU runs on the packed words (relu_e4m3x4): 484 -> 452 us.
-// - Even deals of 256-row sub-tiles: see above.
+// - Even deals of 256-row sub-tiles: see above. A tile of one sub-tile has no
+//   other one to hide its epilogue under: in BF16 (without the tape, whose
+//   stores bound it) a layer's MMAs start on the first half of its K while the
+//   epilogue writes the second, from the other accumulator (issue_solo: 1,000
+//   rows 31.2 -> 29.3 us).
 // Measured against the kernels before (a 4-stage pair kernel in BF16, one CTA
 // per tile in FP8): 786,432 rows BF16 783 -> 546 us, with the tape 1,613 ->
-// 805, FP8 904 -> 452; 1,000 rows BF16 43 -> 31 us, FP8 41 -> 26. A BF16 tile
+// 805, FP8 904 -> 452; 1,000 rows BF16 43 -> 29 us, FP8 41 -> 26. A BF16 tile
 // takes ~51k cycles, 37k of them MMAs; the largest waits left are the rgb
 // heads at the tile boundary (~5k).
 //
@@ -412,6 +416,38 @@ __device__ __forceinline__ void issue_layer(uint32_t sbase, uint32_t tmem, int n
   if (G > 0) actr_phase ^= 1u;
 }
 
+// BF16, a tile of sub-tile A alone (a pair's odd last one, or a small batch's
+// only one): layer G into accumulator G % 2, so that its MMAs can start on the
+// first 128 K, which the epilogue signals on A's barrier, while the epilogue
+// still reads the accumulator before; the rest follows on B's barrier.
+template <int G>
+__device__ __forceinline__ void issue_solo(uint32_t sbase, uint32_t acc, RingPos &rp, uint32_t &actr_phase,
+                                           uint32_t tile_phase, volatile int *abort_flag, int *err) {
+  using L = Layout<false>;
+  constexpr int N = gemm_n(G), H = N / 2, kPer = (int)kPairStage / (H * 32), kHalf = 8 / kPer;
+  constexpr int kEnc = gemm_kp(G) * 2 / 32 - 16;
+  const uint32_t bar_full = sbase + L::kBarFull, bar_empty = sbase + L::kBarEmpty, sw = sbase & 0x3FFFFu;
+  const uint32_t ring_lo = (sw >> 4) | ((uint32_t)H << 16), act_lo = ((sw + L::kActOff) >> 4) | (1u << 16);
+  wait_fast(sbase + L::kBarActr, actr_phase, abort_flag, err);
+  tc_fence_after();
+  issue_run<L::kNst, kHalf, kPer, H, false, true, true>(bar_full, bar_empty, ring_lo, act_lo, acc, idesc_bf16(256, N), true,
+                                                        rp, abort_flag, err);
+  wait_fast(sbase + L::kBarActr + 8, actr_phase, abort_flag, err);
+  tc_fence_after();
+  issue_run<L::kNst, kHalf, kPer, H, false, false, true>(bar_full, bar_empty, ring_lo, act_lo + 2 * (kAtom >> 4), acc,
+                                                         idesc_bf16(256, N), true, rp, abort_flag, err);
+  if constexpr (kEnc > 0) {
+    wait_fast(sbase + (G == 9 ? L::kBarDir : L::kBarEncA), tile_phase, abort_flag, err);
+    tc_fence_after();
+    issue_run<L::kNst, 1, kEnc, H, false, false, true>(bar_full, bar_empty, ring_lo,
+                                                       ((sw + L::kEncOff) >> 4) | (1u << 16), acc, idesc_bf16(256, N),
+                                                       true, rp, abort_flag, err);
+  }
+  if (G == 5) tc_commit_pair(sbase + L::kBarAcc5);
+  tc_commit_pair(sbase + (G == 9 ? L::kBarAcc9 : L::kBarAccf));
+  actr_phase ^= 1u;
+}
+
 // ---------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------
@@ -569,6 +605,19 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
         const int nsub = 2 * tile + 1 < count ? 2 : 1;
         const uint32_t ph = (uint32_t)(tile & 1);
         issue_layer<0, F8>(sbase, tmem, nsub, rp, actr_phase, ph, abort_flag, err);
+        if (!F8 && !STORE && nsub == 1) {
+          if (tile > 0) {  // the tile before's B has been read
+            wait_fast(sbase + L::kBarAct0 + 8, ph, abort_flag, err);
+            tc_fence_after();
+          }
+#pragma unroll 1
+          for (int g = 1; g <= 4; ++g) issue_solo<1>(sbase, tmem + 256 * (g & 1), rp, actr_phase, ph, abort_flag, err);
+          issue_solo<5>(sbase, tmem + 256, rp, actr_phase, ph, abort_flag, err);
+#pragma unroll 1
+          for (int g = 6; g <= 8; ++g) issue_solo<6>(sbase, tmem + 256 * (g & 1), rp, actr_phase, ph, abort_flag, err);
+          issue_solo<9>(sbase, tmem + 256, rp, actr_phase, ph, abort_flag, err);
+          break;  // (the last tile)
+        }
         // (one copy of the issue code for the layers of one shape: the
         // kernel's code is several times the instruction cache's first levels)
 #pragma unroll 1
@@ -751,15 +800,20 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
         for (int i = 0; i < kPk; ++i) cur[i] = nxt[i];
         const long long grow = row_of(tile, s, r);
         const long long p = phys(grow);
-        {
+        if (F8) {
           const float a = tmem_ld1(tlane + s * 256 + 254), b = tmem_ld1(tlane + s * 256 + 255);
           if (grow < n) sigma_out[p] = fmaxf((a + b) + table[kSigmaBOff], 0.0f);
+        } else {
+          float q[4];
+          tmem_ld4(tlane + s * 256 + 252, q);
+          if (grow < n) sigma_out[p] = fmaxf(((q[0] + q[1]) + (q[2] + q[3])) + table[kSigmaBOff], 0.0f);
         }
+        const uint32_t acc9 = tlane + (!F8 && !STORE && nsub == 1 ? 256 : s * 256);  // dense_9's accumulator
         // rgb = sigmoid(h9 . W + b) in FP32. BF16: ((q0 + q1) + (q2 + q3)) of the
         // quarters' sums of 32 columns; FP8: the 128 columns in order.
         float rgb[3] = {0.f, 0.f, 0.f}, half[3] = {0.f, 0.f, 0.f};
         uint32_t ra[16], rb[16];
-        tmem_ld16(tlane + s * 256, ra);
+        tmem_ld16(acc9, ra);
 #pragma unroll 1
         for (int j = 0; j < 4; ++j) {
           float acc[3];
@@ -773,11 +827,13 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
             const int col = 32 * j + 16 * k;
             tmem_wait16(raw);
             if (k == 0)
-              tmem_ld16(tlane + s * 256 + col + 16, rb);
+              tmem_ld16(acc9 + col + 16, rb);
             else if (j < 3)
-              tmem_ld16(tlane + s * 256 + col + 16, ra);
+              tmem_ld16(acc9 + col + 16, ra);
             else if (s < next_subs)
               start_layer0(s);  // the accumulator is read
+            else if (!F8 && !STORE && next_subs == 1)
+              arrive_even(sbase + L::kBarAct0 + 8);  // B's, which a tile alone uses too
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
               const float4 b4 = F8 ? lds_here(sbase + L::kHeadB + 4 * (col + i)) : from_lane(bias9, (col + i) / 4);
@@ -848,7 +904,8 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
     // ---------------- epilogue warps ----------------
     // All eight warps serve whichever sub-tile's accumulator is ready (A, then
     // B, every layer but dense_9). Warp w reads TMEM lane quadrant qd = w % 4
-    // (rows 32*qd ..) and column part cq: kCols columns. (Nothing here may
+    // (rows 32*qd ..) and column part cq: kCols columns, in BF16 as 64 in either
+    // half of the layer, so that its first half is written first. (Nothing here may
     // spill: the 28 KB of L1 beside this much shared memory do not hold
     // spilled registers, and each reload is a trip to L2.)
     constexpr int kCols = 256 / kParts;
@@ -856,25 +913,28 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
     const uint32_t tlane = tmem + ((uint32_t)(32 * qd) << 16);
     // stmatrix row of this lane in the part's first atom, and its swizzle (store_frag)
     const uint32_t frag_row = (uint32_t)(32 * qd + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u +
-                              (uint32_t)(cq * kCols * (int)L::kE / 128) * kAtom;
+                              (uint32_t)cq * kAtom;  // (either way the part's first 128 bytes of K)
     const uint32_t cx = (uint32_t)((lane >> 4) ^ (lane & 7));
     auto arrive_local = [&](uint32_t bar) {
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    float sig0 = 0.0f, sig1 = 0.0f;  // the sigma head's part sums
+    // first of the part's columns, and from its first half's to its second's
+    const int pcol = F8 ? kCols * cq : 64 * cq;
+    float sig[2][2] = {};  // the sigma head's sums, of the part (FP8) or of its halves
     uint32_t accf_phase = 0;         // both sub-tiles' accumulator barriers, per layer
     bool ok = true;
 #pragma unroll 1
     for (int tile = 0; tile < ntiles && ok; ++tile) {
       const int nsub = 2 * tile + 1 < count ? 2 : 1;
+      const bool solo = !F8 && !STORE && nsub == 1;  // (issue_solo)
 #pragma unroll 1
       for (int g = 0; g < 9 && ok; ++g) {
 #pragma unroll 1
         for (int s = 0; s < nsub; ++s) {
           // the first biases, while the accumulator is computed
           FragBias<F8> fb[2];
-          const float *fbias = table + bias_offset(g) + kCols * cq, *fscale = scales + bias_offset(g) + kCols * cq;
+          const float *fbias = table + bias_offset(g) + pcol, *fscale = scales + bias_offset(g) + pcol;
           fb[0].load(fbias, fscale, lane & 3);
           fb[1].load(fbias + 32, fscale + 32, lane & 3);
           bool got = wait_bar(sbase + L::kBarAccf + 8 * s, accf_phase, abort_flag, err);
@@ -891,22 +951,43 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
           tc_fence_after();
           // 16 rows x 64 (or 32) columns at a time, each loaded while the one
           // before is stored (dense_8 is linear, model.py:377-378)
-          const uint32_t fr = sbase + L::kActOff + s * L::kActBytes + frag_row, ta = tlane + s * 256 + kCols * cq;
+          const uint32_t fr = sbase + L::kActOff + s * L::kActBytes + frag_row, ta = tlane + (solo ? 256 * (g & 1) : s * 256) + pcol;
+          // the operand of the sub-tile's next layer is written (and its
+          // accumulator read): one arrival per warp on the even CTA's barrier
+          auto operand_done = [&]() {
+            fence_proxy_async();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive_remote(peer_addr(sbase + L::kBarActr + (solo ? 8 : 8 * s), 0));
+              if (STORE) mbar_arrive(sbase + L::kBarTapeRdy + 8 * s);
+            }
+          };
+          // the operand's first half is written (a tile alone)
+          auto first_half = [&]() {
+            if (solo) {
+              fence_proxy_async();
+              tc_fence_before();  // (the accumulator of the layer before, that the MMAs will overwrite, is read)
+              __syncwarp();
+              if (lane == 0) mbar_arrive_remote(peer_addr(sbase + L::kBarActr, 0));
+            }
+          };
           if (!F8 && g != 7) {
             uint32_t ra[32], rb[32];
             tmem_ld_frag64(ta, ra);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-              const uint32_t dst = fr + (uint32_t)c * kAtom;
+              const uint32_t dst = fr + (uint32_t)(2 * c) * kAtom;
               tmem_wait32(ra);
-              tmem_ld_frag64(ta + (16u << 16) + 64 * c, rb);
+              tmem_ld_frag64(ta + (16u << 16) + 128 * c, rb);
               store_frag64<F8>(dst, cx, 0u, ra, fb, g != 8);
               tmem_wait32(rb);
-              if (c == 0) tmem_ld_frag64(ta + 64, ra);
+              if (c == 0) tmem_ld_frag64(ta + 128, ra);
               store_frag64<F8>(dst + 16 * 128, cx, 0u, rb, fb, g != 8);
               if (c == 0) {
-                fb[0].load(fbias + 64, fscale + 64, lane & 3);
-                fb[1].load(fbias + 96, fscale + 96, lane & 3);
+                fb[0].load(fbias + 128, fscale + 128, lane & 3);
+                fb[1].load(fbias + 160, fscale + 160, lane & 3);
+                first_half();
               }
             }
           } else if (g != 7) {
@@ -931,21 +1012,24 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
             tmem_ld_frag32(ta, ra);
 #pragma unroll
             for (int c = 0; c < kCols / 32; ++c) {
-              const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
+              auto at = [](int piece) { return F8 ? 32 * piece : 32 * (piece % 2) + 128 * (piece / 2); };
+              const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * (2 * kAtom)), ch = F8 ? 2u * c : 4u * (c % 2);
               tmem_wait16(ra);
-              tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
+              tmem_ld_frag32(ta + (16u << 16) + at(c), rb);
               store_frag<F8, true>(dst, cx, ch, ra, fb[c % 2], true);
-              tmem_st_frag32(ta + 32 * c, ra);
+              tmem_st_frag32(ta + at(c), ra);
               tmem_wait16(rb);
-              if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
+              if (c + 1 < kCols / 32) tmem_ld_frag32(ta + at(c + 1), ra);
               store_frag<F8, true>(dst + 16 * 128, cx, ch, rb, fb[c % 2], true);
-              tmem_st_frag32(ta + (16u << 16) + 32 * c, rb);
-              if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
+              tmem_st_frag32(ta + (16u << 16) + at(c), rb);
+              if (c + 2 < kCols / 32) fb[c].load(fbias + at(c + 2), fscale + at(c + 2), lane & 3);
+              if (c == 1) first_half();
             }
+            if (solo) operand_done();  // before the sums: dense_8 has the other accumulator
             tmem_wait_st();
-            // the head's FP32 sums: BF16 two of 64 columns each, side by side
-            // and then added, FP8 one over the part's columns in order
-            const uint32_t sw = sbase + L::kHeadW + 4 * kCols * cq;
+            // the head's FP32 sums: BF16 of either half's 64 columns, side by side,
+            // FP8 one over the part's columns in order
+            const uint32_t sw = sbase + L::kHeadW + 4 * pcol;
             float part_sum = 0.0f, second = 0.0f;
             // channel i of the 32 at accumulator column fp8_row (BF16: in place)
             auto add4 = [&](float &sum, const uint32_t(&v)[32], int i, uint32_t w) {
@@ -957,7 +1041,7 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
             };
 #pragma unroll 1
             for (int c = 0; c < kCols / 2; c += 32) {
-              const int c0 = F8 ? 2 * c : c, c1 = F8 ? 2 * c + 32 : c + 64;
+              const int c0 = F8 ? 2 * c : c, c1 = F8 ? 2 * c + 32 : c + 128;
               uint32_t raw[2][32];
               tmem_ld32(ta + c0, raw[0]);
               tmem_ld32(ta + c1, raw[1]);
@@ -976,23 +1060,17 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
                 }
               }
             }
-            if (!F8) part_sum += second;
-            if (s == 0)
-              sig0 = part_sum;
-            else
-              sig1 = part_sum;
+            if (s == 0) {
+              sig[0][0] = part_sum;
+              sig[0][1] = second;
+            } else {
+              sig[1][0] = part_sum;
+              sig[1][1] = second;
+            }
           }
-          // the operand of the sub-tile's next layer is written and its
-          // accumulator read: one arrival per warp on the even CTA's barrier
-          fence_proxy_async();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_remote(peer_addr(sbase + L::kBarActr + 8 * s, 0));
-            if (STORE) mbar_arrive(sbase + L::kBarTapeRdy + 8 * s);
-          }
+          if (!solo || g != 7) operand_done();
           if (g == 8) {
-            // sigma's part sums to the side warps, in columns 254 and 255 of the
+            // sigma's sums to the side warps, in the last columns of the
             // accumulator, which dense_9 does not write: the second part's own,
             // so the first part's warp waits until they have been read
             if (cq == 0 && !__all_sync(0xffffffffu, wait_bar(sbase + L::kBarRead8 + 8 * s, (uint32_t)(tile & 1),
@@ -1001,7 +1079,9 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
               break;
             }
             tc_fence_after();
-            tmem_st1(tlane + s * 256 + 254 + cq, s == 0 ? sig0 : sig1);
+            const uint32_t sums = tlane + s * 256 + (F8 ? 254 : 252) + cq;
+            tmem_st1(sums, s == 0 ? sig[0][0] : sig[1][0]);
+            if (!F8) tmem_st1(sums + 2, s == 0 ? sig[0][1] : sig[1][1]);
             tmem_wait_st();
             tc_fence_before();
             arrive_local(sbase + (cq == 0 ? L::kBarSig : L::kBarRead8) + 8 * s);
