@@ -668,7 +668,7 @@ def main():
             key = tp if tile == 4096 else tp + "_recompute"
             train[key] = {"rays_per_s": 4096 / (tms / 1000.0), "ms_per_step": tms,
                           "gemms": "BF16 tcgen05 GEMMs forward and backward, FP32 accumulation"
-                          if tp == "bf16" else "FP32 SIMT"}
+                          if tp == "bf16" else "FP32 FMA forward, backward products as six BF16 tcgen05 products"}
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

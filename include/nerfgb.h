@@ -399,7 +399,9 @@ long long nerfgb_mlp_backward_workspace_bytes(long long n_rows);
 /* Gradient of sum(d_rgb * rgb + d_sigma * sigma) of the MLP w.r.t. its flat
  * parameter blob (Keras layout, nerfgb_mlp_param_count floats), ACCUMULATED
  * into grad_params. acts from nerfgb_mlp_forward_train on the same rows with
- * the same FP32 pack. d_sigma may be NULL. FP32 throughout. */
+ * the same FP32 pack. d_sigma may be NULL. FP32 accuracy throughout: the
+ * products run on the tensor cores from exact three-part BF16 splits, summed
+ * in FP32. A timeout of their bounded waits leaves NaN in grad_params. */
 int nerfgb_mlp_backward(const void *packed, const float *acts, long long n_rows,
                         const float *d_rgb, const float *d_sigma,
                         float *grad_params, void *workspace, void *stream);
