@@ -12,7 +12,7 @@
 // mask) in and 512 bytes of dZ out, ~5.7k cycles of an SM's share of the
 // copy bandwidth per 128 rows against 2,048 cycles of MMAs. A GEMM kernel and
 // a mask kernel per layer moved 2.5 KB per row and layer for the same: 4.4 ms of
-// a 4,096-ray step's two networks against 1.9 here (10.1 GB, 5.3 TB/s).
+// a 4,096-ray step's two networks against 1.78 here (10.1 GB, 5.7 TB/s).
 //
 // The machinery is the forward's (mlp_tc.cu): cluster pairs on two 256-row
 // sub-tiles (128 rows per CTA), 2-SM MMAs (M = 256, N = 256, B = W as [k][n],
@@ -24,7 +24,8 @@
 //     activations over it: the epilogue reads them there with ldmatrix (the
 //     fragments its accumulator has) and stores the masked result in their
 //     place with stmatrix, so the mask needs no room of its own. The copy's
-//     latency (~1.5k cycles) hides behind the other sub-tile;
+//     latency (~1.5k cycles) hides behind the other sub-tile; what the region
+//     takes next was fetched into L2 a layer earlier (1.80 -> 1.78 ms);
 //   - stores the region to the layer's dZ.
 // Bias sums: a thread's rows, then a reduce-scatter over the warp's row groups
 // and one atomic per column, warp and sub-tile.
@@ -318,6 +319,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_3d(act, &maps.act, row, acts_offset(g - 1) / 64, mask);
             ++masks;
           }
+          // what the region takes after that, into L2
+          if (g > 1)
+            tma_prefetch_3d(&maps.act, row, acts_offset(g - 2) / 64);
+          else if (2 * (tile + 1) + s < count)
+            tma_prefetch_3d(&maps.dz[9], (int)row_of(tile + 1, s), 0);
           if (!wait_bar(rdy, phase, abort_flag, err)) {
             ok = false;
             break;

@@ -108,6 +108,12 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void *map, 
       "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(bar)
       : "memory");
 }
+// The same box into L2 alone.
+__device__ __forceinline__ void tma_prefetch_3d(const void *map, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)),
+               "r"(0), "r"(c1), "r"(c2)
+               : "memory");
+}
 // A 3-D box from shared memory at src to global memory by a tensor store
 // (the box's image in shared memory: innermost dimension first), in the
 // thread's bulk async-group. Writes to src by other threads must have been
