@@ -24,9 +24,10 @@
 // (262,144 rows) dW took 6.2 ms, 1.6 here, and the chain 5.5, 2.1 here. A stage
 // is 3,072 cycles of MMAs. In dw_kernel, which converts both operands with
 // eight warps, it takes ~4.3k (with four of them 7k for the conversion alone,
-// and 12.7k with the MMAs issued by one of them). In chain_kernel ~5.5k: the
-// sums' warps also write dZ (~2k per stage, the store path), during which no
-// accumulator is free.
+// and 12.7k with the MMAs issued by one of them). In chain_kernel ~5.3k: the
+// sums' warps also write dZ (~2k per stage; half the stores, of 16 bytes, took
+// as long, tensor stores through shared memory longer), during which no
+// accumulator is free, and a CTA moves ~0.6 MB per layer and tile through L2.
 //
 // CTAs run as cluster pairs (tcgen05.mma.cta_group::2, M = 256): each CTA
 // converts its half of either operand's columns, the even CTA issues. Both operands
