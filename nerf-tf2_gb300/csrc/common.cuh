@@ -192,6 +192,42 @@ inline int num_sms() {
   return n;
 }
 
+// Programmatic dependent launch of small kernels in a chain: a launch that
+// leaves SMs free is set up while the kernel before it in the stream runs. The
+// kernel's first statement is after_previous(): until the kernel before is
+// complete and its writes are visible nothing of it is read or written. The
+// kernel after may be set up from there on (not before: it would then have been
+// started, its caches cleared, while the kernel before last was running). Not
+// during stream capture, where the launch is an ordinary one. A 61-ray render
+// (five kernels) 84 -> 78 us, an MLP launch of 1,000 rows 29.2 -> 27.0; launches
+// that fill the chip take no part: their waiting CTAs would hold SMs that another
+// stream's kernels could use.
+__device__ __forceinline__ void after_previous() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+inline bool may_overlap(cudaStream_t stream, cudaLaunchAttribute &attr) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  return true;
+}
+template <typename... P, typename... A>
+inline int launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = grid < num_sms() && may_overlap(stream, attr[0]) ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) return NERFGB_E_CUDA;
+  return launch_status();
+}
+
 inline bool aligned(const void *p, unsigned a) { return ((uintptr_t)p % a) == 0; }
 
 // ---------------------------------------------------------------------------

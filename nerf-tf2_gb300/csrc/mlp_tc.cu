@@ -71,7 +71,8 @@
 //   rows 31.2 -> 29.3 us).
 // Measured against the kernels before (a 4-stage pair kernel in BF16, one CTA
 // per tile in FP8): 786,432 rows BF16 783 -> 546 us, with the tape 1,613 ->
-// 805, FP8 904 -> 452; 1,000 rows BF16 43 -> 29 us, FP8 41 -> 26. A BF16 tile
+// 805, FP8 904 -> 452; 1,000 rows BF16 43 -> 27 us, FP8 41 -> 23.5
+// (2 us of either by after_previous, common.cuh). A BF16 tile
 // takes ~51k cycles, 37k of them MMAs; the largest waits left are the rgb
 // heads at the tile boundary (~5k).
 //
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
                 "tape columns in swizzle atoms");
   using L = Layout<F8>;
   extern __shared__ __align__(1024) uint8_t smem[];
+  after_previous();
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L::kAbort);
@@ -1195,7 +1197,7 @@ static int launch_variant(const void *packed, const float *xyz, const float *dir
   const long long subs = (n + tc::kSubRows - 1) / tc::kSubRows;
   if (subs > 0x7fffffffLL) return NERFGB_E_UNSUPPORTED;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -1226,6 +1228,7 @@ static int launch_variant(const void *packed, const float *xyz, const float *dir
   if (max_pairs < 1) return NERFGB_E_UNSUPPORTED;
   const long long pairs = subs < max_pairs ? (subs > 0 ? subs : 1) : max_pairs;
   cfg.gridDim = dim3((unsigned)(2 * pairs));
+  if (pairs < max_pairs && may_overlap(stream, attr[1])) cfg.numAttrs = 2;
   tc::PairMaps maps{};
   int rc = pair_maps(pk, F8, maps);
   if (rc != NERFGB_OK) return rc;

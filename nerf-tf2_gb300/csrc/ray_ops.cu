@@ -23,6 +23,7 @@ __global__ void coarse_sample_kernel(const float *__restrict__ rays_o, const flo
                                      int perturb, int lin_inv, float *__restrict__ xyz, float *__restrict__ dirs,
                                      float *__restrict__ t_out, float *__restrict__ edges,
                                      float *__restrict__ widths) {
+  after_previous();
   long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= (long long)R * S) return;
   int r = (int)(gid / S), i = (int)(gid - (long long)r * S);
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(32 * kCompWarps)
                      float *__restrict__ pred_depth, float *__restrict__ acc_map, float tau,
                      unsigned char *__restrict__ gate_mask, int *__restrict__ gate_map, int *__restrict__ gate_count,
                      float *__restrict__ gate_sig_zero) {
+  after_previous();
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *s_t = smem + warp * (6 * S + 1);
@@ -217,6 +219,7 @@ __global__ void __launch_bounds__(32 * kFineWarps, 8)
                        int Sf, float *__restrict__ xyz, float *__restrict__ dirs,
                        float *__restrict__ t_out, int *__restrict__ piece_idxs,
                        int *__restrict__ sort_perm, int P, FineFuse fz) {
+  after_previous();
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = Sc + Sf;
@@ -564,9 +567,8 @@ int launch_coarse_sample(const float *rays_o, const float *rays_d, const float *
                          float *xyz, float *dirs, float *t_vals, float *edges, float *widths, cudaStream_t stream) {
   const long long n = (long long)R * S;
   if (n == 0) return NERFGB_OK;
-  coarse_sample_kernel<<<grid_for(n, 256), 256, 0, stream>>>(rays_o, rays_d, near, far, u_vals, seed, R, S,
-                                                             perturb, lin_inv, xyz, dirs, t_vals, edges, widths);
-  return launch_status();
+  return launch_after(coarse_sample_kernel, grid_for(n, 256), 256, 0, stream, rays_o, rays_d, near, far, u_vals, seed, R,
+                      S, perturb, lin_inv, xyz, dirs, t_vals, edges, widths);
 }
 }  // namespace nerfgb
 
@@ -606,10 +608,9 @@ int launch_composite(const float *sample_rgb, const float *sigma, const float *t
   int sms = num_sms();
   int blocks = (n_rays + kCompWarps - 1) / kCompWarps;
   int cap = (sms > 0 ? sms : 148) * 16;
-  composite_kernel<<<blocks < cap ? blocks : cap, 32 * kCompWarps, smem, stream>>>(
-      sample_rgb, sigma, t_vals, n_rays, n_samples, white_bg, trans_mode, last_delta, weights, pred_rgb,
-      pred_depth, acc_map, gate.tau, gate.mask, gate.row_map, gate.count, gate.sig_zero);
-  return launch_status();
+  return launch_after(composite_kernel, blocks < cap ? blocks : cap, 32 * kCompWarps, smem, stream, sample_rgb, sigma,
+                      t_vals, n_rays, n_samples, white_bg, trans_mode, last_delta, weights, pred_rgb, pred_depth, acc_map,
+                      gate.tau, gate.mask, gate.row_map, gate.count, gate.sig_zero);
 }
 }  // namespace nerfgb
 
@@ -674,10 +675,9 @@ int launch_fine_sample(const float *rays_o, const float *rays_d, const float *bi
   int sms = num_sms();
   int blocks = (n_rays + kFineWarps - 1) / kFineWarps;
   int cap = (sms > 0 ? sms : 148) * 16;
-  fine_sample_kernel<<<blocks < cap ? blocks : cap, 32 * kFineWarps, smem, stream>>>(
-      rays_o, rays_d, bin_weights, left_edges, ld_left, bin_widths, t_vals_coarse, u_vals, n_rays, n_coarse,
-      n_fine, xyz, dirs, t_vals, piece_idxs, sort_perm, P, fz);
-  return launch_status();
+  return launch_after(fine_sample_kernel, blocks < cap ? blocks : cap, 32 * kFineWarps, smem, stream, rays_o, rays_d,
+                      bin_weights, left_edges, ld_left, bin_widths, t_vals_coarse, u_vals, n_rays, n_coarse, n_fine, xyz,
+                      dirs, t_vals, piece_idxs, sort_perm, P, fz);
 }
 }  // namespace nerfgb
 
