@@ -22,7 +22,9 @@
 // Six BF16 products are still four to five times the rate of the FP32 FMA
 // pipe, which bound the kernels before: of a 1,024-ray step's two networks
 // (262,144 rows) dW took 6.2 ms, 1.6 here, and the chain 5.5, 2.1 here. A stage
-// is 3,072 cycles of MMAs. In dw_kernel, which converts both operands with
+// is 3,072 cycles of MMAs, and ~450 KB through an SM's shared memory and L1 (the
+// MMAs' operands 288, the parts' stores, the loads), 3.6k cycles at 128 bytes per
+// cycle. In dw_kernel, which converts both operands with
 // eight warps, it takes ~4.3k (with four of them 7k for the conversion alone,
 // and 12.7k with the MMAs issued by one of them). In chain_kernel ~5.3k: the
 // sums' warps also write dZ (~2k per stage; half the stores, of 16 bytes, took
