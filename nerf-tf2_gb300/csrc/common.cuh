@@ -209,7 +209,11 @@ __device__ __forceinline__ void after_previous() {
 }
 inline bool may_overlap(cudaStream_t stream, cudaLaunchAttribute &attr) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  if (capture != cudaStreamCaptureStatusNone) return false;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   return true;
@@ -224,8 +228,9 @@ inline int launch_after(void (*kernel)(P...), int grid, int block, size_t smem, 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = grid < num_sms() && may_overlap(stream, attr[0]) ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) return NERFGB_E_CUDA;
-  return launch_status();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  const int rc = launch_status();  // (clears a failed launch's error)
+  return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }
 
 inline bool aligned(const void *p, unsigned a) { return ((uintptr_t)p % a) == 0; }

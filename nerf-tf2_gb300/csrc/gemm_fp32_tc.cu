@@ -768,8 +768,9 @@ static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cuda
   }
   if (most < 1) return NERFGB_E_UNSUPPORTED;
   cfg.gridDim = dim3((unsigned)(2 * (work < most ? work : most)));
-  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return NERFGB_E_CUDA;
-  return launch_status();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  const int rc = launch_status();  // (clears a failed launch's error)
+  return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }
 }  // namespace split
 

@@ -412,8 +412,9 @@ int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, f
         return rc;
     }
   }
-  if (cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, maps) != cudaSuccess) return NERFGB_E_CUDA;
-  if ((rc = launch_status()) != NERFGB_OK) return rc;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, maps);
+  if ((rc = launch_status()) != NERFGB_OK) return rc;  // (clears a failed launch's error)
+  if (e != cudaSuccess) return NERFGB_E_CUDA;
   reduce_kernel<<<red_first(kJobs), kRedElems, 0, st>>>(part, stages, pairs, grads);
   return launch_status();
 }

@@ -511,8 +511,9 @@ int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *ta
     if ((rc = encode_tensor_map_u16(&maps.dz[l], dz + (long long)l * n * 256, 3, dims, strides, box, true)) != NERFGB_OK)
       return rc;
   }
-  if (cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, grads, err, maps) != cudaSuccess) return NERFGB_E_CUDA;
-  return launch_status();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, grads, err, maps);
+  rc = launch_status();  // (clears a failed launch's error)
+  return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }
 
 }  // namespace nerfgb

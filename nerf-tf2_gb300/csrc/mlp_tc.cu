@@ -1245,10 +1245,10 @@ static int launch_variant(const void *packed, const float *xyz, const float *dir
       if ((rc = encode_tensor_map_u16(&maps.tape[i], tape, 3, dims, strides, box, true)) != NERFGB_OK) return rc;
     }
   }
-  if (cudaLaunchKernelEx(&cfg, kern, pk, xyz, dirs, n, rpd, rgb, sigma, err_word, rm, tape, wait_ns, withhold,
-                         maps) != cudaSuccess)
-    return NERFGB_E_CUDA;
-  return launch_status();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, pk, xyz, dirs, n, rpd, rgb, sigma, err_word, rm, tape, wait_ns,
+                                           withhold, maps);
+  rc = launch_status();  // (clears a failed launch's error)
+  return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }
 
 int launch_mlp_bf16(const void *packed, const float *xyz, const float *dirs, long long n, int rpd, float *rgb,
