@@ -281,7 +281,8 @@ __device__ __forceinline__ uint32_t relu_e4m3x4(uint32_t w) {
 // stmatrix row (row 8*((lane>>3)&1) + lane%8 of the 16, chunk 0), cx = (lane>>4) ^
 // (lane & 7) its swizzled chunk in units of 16 bytes, c0 the columns' first
 // chunk in the atom (even).
-// KEEP: raw becomes the ReLU of the FP32 values.
+// KEEP: raw becomes the ReLU of the FP32 values (fmaxf: 0 for NaN, as the sigma
+// head has it; the BF16 operand keeps NaN, as in every other layer).
 template <bool F8, bool KEEP>
 __device__ __forceinline__ void store_frag(uint32_t addr, uint32_t cx, uint32_t c0, uint32_t (&raw)[16],
                                            const FragBias<F8> &fb, bool relu) {
@@ -291,8 +292,9 @@ __device__ __forceinline__ void store_frag(uint32_t addr, uint32_t cx, uint32_t 
   if (KEEP) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      v[i] = fmaxf(v[i], 0.0f);
-      raw[i] = __float_as_uint(v[i]);
+      const float m = fmaxf(v[i], 0.0f);
+      raw[i] = __float_as_uint(m);
+      if (F8) v[i] = m;
     }
   }
   uint32_t w[F8 ? 4 : 8];
