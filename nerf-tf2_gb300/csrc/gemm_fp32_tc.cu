@@ -10,26 +10,34 @@
 // three BF16 values (x rounded, what that leaves rounded, and the rest: 24
 // significant bits in three groups of eight); of the nine products of two such
 // sums the six largest are taken (x0 y0, x0 y1, x1 y0, x1 y1, x0 y2, x2 y0: what
-// is left out is below 2^-24 of the product and of either sign; parts cut off
-// instead of rounded left a bias of 6e-8 per layer), smallest first, in FP32
-// accumulators in TMEM. The tensor core's FP32 accumulation truncates, so an
-// accumulator takes only the 64 terms of one stage (four accumulations at full
-// magnitude) and the stages' sums are added in registers with rounding. The
-// gradient is closer to 64-bit arithmetic than from the chains of FMAs before:
-// 1.7e-7 of its norm for 1,000 rows (5.0e-7), 3.5e-7 for 100,000 (1.1e-6), and
-// for every layer. What is not finite becomes NaN.
+// is left out is below 2^-24 of the product and of either sign).
+//
+// The tensor core's FP32 accumulation truncates. So x0 y0, a product of 16 bits,
+// has an accumulator of its own for the 64 terms of one stage (four
+// accumulations): a sum of few such terms is exact, one of 64 loses little, and
+// the stages' sums are added in registers with rounding. The five low products,
+// smallest first, gather in a second accumulator over a layer of a tile
+// (chain_kernel) or kLow stages (dw_kernel); what truncation takes of them is
+// 2^-8 of that. With all six in one accumulator per stage every product was cut
+// off instead of rounded (a single one off by 5e-8 RMS, mean -4.3e-8) and a
+// layer's dZ came out 4e-8 too small. The gradient's error of its norm against
+// 64-bit arithmetic (from the chains of FMAs before): 1 row 1.0e-7 (2.5e-7),
+// 1,000 rows 1.3e-7 (4.4e-7), 65,536 3.1e-7 (1.3e-6), and for every layer no
+// larger; a single product's 2.6e-8 RMS (2.5e-8; x1 y2 and x2 y1 would make that
+// 2.5e-8 too, and the kernels 22 % slower). What is not finite, or above 3.39e38
+// (BF16's largest), becomes NaN.
 //
 // Six BF16 products are still four to five times the rate of the FP32 FMA
 // pipe, which bound the kernels before: of a 1,024-ray step's two networks
-// (262,144 rows) dW took 6.2 ms, 1.6 here, and the chain 5.5, 2.1 here. A stage
+// (262,144 rows) dW took 6.2 ms, 1.65 here, and the chain 5.5, 2.1 here. A stage
 // is 3,072 cycles of MMAs, and ~450 KB through an SM's shared memory and L1 (the
 // MMAs' operands 288, the parts' stores, the loads), 3.6k cycles at 128 bytes per
-// cycle. In dw_kernel, which converts both operands with
-// eight warps, it takes ~4.3k (with four of them 7k for the conversion alone,
-// and 12.7k with the MMAs issued by one of them). In chain_kernel ~5.3k: the
-// sums' warps also write dZ (~2k per stage; half the stores, of 16 bytes, took
-// as long, tensor stores through shared memory longer), during which no
-// accumulator is free, and a CTA moves ~0.6 MB per layer and tile through L2.
+// cycle. dw_kernel converts both operands with eight warps, which takes longer
+// than the MMAs and the reading of their sums in turn (with four of them 7k
+// cycles per stage, and 12.7k with the MMAs issued by one of them). In
+// chain_kernel the sums' warps also write dZ, and a CTA moves ~0.6 MB per layer
+// and tile through L2 (half the stores, of 16 bytes, took as long, tensor stores
+// through shared memory longer).
 //
 // CTAs run as cluster pairs (tcgen05.mma.cta_group::2, M = 256): each CTA
 // converts its half of either operand's columns, the even CTA issues. Both operands
@@ -39,8 +47,9 @@
 // Warp roles (16 warps): 0-7 add each stage's accumulator to the item's sums,
 // 128 registers per thread, and at the item's end add those to the gradient;
 // 8-15 convert, with rows fetched into L2 ahead of them. Thread 0 of the even
-// CTA issues a stage's MMAs before it adds the stage before. The warp groups
-// trade registers (setmaxnreg): 168 for the sums, 88 for the conversion.
+// CTA issues the MMAs (a 17th warp for that would make the block's registers
+// those of 20). The warp groups trade registers (setmaxnreg): 168 for the sums,
+// 88 for the conversion.
 //
 // Every mbarrier wait is bounded (tc::wait_bar): on a timeout every role
 // stops, the issuer drains its MMAs, TMEM is freed and the CTA writes NaN into
@@ -61,6 +70,7 @@ namespace split {
 using namespace tc;
 
 constexpr int kRows = 64;  // rows (K) per stage
+constexpr int kLow = 8;    // stages per window of low sums (dw_kernel)
 constexpr int kAhead = 4;  // stages fetched into L2 ahead of the one converted
 constexpr int kSumWarps = 8, kConvWarps = 8, kThreads = 32 * (kSumWarps + kConvWarps);
 // Registers of the two kinds of warp group (the block is launched with 128 a thread).
@@ -72,8 +82,8 @@ constexpr uint32_t kOperand = 3 * kPart;
 constexpr uint32_t kStage = 2 * kOperand;        // A, B
 constexpr uint32_t kBar0 = 2 * kStage;
 constexpr uint32_t kBarFull = kBar0;             // [2] operands of the stage written (both CTAs)
-constexpr uint32_t kBarDone = kBar0 + 16;        // [2] its MMAs are complete: stage free, accumulator full
-constexpr uint32_t kBarRead = kBar0 + 32;        // [2] its accumulator has been read (both CTAs)
+constexpr uint32_t kBarDone = kBar0 + 16;        // [2] its MMAs are complete: stage free, accumulators full
+constexpr uint32_t kBarRead = kBar0 + 32;        // they have been read (by both CTAs), once per stage
 constexpr uint32_t kBarB = kBar0 + 48;           // [2] chain: its weights have arrived (both CTAs')
 constexpr uint32_t kBarZ = kBar0 + 64;           // [2] chain: a tile's dZ of the layer is written
 constexpr uint32_t kBarMask = kBar0 + 80;        // [2] chain: a tile's mask of the layer is written
@@ -82,6 +92,7 @@ constexpr uint32_t kTmemSlot = kBar0 + 104;
 constexpr uint32_t kAbort = kBar0 + 112;         // int, then the wait limit (u64) at +8
 constexpr uint32_t kErr = kBar0 + 128;           // int
 constexpr uint32_t kMask = kBar0 + 144;          // [2][256 threads] chain: mask bits, 16 bytes each
+constexpr uint32_t kShare = kMask;               // [12] dw: Share of a job
 constexpr uint32_t kSmem = kMask + 2 * 4096;
 static_assert(kSmem <= 227 * 1024, "two stages");
 
@@ -112,6 +123,15 @@ constexpr int cost_sum() {
   return c;
 }
 
+// What the sums' warps need of a job, from shared memory when they do.
+struct __align__(16) Share {
+  int begin, end;         // the pair's stages
+  uint32_t idesc;
+  int to;                 // D's first element in the gradient
+  int rows, cols, rs, cs;  // of D: those that count, their strides in the gradient
+  int part;               // columns per half of the sums' warps
+};
+
 // A pair's stages of job j (every job has `stages`): all jobs' stages in order,
 // each at the sum of the costs before it, are dealt evenly by cost.
 __device__ __forceinline__ void stages_of(int j, int stages, int pair, int pairs, int &b, int &e) {
@@ -135,11 +155,11 @@ __device__ __forceinline__ uint32_t begin(uint8_t *smem, uint32_t sbase, volatil
     for (int s = 0; s < 2; ++s) {
       mbar_init(sbase + kBarFull + 8 * s, 2 * kConvWarps);
       mbar_init(sbase + kBarDone + 8 * s, 1);
-      mbar_init(sbase + kBarRead + 8 * s, 2 * kSumWarps);
       mbar_init(sbase + kBarB + 8 * s, 1);
       mbar_init(sbase + kBarZ + 8 * s, kSumWarps);
       mbar_init(sbase + kBarMask + 8 * s, kConvWarps);
     }
+    mbar_init(sbase + kBarRead, 2 * kSumWarps);
     mbar_init(sbase + kBarDrain, 1);
     *abort_flag = aligned ? 0 : 1;
     *err = 0;
@@ -158,16 +178,50 @@ __device__ __forceinline__ uint32_t begin(uint8_t *smem, uint32_t sbase, volatil
   return *reinterpret_cast<volatile uint32_t *>(smem + kTmemSlot);
 }
 
-// The MMAs of a stage: the six products, smallest first, of K-steps `step`
-// descriptor units apart.
-__device__ __forceinline__ void issue_stage(uint32_t acc, uint64_t a, uint64_t b, uint32_t step, uint32_t idesc) {
+// MMAs of a stage, of K-steps `step` descriptor units apart: of the six products
+// FROM .. TO - 1, the five low ones first, smallest first, into the second
+// accumulator, which `first` starts again, the high one last, into the first.
+template <int FROM, int TO>
+__device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64_t b, uint32_t step, uint32_t idesc,
+                                               bool first) {
   constexpr int px[6] = {0, 2, 1, 0, 1, 0}, py[6] = {2, 0, 1, 1, 0, 0};
+  asm volatile("" : "+l"(a), "+l"(b));  // (the descriptors made here, not kept in registers from stage to stage)
 #pragma unroll
-  for (int i = 0; i < 6; ++i)
+  for (int i = FROM; i < TO; ++i)
 #pragma unroll
     for (int s = 0; s < kRows / 16; ++s)
-      tc_mma_pair(acc, a + px[i] * (kPart >> 4) + s * step, b + py[i] * (kPart >> 4) + s * step, idesc,
-                  i + s > 0 ? 1u : 0u);
+      tc_mma_pair(tmem + (i < 5 ? 256u : 0u), a + px[i] * (kPart >> 4) + s * step, b + py[i] * (kPart >> 4) + s * step,
+                  idesc, (i == 5 && s == 0) || (first && i + s == 0) ? 0u : 1u);
+}
+
+// A warp's part (cols of 128) of an accumulator added to its sums: eight
+// fragments of 16 rows x 32 columns, those from column `cols` on left out.
+__device__ __forceinline__ void add_accumulator(uint32_t taddr, int cols, float (&sum)[4][2][16]) {
+#pragma unroll
+  for (int f = 0; f < 8; ++f) {
+    if (32 * (f / 2) < cols) {
+      uint32_t raw[16];
+      tmem_ld_frag32(taddr + ((uint32_t)(16 * (f % 2)) << 16) + 32 * (f / 2), raw);
+      tmem_wait16(raw);
+      float *s = sum[f / 2][f % 2];
+#pragma unroll
+      for (int i = 0; i < 16; i += 2)
+        add_f32x2(s[i], s[i + 1], s[i], s[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
+    }
+  }
+}
+// By a sums' warp: stage q's high sums, at the end of a window also its low ones,
+// added. False after a timeout.
+__device__ __forceinline__ bool add_stage(uint32_t sbase, uint32_t taddr, uint32_t q, bool low, int cols, int lane,
+                                          float (&sum)[4][2][16], volatile int *abort_flag, int *err) {
+  if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * (q & 1u), (q >> 1) & 1u, abort_flag, err))) return false;
+  tc_fence_after();
+#pragma unroll 1
+  for (uint32_t at = 0; at <= (low ? 256u : 0u); at += 256u) add_accumulator(taddr + at, cols, sum);
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarRead, 0));
+  return true;
 }
 
 // Both CTAs must hold the same TMEM columns (the collective allocation gives them).
@@ -248,6 +302,20 @@ __global__ void __launch_bounds__(kThreads, 1)
   // (the swizzled stages need 1024-byte alignment: without it nothing runs)
   const bool aligned = (sbase & 1023u) == 0;
   const int stages = aligned ? (int)((n + kRows - 1) / kRows) : 0;
+  if (threadIdx.x < kJobs) {
+    const Job job = job_of(threadIdx.x);
+    Share sh;
+    stages_of(threadIdx.x, stages, pair, pairs, sh.begin, sh.end);
+    sh.idesc = idesc_bf16(256, 0) | (1u << 15) | (1u << 16) | ((uint32_t)(job.n_mma() >> 3) << 17);
+    sh.to = (int)flat_offset(job.flat) + job.k_dst0 * job.N;
+    // D's rows are the layer's inputs (flipped: outputs), its columns the outputs (inputs)
+    sh.rows = job.flip ? job.N : job.K;
+    sh.cols = job.flip ? job.K : job.N;
+    sh.rs = job.flip ? 1 : job.N;
+    sh.cs = job.flip ? job.N : 1;
+    sh.part = (job.flip ? 64 : job.N) / 2;
+    reinterpret_cast<Share *>(smem + kShare)[threadIdx.x] = sh;
+  }
 
   const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned);
 
@@ -379,88 +447,54 @@ __global__ void __launch_bounds__(kThreads, 1)
     // that count, as 16 x 32 fragments (tcgen05.cuh).
     const int qd = warp & 3, h = warp >> 2;
     const uint32_t tl = tmem + ((uint32_t)(32 * qd) << 16);
-    // The issuer: one thread of the even CTA, a stage ahead of the sums.
     const bool issuer = crank == 0 && threadIdx.x == 0;
-    int ij = -1, ileft = 0;  // its job, the job's stages left
-    uint32_t iq = 0;
     if (issuer) check_tmem(sbase, tmem, abort_flag);
-    auto issue_next = [&]() {
-      while (ileft == 0) {
-        if (++ij >= kJobs) {
-          ij = kJobs;
-          return;
-        }
-        int b, e;
-        stages_of(ij, stages, pair, pairs, b, e);
-        ileft = e > b ? e - b : 0;
-      }
-      const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
-      --ileft;
-      ++iq;
-      if (!wait_bar(sbase + kBarFull + 8 * k, ph, abort_flag, err) ||
-          !wait_bar(sbase + kBarRead + 8 * k, ph ^ 1u, abort_flag, err))
+    const volatile Share *share = reinterpret_cast<const volatile Share *>(smem + kShare);
+    auto issue = [&](uint32_t q, uint32_t idesc, bool first) {
+      const uint32_t k = q & 1u, sa = sbase + k * kStage;
+      if (!wait_bar(sbase + kBarFull + 8 * k, (q >> 1) & 1u, abort_flag, err) ||
+          !wait_bar(sbase + kBarRead, k ^ 1u, abort_flag, err))
         return;
       tc_fence_after();
-      const uint32_t idesc = idesc_bf16(256, 0) | (1u << 15) | (1u << 16) | ((uint32_t)(job_of(ij).n_mma() >> 3) << 17);
-      const uint32_t sa = sbase + k * kStage, acc = tmem + 256u * k;
-      issue_stage(acc, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc);
+      issue_products<0, 6>(tmem, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc, first);
       tc_commit_pair(sbase + kBarDone + 8 * k);
     };
-    if (issuer) issue_next();
-    __syncwarp();
     bool ok = true;
-    uint32_t q = 0;
+    uint32_t q = 0;  // stages so far
 #pragma unroll 1
     for (int j = 0; j < kJobs && ok; ++j) {
-      const Job job = job_of(j);
-      int sb, se;
-      stages_of(j, stages, pair, pairs, sb, se);
-      if (sb >= se) continue;
-      const int cols = (job.flip ? 64 : job.N) / 2, c0 = h * cols;  // 128, 64 or 32
+      int left = share[j].end - share[j].begin;
+      if (left <= 0) continue;
+      const int cols = share[j].part, c0 = h * cols;
       float sum[4][2][16];
 #pragma unroll
       for (int f = 0; f < 8; ++f)
 #pragma unroll
         for (int i = 0; i < 16; ++i) sum[f / 2][f % 2][i] = 0.0f;
+      int window = 0;  // stages in the window of low sums
 #pragma unroll 1
-      for (int st = sb; st < se; ++st, ++q) {
-        const int k = (int)(q & 1);
-        if (issuer) issue_next();
-        if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, (uint32_t)((q >> 1) & 1), abort_flag, err))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int f = 0; f < 8; ++f) {
-          if (32 * (f / 2) < cols) {
-            uint32_t raw[16];
-            tmem_ld_frag32(tl + ((uint32_t)(16 * (f % 2)) << 16) + 256u * k + c0 + 32 * (f / 2), raw);
-            tmem_wait16(raw);
-            float *s = sum[f / 2][f % 2];
-#pragma unroll
-            for (int i = 0; i < 16; i += 2)
-              add_f32x2(s[i], s[i + 1], s[i], s[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
-          }
-        }
-        tc_fence_before();
+      for (; left > 0 && ok; --left, ++q) {
+        if (issuer) issue(q, share[j].idesc, window == 0);
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarRead + 8 * k, 0));
+        const bool end = left == 1 || ++window == kLow;
+        ok = add_stage(sbase, tl + c0, q, end, cols, lane, sum, abort_flag, err);
+        if (end) window = 0;
       }
       if (!ok) break;
-      // D's rows are the layer's inputs (flipped: outputs), its columns the outputs (inputs)
-      float *dW = grads + flat_offset(job.flat) + (long long)job.k_dst0 * job.N;
+      // (addresses from what is read here: kept over the stages they would spill)
+      const volatile Share &sh = share[j];
+      int l = lane;
+      asm volatile("" : "+r"(l));
+      const int row0 = (int)crank * 128 + 32 * qd + l / 4, cl0 = c0 + 2 * (l % 4);
+      const int rows = sh.rows, cls = sh.cols, rs = sh.rs, cs = sh.cs;
+      float *dW = grads + sh.to + row0 * rs + cl0 * cs;
 #pragma unroll
       for (int f = 0; f < 8; ++f) {
         if (32 * (f / 2) >= cols) continue;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int row = (int)crank * 128 + 32 * qd + 16 * (f % 2) + lane / 4 + 8 * ((i >> 1) & 1);
-          const int cl = c0 + 32 * (f / 2) + 8 * (i / 4) + 2 * (lane % 4) + (i & 1);
-          if (!job.flip)
-            atomicAdd(dW + (long long)row * job.N + cl, sum[f / 2][f % 2][i]);
-          else if (cl < job.K && row < job.N)
-            atomicAdd(dW + (long long)cl * job.N + row, sum[f / 2][f % 2][i]);
+          const int row = 16 * (f % 2) + 8 * ((i >> 1) & 1), cl = 32 * (f / 2) + 8 * (i / 4) + (i & 1);
+          if (row0 + row < rows && cl0 + cl < cls) atomicAdd(dW + row * rs + cl * cs, sum[f / 2][f % 2][i]);
         }
       }
     }
@@ -627,24 +661,30 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool issuer = crank == 0 && threadIdx.x == 0;
     const uint32_t total = (uint32_t)count * first_chunk(0);
     if (issuer) check_tmem(sbase, tmem, abort_flag);
-    uint32_t iq = 0;  // stages issued
-    auto issue = [&]() {
-      if (iq >= total) return;
-      const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
-      ++iq;
-      if (!wait_bar(sbase + kBarFull + 8 * k, ph, abort_flag, err) ||
-          !wait_bar(sbase + kBarB + 8 * k, ph, abort_flag, err) ||
-          !wait_bar(sbase + kBarRead + 8 * k, ph ^ 1u, abort_flag, err))
-        return;
+    auto desc = [&](uint32_t addr) { return (uint64_t)kDescHiA << 32 | ((addr & 0x3FFFFu) >> 4) | (1u << 16); };
+    // Stage q is issued in two parts: kEarly of its low products as soon as its
+    // operands are there, under the reading of the accumulators of the stage
+    // before (unless that reads the low sums too), then the rest.
+    constexpr int kEarly = 2;
+    auto early = [&](uint32_t q, bool first) {
+      const uint32_t sa = sbase + (q & 1u) * kStage;
       tc_fence_after();
-      const uint32_t sa = (sbase + k * kStage) & 0x3FFFFu;
-      const uint64_t hi = (uint64_t)kDescHiA << 32;
-      issue_stage(tmem + 256u * k, hi | (sa >> 4) | (1u << 16), hi | ((sa + kOperand) >> 4) | (1u << 16), 32 >> 4,
-                  idesc_bf16(256, 256));
+      issue_products<0, kEarly>(tmem, desc(sa), desc(sa + kOperand), 32 >> 4, idesc_bf16(256, 256), first);
+    };
+    auto issue = [&](uint32_t q, bool first, bool begun) {
+      const uint32_t k = q & 1u, ph = (q >> 1) & 1u, sa = sbase + k * kStage;
+      if ((!begun && (!wait_bar(sbase + kBarFull + 8 * k, ph, abort_flag, err) ||
+                      !wait_bar(sbase + kBarB + 8 * k, ph, abort_flag, err))) ||
+          !wait_bar(sbase + kBarRead, k ^ 1u, abort_flag, err))
+        return;
+      if (!begun) early(q, first);
+      tc_fence_after();
+      issue_products<kEarly, 6>(tmem, desc(sa), desc(sa + kOperand), 32 >> 4, idesc_bf16(256, 256), false);
       tc_commit_pair(sbase + kBarDone + 8 * k);
     };
     bool ok = true;
-    uint32_t q = 0;
+    uint32_t q = 0, iq = 0;  // stages so far, stages issued
+    bool begun = false;      // of stage iq the early part is
 #pragma unroll 1
     for (int t = 0; t < count && ok; t += 2) {
       const int subs = min(2, count - t);
@@ -662,30 +702,19 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int i = 0; i < 16; ++i) sum[f / 2][f % 2][i] = 0.0f;
 #pragma unroll 1
           for (int ch = 0; ch < chunks; ++ch, ++q) {
-            const uint32_t k = q & 1u;
+            const bool last = ch + 1 == chunks;
             if (issuer) {
-              if (iq == q) issue();
-              // a stage ahead, unless that waits for the dZ of this one (a tile alone)
-              if (iq == q + 1 && (subs == 2 || ch + 1 < chunks)) issue();
+              if (iq == q) issue(iq++, ch == 0, begun);
+              const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
+              begun = !last && mbar_test(sbase + kBarFull + 8 * k, ph) && mbar_test(sbase + kBarB + 8 * k, ph);
+              if (begun) early(iq, false);
             }
-            if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * k, (q >> 1) & 1u, abort_flag, err))) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-#pragma unroll
-            for (int f = 0; f < 8; ++f) {
-              uint32_t raw[16];
-              tmem_ld_frag32(tl + ((uint32_t)(16 * (f % 2)) << 16) + 256u * k + 32 * (f / 2), raw);
-              tmem_wait16(raw);
-              float *a = sum[f / 2][f % 2];
-#pragma unroll
-              for (int i = 0; i < 16; i += 2)
-                add_f32x2(a[i], a[i + 1], a[i], a[i + 1], __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
-            }
-            tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarRead + 8 * k, 0));
+            if (!(ok = add_stage(sbase, tl, q, last, 128, lane, sum, abort_flag, err))) break;
+            // the next layer's (the other tile's) first stage under the writing of
+            // dZ, unless it waits for that (a tile alone)
+            if (issuer && last && subs == 2 && iq < total) issue(iq++, true, false);
+            __syncwarp();
           }
           if (!ok) break;
           // dense_9's input, the bottleneck, is linear: no mask
