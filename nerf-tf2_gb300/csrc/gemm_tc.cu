@@ -16,14 +16,16 @@
 // all jobs in order are dealt evenly to the pairs, so a pair has one or two
 // layers' sums at a time. The tensor core's FP32 accumulation
 // truncates (4e-6 relative over 4,096 rows of random signs), so an accumulator
-// takes kWindow stages and the windows' sums are added in registers with
-// rounding, one accumulator in TMEM being read while the other fills. A layer's
-// pairs leave partial sums in a workspace that one reduction kernel adds into
-// the gradient, always in the same order. With the accumulators themselves as
-// the partial sums a layer had to be split 152 times (up to ~5,000 rows each)
-// and their 0.48 GB were written and read per network: 2.0 ms of the step, and
-// 0.22 for the reduction; 1.73 and 0.04 here (6.5 TB/s). The gradient of 786,432
-// rows is 6e-7 - 7e-7 of its norm from the sum over 4,096-row calls (4e-6 - 6e-6).
+// takes a window of 1, 2 or 4 stages (launch_gemm_dw) and the windows' sums are
+// added in registers with rounding, one accumulator in TMEM being read while the
+// other fills. A layer's pairs leave partial sums in a workspace that one
+// reduction kernel adds into the gradient, always in the same order, without the
+// additions' rounding. With the accumulators themselves as the partial sums a
+// layer had to be split 152 times (up to ~5,000 rows each) and their 0.48 GB were
+// written and read per network: 2.0 ms of the step, and 0.22 for the reduction;
+// 1.73 and 0.04 here (6.5 TB/s). Error of the sums against 64 bits, from the same
+// dZ, of their norm (as split 152 times): 1,000 rows 6e-8 (7e-8), 20,000 1.3e-7
+// (1.6e-7), 786,432 4e-7 (5e-6).
 //
 // Warp roles (12 warps): 0-7 the windows' sums (TMEM lane quadrant w % 4, column
 // half w / 4; 128 registers each), 8 the loader (one thread, a kNst-stage ring,
@@ -48,7 +50,6 @@ namespace gemm {
 using namespace tc;
 
 constexpr int kRows = 64;   // rows (K) per stage: 4 MMAs of K = 16
-constexpr int kWindow = 4;  // stages per accumulator
 constexpr int kSumWarps = 8, kLoadWarp = 8, kIssuerWarp = 9, kThreads = 12 * 32;
 constexpr uint32_t kAtomBytes = 64 * 128;  // 64 columns x kRows rows
 constexpr uint32_t kOperand = 2 * kAtomBytes;
@@ -119,7 +120,8 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    dw_kernel(float *__restrict__ part, int *__restrict__ err, long long n, const __grid_constant__ Maps maps) {
+    dw_kernel(float *__restrict__ part, int *__restrict__ err, long long n, int window,
+              const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -210,8 +212,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         long long sb, se;
         stages_of(j, stages, pair, pairs, sb, se);
         const uint32_t idesc = idesc_bf16(256, 0) | (1u << 15) | (1u << 16) | ((uint32_t)(job.n_mma() >> 3) << 17);
-        for (long long i = sb; i < se && !*abort_flag; i += kWindow, ++w) {
-          const int count = (int)(se - i < kWindow ? se - i : kWindow);
+        for (long long i = sb; i < se && !*abort_flag; i += window, ++w) {
+          const int count = (int)(se - i < window ? se - i : window);
           // the sums have read the window before last
           if (!wait_bar(sbase + kBarRead + 8 * (w & 1), ((w >> 1) & 1u) ^ 1u, abort_flag, err)) break;
           tc_fence_after();
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int i = 0; i < 16; ++i) sum[f / 2][f % 2][i] = 0.0f;
 #pragma unroll 1
-      for (int left = (int)((se - sb + kWindow - 1) / kWindow); left > 0; --left, ++w) {
+      for (int left = (int)((se - sb + window - 1) / window); left > 0; --left, ++w) {
         if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarAcc + 8 * (w & 1), (w >> 1) & 1u, abort_flag, err))) {
           ok = false;
           break;
@@ -346,10 +348,16 @@ __global__ void __launch_bounds__(kRedElems)
   }
   __syncthreads();
   const float *src = part + (long long)(first + j) * 65536 + at;
-  float s = 0.0f;
+  // (with what each addition rounds off kept beside it, as every term is a sum
+  // that was rounded as it grew)
+  float s = 0.0f, rest = 0.0f;
 #pragma unroll 4
-  for (int p = 0; p < count; ++p) s += any[p] ? src[p * 65536LL] : 0.0f;
-  grads[flat_offset(job.flat) + (long long)(job.k_dst0 + k) * job.N + c] += s;
+  for (int p = 0; p < count; ++p) {
+    const float x = any[p] ? src[p * 65536LL] : 0.0f, t = fadd(s, x), y = fsub(t, s);
+    rest = fadd(rest, fadd(fsub(s, fsub(t, y)), fsub(x, y)));
+    s = t;
+  }
+  grads[flat_offset(job.flat) + (long long)(job.k_dst0 + k) * job.N + c] += s + rest;
 }
 
 }  // namespace gemm
@@ -412,7 +420,15 @@ int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, f
         return rc;
     }
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, maps);
+  // Stages per window: short ones for few rows, where what an accumulator cuts
+  // off is most of the error (a pair of 2 to 32 stages: 6e-8 - 9e-8 of the sums'
+  // norm with windows of one, 9e-8 - 1.2e-7 of two, 1.1e-7 - 1.9e-7 of four), longer
+  // ones for many, where it is the additions' rounding (1,940 stages: 7.5e-7 with
+  // one, 5.4e-7 with two, 4.1e-7 with four). The times are alike (786,432 rows 2.82, 2.82,
+  // 2.81 ms of backward).
+  const long long each = kJobs * stages / pairs;
+  const int window = each <= 32 ? 1 : each <= 512 ? 2 : 4;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, window, maps);
   if ((rc = launch_status()) != NERFGB_OK) return rc;  // (clears a failed launch's error)
   if (e != cudaSuccess) return NERFGB_E_CUDA;
   reduce_kernel<<<red_first(kJobs), kRedElems, 0, st>>>(part, stages, pairs, grads);
