@@ -319,8 +319,21 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// A sum with what each addition rounds off kept beside it (TwoSum), for terms
+// that were themselves rounded as they grew.
+struct Sum {
+  float s = 0.0f, rest = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = fadd(s, x), y = fsub(t, s);
+    rest = fadd(rest, fadd(fsub(s, fsub(t, y)), fsub(x, y)));
+    s = t;
+  }
+  __device__ __forceinline__ float total() const { return fadd(s, rest); }
+};
+
 // grads[k_dst0 + k][c] += the job's partial sums, pair after pair; blocks
-// [first(j), first(j + 1)) are job j's, kRedElems elements each.
+// [first(j), first(j + 1)) are job j's, kRedElems elements each; those from
+// first(kJobs) on add the CTAs' bias sums of dense_0 .. dense_8.
 constexpr int kRedElems = 64;
 __host__ __device__ constexpr int red_first(int j) {
   int b = 0;
@@ -330,7 +343,17 @@ __host__ __device__ constexpr int red_first(int j) {
 static_assert(27 * 128 % kRedElems == 0 && 63 * 256 % kRedElems == 0, "whole blocks per job");
 
 __global__ void __launch_bounds__(kRedElems)
-    reduce_kernel(const float *__restrict__ part, long long stages, int pairs, float *__restrict__ grads) {
+    reduce_kernel(const float *__restrict__ part, long long stages, int pairs, const float *__restrict__ bias, int ctas,
+                  float *__restrict__ grads) {
+  if ((int)blockIdx.x >= red_first(kJobs)) {
+    const int e = ((int)blockIdx.x - red_first(kJobs)) * kRedElems + threadIdx.x, l = e / kW;
+    const int fl = flat_idx_of_gemm(l);
+    Sum sum;
+#pragma unroll 8
+    for (int i = 0; i < ctas; ++i) sum.add(bias[(long long)i * kChainBias + e]);
+    grads[flat_offset(fl) + (long long)flat_in(fl) * flat_out(fl) + e % kW] += sum.total();
+    return;
+  }
   int j = 0;
   while (j + 1 < kJobs && (int)blockIdx.x >= red_first(j + 1)) ++j;
   const Job job = job_of(j);
@@ -348,24 +371,18 @@ __global__ void __launch_bounds__(kRedElems)
   }
   __syncthreads();
   const float *src = part + (long long)(first + j) * 65536 + at;
-  // (with what each addition rounds off kept beside it, as every term is a sum
-  // that was rounded as it grew)
-  float s = 0.0f, rest = 0.0f;
+  Sum sum;
 #pragma unroll 4
-  for (int p = 0; p < count; ++p) {
-    const float x = any[p] ? src[p * 65536LL] : 0.0f, t = fadd(s, x), y = fsub(t, s);
-    rest = fadd(rest, fadd(fsub(s, fsub(t, y)), fsub(x, y)));
-    s = t;
-  }
-  grads[flat_offset(job.flat) + (long long)(job.k_dst0 + k) * job.N + c] += s + rest;
+  for (int p = 0; p < count; ++p) sum.add(any[p] ? src[p * 65536LL] : 0.0f);
+  grads[flat_offset(job.flat) + (long long)(job.k_dst0 + k) * job.N + c] += sum.total();
 }
 
 }  // namespace gemm
 
 long long gemm_dw_partial_floats() { return (gemm::kMaxPairs + gemm::kJobs) * 65536LL; }
 
-int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part, int *err,
-                   cudaStream_t st) {
+int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
+                   const float *bias, int ctas, int *err, cudaStream_t st) {
   using namespace gemm;
   if (n == 0) return NERFGB_OK;
   if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
@@ -431,7 +448,8 @@ int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, f
   const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, window, maps);
   if ((rc = launch_status()) != NERFGB_OK) return rc;  // (clears a failed launch's error)
   if (e != cudaSuccess) return NERFGB_E_CUDA;
-  reduce_kernel<<<red_first(kJobs), kRedElems, 0, st>>>(part, stages, pairs, grads);
+  static_assert(kChainBias % kRedElems == 0, "whole blocks of bias sums");
+  reduce_kernel<<<red_first(kJobs) + kChainBias / kRedElems, kRedElems, 0, st>>>(part, stages, pairs, bias, ctas, grads);
   return launch_status();
 }
 

@@ -4,7 +4,7 @@
 // dense_9 down to dense_1,
 //   raw[m][k] = bf16(sum_n dZ_g[m][n] W_g[k][n])            (k < 256)
 //   z = raw (+ dpre_sigma[m] ws[k] below dense_8) (* [h_{g-1}[m][k] > 0])
-//   dZ_{g-1} = bf16(z),  db_{g-1}[k] += sum_m z[m][k]
+//   dZ_{g-1} = bf16(z),  db_{g-1}[k] = sum_m z[m][k]
 // with dZ in shared memory from one layer to the next. dZ of every layer goes
 // to HBM for the weight gradients (gemm_tc.cu).
 //
@@ -28,7 +28,11 @@
 //     takes next was fetched into L2 a layer earlier (1.80 -> 1.78 ms);
 //   - stores the region to the layer's dZ.
 // Bias sums: a thread's rows, then a reduce-scatter over the warp's row groups
-// and one atomic per column, warp and sub-tile.
+// and one atomic per column, warp and sub-tile into the CTA's own sums in the
+// workspace, which the weight gradients' reduction adds up (gemm_tc.cu). With the
+// gradient itself as their target one number took an addition for every 32 rows:
+// of 786,432 rows alike 2e-4 of it was lost, 1e-6 here, and the backward took
+// 2.82 ms, 2.77 here.
 //
 // Every mbarrier wait is bounded; on a timeout the kernel reports, drains and
 // returns as mlp_tc.cu's does.
@@ -172,7 +176,7 @@ __device__ __forceinline__ void add_columns(const float (&sum)[16], int lane, fl
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    chain_kernel(const float *__restrict__ ws, const float *__restrict__ dsp, long long n, float *__restrict__ grads,
+    chain_kernel(const float *__restrict__ ws, const float *__restrict__ dsp, long long n, float *__restrict__ bias,
                  int *__restrict__ err, const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
@@ -188,6 +192,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     count = (sbase & 1023u) != 0 ? 0 : (int)(q + (p < rest ? 1u : 0u));
   }
   const int ntiles = (count + 1) / 2;
+  bias += (long long)blockIdx.x * kChainBias;
+  for (int e = threadIdx.x; e < kChainBias; e += kThreads) bias[e] = 0.0f;
   auto row_of = [&](int k, int s) -> long long {
     return (long long)(first + 2 * k + s) * kSubRows + (int)crank * 128;
   };
@@ -358,9 +364,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int nsub = 2 * tile + 1 < count ? 2 : 1;
 #pragma unroll 1
       for (int g = 9; g >= 1 && ok; --g) {
-        // bias gradient of the layer whose dZ this is (dense_8 below dense_9, dense_{g-1} below dense_g)
-        const int fl = g == 9 ? 9 : g - 1;
-        float *db = grads + flat_offset(fl) + (long long)flat_in(fl) * flat_out(fl) + 128 * hf;
+        // bias gradient of the layer whose dZ this is, dense_{g-1}
+        float *db = bias + (g - 1) * kW + 128 * hf;
 #pragma unroll 1
         for (int s = 0; s < nsub; ++s) {
           const uint32_t dst = sbase + kActOff + s * kActBytes + frag_row, ta = tlane + s * 256;
@@ -455,8 +460,9 @@ int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t st
 }
 
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
-                     __nv_bfloat16 *dz, float *grads, int *err, cudaStream_t stream) {
+                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream) {
   using namespace tcb;
+  *ctas = 0;
   if (n == 0) return NERFGB_OK;
   if (cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
     return NERFGB_E_CUDA;
@@ -487,11 +493,12 @@ int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *ta
       if (cudaOccupancyMaxActiveClusters(&m, chain_kernel, &cfg) != cudaSuccess) return NERFGB_E_CUDA;
       hit = pairs_of_device.emplace(dev, m).first;
     }
-    max_pairs = hit->second;
+    max_pairs = hit->second < kChainMaxPairs ? hit->second : kChainMaxPairs;
   }
   if (max_pairs < 1) return NERFGB_E_UNSUPPORTED;
   const long long subs = (n + kSubRows - 1) / kSubRows, pairs = subs < max_pairs ? subs : max_pairs;
   cfg.gridDim = dim3((unsigned)(2 * pairs));
+  *ctas = (int)(2 * pairs);
   Maps maps{};
   int rc;
   {
@@ -511,7 +518,7 @@ int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *ta
     if ((rc = encode_tensor_map_u16(&maps.dz[l], dz + (long long)l * n * 256, 3, dims, strides, box, true)) != NERFGB_OK)
       return rc;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, grads, err, maps);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, bias, err, maps);
   rc = launch_status();  // (clears a failed launch's error)
   return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }

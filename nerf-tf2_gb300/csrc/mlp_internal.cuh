@@ -54,13 +54,15 @@ int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const
                     const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *grads, cudaStream_t stream);
 
 // The dX products of the BF16 backward (mlp_bwd_tc.cu): dz [10][n][256] BF16,
-// dz[9] in, dz[8] .. dz[0] out, the bias gradients of dense_0 .. dense_8 added
-// to grads. wpack (mlp_chain_pack_bytes, 16-byte aligned) from the FP32 pack's
-// weights by launch_mlp_chain_pack; sigma_w: the sigma head's weights.
+// dz[9] in, dz[8] .. dz[0] out. bias [kChainMaxPairs * 2][kChainBias]: each
+// CTA's sums of the dZ of dense_0 .. dense_8 (256 columns each), of *ctas CTAs.
+// wpack (mlp_chain_pack_bytes, 16-byte aligned) from the FP32 pack's weights by
+// launch_mlp_chain_pack; sigma_w: the sigma head's weights.
+constexpr int kChainMaxPairs = 76, kChainBias = 9 * 256;
 long long mlp_chain_pack_bytes();
 int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t stream);
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
-                     __nv_bfloat16 *dz, float *grads, int *err, cudaStream_t stream);
+                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream);
 
 // The dX products of the FP32 backward (gemm_fp32_tc.cu): dz [10][n][256],
 // dz[9] in (128 columns), dz[8] .. dz[0] out. wpack (fp32_chain_pack_bytes,
@@ -78,9 +80,10 @@ int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads
 
 // Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
 // layer's In^T dZ over n rows added to the flat gradient blob, In from the
-// BF16 tape, dz [10][n][256] BF16; part: gemm_dw_partial_floats() floats.
-int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part, int *err,
-                   cudaStream_t stream);
+// BF16 tape, dz [10][n][256] BF16; part: gemm_dw_partial_floats() floats. With
+// them the chain's bias sums (of `ctas` CTAs).
+int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
+                   const float *bias, int ctas, int *err, cudaStream_t stream);
 long long gemm_dw_partial_floats();
 // The BF16 (pair) or FP8 tensor-core forward with a chosen limit on every
 // bounded wait (ns) and the weight chunk at position `withhold` of the load

@@ -57,3 +57,32 @@ def test_sums_over_few_rows(ng, cuda, n, one_sign):
         # 3.6e-7, 1.1e-7 - 1.9e-7 at 1,000 to 5,000 rows). The few additions of
         # the accumulators round off 2^-25 of the sum each.
         assert err < 1.07e-7, (k, err)
+
+
+@pytest.mark.parametrize("repeats", [33, 8192, 24_576])
+def test_bias_sums_over_many_rows(ng, cuda, repeats):
+    blob = _blob(ng)
+    off = ng.weights.offsets()
+    mlp = ng.get_coarse_or_fine_model("fine", params=blob, precision="bf16")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    x = torch.rand(32, 3, device="cuda", generator=g) * 4 - 2
+    d = torch.nn.functional.normalize(torch.randn(32, 3, device="cuda", generator=g), dim=1)
+    dr, ds = torch.randn(32, 3, device="cuda", generator=g), torch.randn(32, 1, device="cuda", generator=g)
+
+    def grads(k):
+        tape = mlp.forward_train(x.repeat(k, 1), d.repeat(k, 1), precision="bf16")[2]
+        out = torch.zeros(len(blob), device="cuda")
+        mlp.backward(tape, dr.repeat(k, 1), ds.repeat(k, 1), out)
+        return out
+
+    got, want = grads(repeats), grads(1).double() * repeats
+    mlp.check_device_errors()
+    # A CTA adds the sums of 32 rows (a warp's) one after another, at most 216 of
+    # them here (2^20 rows over 152 CTAs); all terms alike, every addition may
+    # round the same way, half a unit of the sum so far: 216 / 2 * 2^-24 = 6.4e-6
+    # at the most. (Added to the gradient itself, 24,576 of them: 1.9e-4.)
+    for k in range(9):
+        _, b, _, o = off[f"dense_{k}"]
+        err = float((got[b:b + o].double() - want[b:b + o]).norm() / want[b:b + o].norm())
+        assert err < 6.4e-6, (k, err)
