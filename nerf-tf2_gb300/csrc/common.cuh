@@ -138,6 +138,18 @@ __device__ __forceinline__ void fma_f32x2(float &d0, float &d1, float x0, float 
       : "f"(x0), "f"(x1), "f"(y0), "f"(y1), "f"(z0), "f"(z1));
 }
 
+// A sum with what each addition rounds off kept beside it (TwoSum), for terms
+// that were themselves rounded as they grew.
+struct Sum {
+  float s = 0.0f, rest = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = fadd(s, x), y = fsub(t, s);
+    rest = fadd(rest, fadd(fsub(s, fsub(t, y)), fsub(x, y)));
+    s = t;
+  }
+  __device__ __forceinline__ float total() const { return fadd(s, rest); }
+};
+
 // fp32(2^l) * fp32(pi): PositionalEncoder multipliers (model.py:309-311).
 __device__ __forceinline__ float enc_multiplier(int l) {
   return fmul((float)(1u << l), 3.14159265358979323846f);

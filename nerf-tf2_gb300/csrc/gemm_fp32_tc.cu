@@ -291,7 +291,8 @@ __device__ __forceinline__ void split_store(const float4 &u, const float4 &v, ui
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, long long n, float *__restrict__ grads) {
+    dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, const float *__restrict__ heads,
+              int head_blocks, long long n, float *__restrict__ grads) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -440,6 +441,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+    // the heads' sums, a warp per element, under the last stages' MMAs
+#pragma unroll 1
+    for (int e = (int)blockIdx.x * kConvWarps + w; e < kHeadSumsFp32; e += (int)gridDim.x * kConvWarps)
+      add_head_sums(heads, head_blocks, e, lane, grads);
   } else {
     // ---------------- the stages' sums (and the issuer) ----------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSumRegs));
@@ -803,11 +808,12 @@ static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cuda
 }
 }  // namespace split
 
-int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t st) {
+int launch_fp32_dw(const float *acts, const float *dz, const float *heads, int head_blocks, long long n, float *grads,
+                   cudaStream_t st) {
   using namespace split;
   if (n == 0) return NERFGB_OK;
   static Pairs pairs;
-  return launch_pairs(dw_kernel, pairs, kJobs * ((n + kRows - 1) / kRows), st, acts, dz, n, grads);
+  return launch_pairs(dw_kernel, pairs, kJobs * ((n + kRows - 1) / kRows), st, acts, dz, heads, head_blocks, n, grads);
 }
 
 long long fp32_chain_pack_bytes() { return split::kPackBytes; }

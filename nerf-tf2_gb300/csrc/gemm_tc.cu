@@ -319,21 +319,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// A sum with what each addition rounds off kept beside it (TwoSum), for terms
-// that were themselves rounded as they grew.
-struct Sum {
-  float s = 0.0f, rest = 0.0f;
-  __device__ __forceinline__ void add(float x) {
-    const float t = fadd(s, x), y = fsub(t, s);
-    rest = fadd(rest, fadd(fsub(s, fsub(t, y)), fsub(x, y)));
-    s = t;
-  }
-  __device__ __forceinline__ float total() const { return fadd(s, rest); }
-};
-
 // grads[k_dst0 + k][c] += the job's partial sums, pair after pair; blocks
 // [first(j), first(j + 1)) are job j's, kRedElems elements each; those from
-// first(kJobs) on add the CTAs' bias sums of dense_0 .. dense_8.
+// first(kJobs) on add the CTAs' bias sums of dense_0 .. dense_8, then the heads'
+// (a warp per element).
 constexpr int kRedElems = 64;
 __host__ __device__ constexpr int red_first(int j) {
   int b = 0;
@@ -344,7 +333,13 @@ static_assert(27 * 128 % kRedElems == 0 && 63 * 256 % kRedElems == 0, "whole blo
 
 __global__ void __launch_bounds__(kRedElems)
     reduce_kernel(const float *__restrict__ part, long long stages, int pairs, const float *__restrict__ bias, int ctas,
-                  float *__restrict__ grads) {
+                  const float *__restrict__ heads, int head_blocks, float *__restrict__ grads) {
+  constexpr int kBiasEnd = red_first(kJobs) + kChainBias / kRedElems;
+  if ((int)blockIdx.x >= kBiasEnd) {
+    const int e = ((int)blockIdx.x - kBiasEnd) * (kRedElems / 32) + threadIdx.x / 32;
+    add_head_sums(heads, head_blocks, e, threadIdx.x % 32, grads);
+    return;
+  }
   if ((int)blockIdx.x >= red_first(kJobs)) {
     const int e = ((int)blockIdx.x - red_first(kJobs)) * kRedElems + threadIdx.x, l = e / kW;
     const int fl = flat_idx_of_gemm(l);
@@ -382,7 +377,7 @@ __global__ void __launch_bounds__(kRedElems)
 long long gemm_dw_partial_floats() { return (gemm::kMaxPairs + gemm::kJobs) * 65536LL; }
 
 int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
-                   const float *bias, int ctas, int *err, cudaStream_t st) {
+                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t st) {
   using namespace gemm;
   if (n == 0) return NERFGB_OK;
   if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
@@ -448,8 +443,9 @@ int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, f
   const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, window, maps);
   if ((rc = launch_status()) != NERFGB_OK) return rc;  // (clears a failed launch's error)
   if (e != cudaSuccess) return NERFGB_E_CUDA;
-  static_assert(kChainBias % kRedElems == 0, "whole blocks of bias sums");
-  reduce_kernel<<<red_first(kJobs) + kChainBias / kRedElems, kRedElems, 0, st>>>(part, stages, pairs, bias, ctas, grads);
+  static_assert(kChainBias % kRedElems == 0 && kHeadSums % (kRedElems / 32) == 0, "whole blocks of bias and head sums");
+  reduce_kernel<<<red_first(kJobs) + kChainBias / kRedElems + kHeadSums / (kRedElems / 32), kRedElems, 0, st>>>(
+      part, stages, pairs, bias, ctas, heads, head_blocks, grads);
   return launch_status();
 }
 

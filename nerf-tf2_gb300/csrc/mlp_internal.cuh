@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
 #include "nerfgb.h"
 
 namespace nerfgb {
@@ -46,12 +47,35 @@ int launch_mlp_bf16_train(const void *packed, const float *xyz, const float *dir
 
 // Backward of the sigma and rgb heads (mlp_train.cu) from an FP32 or a BF16
 // activation tape: dz9 = dL/d(dense_9 pre-activation), row stride 256 (128
-// used), FP32, or BF16 with dense_9's bias gradient added to grads; dsp [n] =
-// dL/d(sigma pre-activation); head gradients into grads.
+// used), FP32 or BF16; dsp [n] = dL/d(sigma pre-activation). sums
+// [kHeadMaxBlocks][kHeadSums]: each block's sums for the gradients of the heads
+// and (BF16) of dense_9's bias, of *blocks blocks; add_head_sums adds one element
+// up, by a warp: the gradient then takes one addition per call, whatever the
+// number of rows and blocks.
+constexpr int kHeadMaxBlocks = 512;
+// the rgb head's kernel [128][3] and bias, the sigma head's kernel [256] and bias
+// (as in the flat blob), dense_9's bias [128]
+constexpr int kHeadSumsFp32 = 644, kHeadSums = 772;
 int launch_head_bwd(const float *table, const float *tape, long long n, const float *d_rgb, const float *d_sigma,
-                    float *dz9, float *dsp, float *grads, cudaStream_t stream);
+                    float *dz9, float *dsp, float *sums, int *blocks, cudaStream_t stream);
 int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const float *d_rgb,
-                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *grads, cudaStream_t stream);
+                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *sums, int *blocks,
+                    cudaStream_t stream);
+__device__ __forceinline__ void add_head_sums(const float *__restrict__ sums, int blocks, int e, int lane,
+                                              float *__restrict__ grads) {
+  Sum sum;
+  for (int b = lane; b < blocks; b += 32) sum.add(sums[(long long)b * kHeadSums + e]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float s = __shfl_xor_sync(0xffffffffu, sum.s, o), rest = __shfl_xor_sync(0xffffffffu, sum.rest, o);
+    sum.add(s);
+    sum.rest = fadd(sum.rest, rest);
+  }
+  const long long at = e < 387   ? flat_offset(11) + e
+                       : e < 644 ? flat_offset(8) + (e - 387)
+                                 : flat_offset(10) + (long long)flat_in(10) * flat_out(10) + (e - 644);
+  if (lane == 0) grads[at] += sum.total();
+}
 
 // The dX products of the BF16 backward (mlp_bwd_tc.cu): dz [10][n][256] BF16,
 // dz[9] in, dz[8] .. dz[0] out. bias [kChainMaxPairs * 2][kChainBias]: each
@@ -75,15 +99,18 @@ int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts
 
 // Weight and bias gradients of dense_0 .. dense_9 in the FP32 backward
 // (gemm_fp32_tc.cu): every layer's In^T dZ and column sums of dZ over n rows
-// added to the flat gradient blob, In from the FP32 tape, dz [10][n][256].
-int launch_fp32_dw(const float *acts, const float *dz, long long n, float *grads, cudaStream_t stream);
+// added to the flat gradient blob, In from the FP32 tape, dz [10][n][256]. With
+// them the heads' sums of `head_blocks` blocks.
+int launch_fp32_dw(const float *acts, const float *dz, const float *heads, int head_blocks, long long n, float *grads,
+                   cudaStream_t stream);
 
 // Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
 // layer's In^T dZ over n rows added to the flat gradient blob, In from the
 // BF16 tape, dz [10][n][256] BF16; part: gemm_dw_partial_floats() floats. With
-// them the chain's bias sums (of `ctas` CTAs).
+// them the chain's bias sums (of `ctas` CTAs) and the heads' (of `head_blocks`
+// blocks).
 int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
-                   const float *bias, int ctas, int *err, cudaStream_t stream);
+                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t stream);
 long long gemm_dw_partial_floats();
 // The BF16 (pair) or FP8 tensor-core forward with a chosen limit on every
 // bounded wait (ns) and the weight chunk at position `withhold` of the load

@@ -6,7 +6,8 @@
 // rows to `acts` (kActsLd floats per row). The backward takes the rows in
 // chunks of kChunkRows; per chunk
 //   head kernel   rgb = sigmoid(h9 Wr + br), sigma = ReLU(h7 ws + bs):
-//                 dZ9 = (dpre_rgb Wr^T) * [h9 > 0], dpre_sigma, head grads
+//                 dZ9 = (dpre_rgb Wr^T) * [h9 > 0], dpre_sigma, sums per block
+//                 for the head gradients
 //   chain kernel  for every layer from dense_9 down:
 //                 dZ_prev[m][k] = (sum_n dZ[m][n] W[k][n] + dpre_sigma[m] ws[k])
 //                                 * [h_prev[m][k] > 0]
@@ -87,8 +88,8 @@ struct HeadRow<uint16_t> {
 // eight: 40 shuffles and six sigmoids per lane and two rows, 0.50 ms of a
 // 4,096-ray BF16 step, 0.23 here). dZ9 is written 16 bytes per lane, and the head
 // weights' gradients accumulate in the lanes' registers over all of the warp's
-// rows; they reach the blob once per block (shared atomics, then one global
-// atomic per parameter).
+// rows; a block's sums (shared atomics) go to the workspace, where the weight
+// gradients' kernels add them up (add_head_sums).
 constexpr int kHeadWarps = 8;
 constexpr int kHeadRows = 2;
 
@@ -98,9 +99,9 @@ template <typename T, typename TZ>
 __global__ void __launch_bounds__(32 * kHeadWarps, 2)
     head_bwd_kernel(const float *__restrict__ table, const T *__restrict__ acts, long long n,
                     const float *__restrict__ d_rgb, const float *__restrict__ d_sigma, TZ *__restrict__ dz9,
-                    float *__restrict__ dsp_out, float *__restrict__ grads) {
+                    float *__restrict__ dsp_out, float *__restrict__ sums) {
   constexpr bool kBf16 = !std::is_same<TZ, float>::value;
-  constexpr int kAcc = kBf16 ? 772 : 644;
+  constexpr int kAcc = kBf16 ? kHeadSums : kHeadSumsFp32;
   __shared__ float sAcc[kAcc];  // dWr [128][3], dbr [3], dws [256], dbs [1] (BF16: db9 [128])
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int e = threadIdx.x; e < kAcc; e += blockDim.x) sAcc[e] = 0.0f;
@@ -215,49 +216,42 @@ __global__ void __launch_bounds__(32 * kHeadWarps, 2)
   }
   if ((lane & 3) == 0) atomicAdd(&sAcc[comp < 3 ? 384 + comp : 643], gbias);
   __syncthreads();
-  float *gWr = grads + flat_offset(11), *gbr_out = gWr + 128 * 3;
-  float *gws_out = grads + flat_offset(8), *gbs_out = gws_out + 256;
-  float *gb9_out = grads + flat_offset(10) + (long long)flat_in(10) * flat_out(10);
-  for (int e = threadIdx.x; e < kAcc; e += blockDim.x) {
-    float *dst = e < 384   ? gWr + e
-                 : e < 387 ? gbr_out + (e - 384)
-                 : e < 643 ? gws_out + (e - 387)
-                 : e < 644 ? gbs_out
-                           : gb9_out + (e - 644);
-    atomicAdd(dst, sAcc[e]);
-  }
+  for (int e = threadIdx.x; e < kAcc; e += blockDim.x) sums[(long long)blockIdx.x * kHeadSums + e] = sAcc[e];
 }
 
 }  // namespace train
 
 template <typename T, typename TZ>
 static int launch_head_bwd_t(const float *table, const T *tape, long long n, const float *d_rgb,
-                             const float *d_sigma, TZ *dz9, float *dsp, float *grads, cudaStream_t st) {
+                             const float *d_sigma, TZ *dz9, float *dsp, float *sums, int *used, cudaStream_t st) {
   using namespace train;
+  *used = 0;
   if (n == 0) return NERFGB_OK;
   const long long rows_per_block = (long long)kHeadWarps * kHeadRows;
   const long long blocks = (n + rows_per_block - 1) / rows_per_block;
   const int sms = num_sms();
-  const long long cap = (long long)(sms > 0 ? sms : 148) * 2;  // two blocks per SM (launch bounds)
-  head_bwd_kernel<T, TZ><<<(unsigned)(blocks < cap ? blocks : cap), 32 * kHeadWarps, 0, st>>>(table, tape, n, d_rgb,
-                                                                                        d_sigma, dz9, dsp, grads);
+  long long cap = (long long)(sms > 0 ? sms : 148) * 2;  // two blocks per SM (launch bounds)
+  if (cap > kHeadMaxBlocks) cap = kHeadMaxBlocks;
+  *used = (int)(blocks < cap ? blocks : cap);
+  head_bwd_kernel<T, TZ><<<(unsigned)*used, 32 * kHeadWarps, 0, st>>>(table, tape, n, d_rgb, d_sigma, dz9, dsp, sums);
   return launch_status();
 }
 
 int launch_head_bwd(const float *table, const float *tape, long long n, const float *d_rgb, const float *d_sigma,
-                    float *dz9, float *dsp, float *grads, cudaStream_t st) {
-  return launch_head_bwd_t(table, tape, n, d_rgb, d_sigma, dz9, dsp, grads, st);
+                    float *dz9, float *dsp, float *sums, int *blocks, cudaStream_t st) {
+  return launch_head_bwd_t(table, tape, n, d_rgb, d_sigma, dz9, dsp, sums, blocks, st);
 }
 
 int launch_head_bwd(const float *table, const uint16_t *tape, long long n, const float *d_rgb,
-                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *grads, cudaStream_t st) {
-  return launch_head_bwd_t(table, tape, n, d_rgb, d_sigma, dz9, dsp, grads, st);
+                    const float *d_sigma, __nv_bfloat16 *dz9, float *dsp, float *sums, int *blocks,
+                    cudaStream_t st) {
+  return launch_head_bwd_t(table, tape, n, d_rgb, d_sigma, dz9, dsp, sums, blocks, st);
 }
 
 namespace train {
 
 struct Ws {
-  float *wpack, *dsp, *dz;
+  float *wpack, *heads, *dsp, *dz;
   long long rows, bytes;
 };
 static Ws carve(void *base, long long n) {
@@ -265,10 +259,12 @@ static Ws carve(void *base, long long n) {
   float *p = reinterpret_cast<float *>(base);
   w.rows = n < kChunkRows ? n : kChunkRows;
   const long long pack = fp32_chain_pack_bytes() / (long long)sizeof(float);
+  constexpr long long heads = (long long)kHeadMaxBlocks * kHeadSums;
   w.wpack = p;
-  w.dz = p + pack;
+  w.heads = p + pack;
+  w.dz = w.heads + heads;
   w.dsp = w.dz + kNumGemm * w.rows * kDzLd;
-  w.bytes = (pack + w.rows * (kNumGemm * kDzLd + 1)) * (long long)sizeof(float);
+  w.bytes = (pack + heads + w.rows * (kNumGemm * kDzLd + 1)) * (long long)sizeof(float);
   return w;
 }
 
@@ -310,12 +306,13 @@ extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long l
   for (long long r0 = 0; r0 < n_rows; r0 += kChunkRows) {
     const long long n = n_rows - r0 < kChunkRows ? n_rows - r0 : kChunkRows;
     const float *a = acts + r0 * kActsLd;
+    int head_blocks = 0;
     if ((rc = launch_head_bwd(table, a, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * kDzLd,
-                              w.dsp, grad_params, st)) != NERFGB_OK)
+                              w.dsp, w.heads, &head_blocks, st)) != NERFGB_OK)
       return rc;
     if ((rc = launch_fp32_chain(w.wpack, table + kSigmaWOff, a, w.dsp, n, w.dz, grad_params, st)) != NERFGB_OK)
       return rc;
-    if ((rc = launch_fp32_dw(a, w.dz, n, grad_params, st)) != NERFGB_OK) return rc;
+    if ((rc = launch_fp32_dw(a, w.dz, w.heads, head_blocks, n, grad_params, st)) != NERFGB_OK) return rc;
   }
   return NERFGB_OK;
 }

@@ -4,10 +4,11 @@
 // The forward is the tensor-core BF16 kernel with its tape (mlp_tc.cu,
 // STORE): each layer's BF16 activations are exactly the operands its
 // successor's MMAs read. The backward, in chunks of kChunkRows rows:
-//   heads   dZ_9 (BF16), dpre_sigma, the heads' and dense_9's bias gradients (mlp_train.cu)
+//   heads   dZ_9 (BF16), dpre_sigma, sums per block for the gradients of the
+//           heads and of dense_9's bias (mlp_train.cu)
 //   chain   dZ_8 .. dZ_0 and their column sums per CTA, one kernel (mlp_bwd_tc.cu)
-//   dW      every layer's In^T dZ, one kernel and a reduction, which adds up the
-//           column sums too (gemm_tc.cu)
+//   dW      every layer's In^T dZ, one kernel and a reduction, which adds up
+//           those sums too (gemm_tc.cu)
 // every product on the tensor cores from BF16 operands (W the BF16 rounding
 // of the FP32 master weights), accumulating in FP32.
 #include <cuda_bf16.h>
@@ -26,7 +27,7 @@ struct Ws {
   float *dsp, *part;    // dpre_sigma, the dW kernel's partial sums
   __nv_bfloat16 *dz;    // [10][rows][256]
   void *wpack;          // the chain's BF16 weights
-  float *bias;          // the chain's bias sums
+  float *bias, *heads;  // the chain's bias sums, the heads' sums
   long long bytes;
 };
 
@@ -46,6 +47,7 @@ static Ws carve(void *base, long long n) {
   w.wpack = take(mlp_chain_pack_bytes());
   w.part = reinterpret_cast<float *>(take(gemm_dw_partial_floats() * 4));
   w.bias = reinterpret_cast<float *>(take(2LL * kChainMaxPairs * kChainBias * 4));
+  w.heads = reinterpret_cast<float *>(take((long long)kHeadMaxBlocks * kHeadSums * 4));
   w.bytes = off;
   return w;
 }
@@ -91,14 +93,16 @@ extern "C" int nerfgb_mlp_backward_bf16(const void *packed_fp32, const void *tap
   for (long long r0 = 0; r0 < n_rows; r0 += kChunkRows) {
     const long long n = n_rows - r0 < kChunkRows ? n_rows - r0 : kChunkRows;
     const uint16_t *t = tp + r0 * kActsLd;
+    int head_blocks = 0, ctas = 0;
     if ((rc = launch_head_bwd(table, t, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * 256, w.dsp,
-                              grad_params, st)) != NERFGB_OK)
+                              w.heads, &head_blocks, st)) != NERFGB_OK)
       return rc;
-    int ctas = 0;
     if ((rc = launch_mlp_chain(w.wpack, table + kSigmaWOff, t, w.dsp, n, w.dz, w.bias, &ctas, err_word, st)) !=
         NERFGB_OK)
       return rc;
-    if ((rc = launch_gemm_dw(t, w.dz, n, grad_params, w.part, w.bias, ctas, err_word, st)) != NERFGB_OK) return rc;
+    if ((rc = launch_gemm_dw(t, w.dz, n, grad_params, w.part, w.bias, ctas, w.heads, head_blocks, err_word, st)) !=
+        NERFGB_OK)
+      return rc;
   }
   return NERFGB_OK;
 }
