@@ -401,10 +401,32 @@ long long nerfgb_mlp_backward_workspace_bytes(long long n_rows);
  * into grad_params. acts from nerfgb_mlp_forward_train on the same rows with
  * the same FP32 pack. d_sigma may be NULL. FP32 accuracy throughout: the
  * products run on the tensor cores from exact three-part BF16 splits, summed
- * in FP32. A timeout of their bounded waits leaves NaN in grad_params. */
+ * in FP32. Where an activation, a weight or a gradient on the way is not
+ * finite, or above 3.39e38 (BF16's largest), the sums that it enters are NaN.
+ * A timeout of the kernels' bounded waits makes all of grad_params NaN. */
 int nerfgb_mlp_backward(const void *packed, const float *acts, long long n_rows,
                         const float *d_rgb, const float *d_sigma,
                         float *grad_params, void *workspace, void *stream);
+
+/* nerfgb_mlp_backward that reports a timeout in err_word too (caller-zeroed
+ * device int32: NERFGB_E_TIMEOUT). */
+int nerfgb_mlp_backward_checked(const void *packed, const float *acts,
+                                long long n_rows, const float *d_rgb,
+                                const float *d_sigma, float *grad_params,
+                                void *workspace, int *err_word, void *stream);
+
+/* Diagnostic of the failure path, as nerfgb_mlp_forward_wait_test: the
+ * backward of `precision` (FP32 or BF16, with its tape) with every bounded
+ * wait limited to wait_ns (1 us to 10 s) and withhold = 0: nothing, 1: a
+ * weight copy of the dX kernel, 2: a stage's operands of the weight-gradient
+ * kernel left out, so that a wait runs out. Too few rows (fewer than two
+ * 64-row stages per kernel) leave nothing to withhold. */
+int nerfgb_mlp_backward_wait_test(const void *packed_fp32, int precision,
+                                  const void *tape, long long n_rows,
+                                  const float *d_rgb, const float *d_sigma,
+                                  float *grad_params, void *workspace,
+                                  int *err_word, unsigned long long wait_ns,
+                                  int withhold, void *stream);
 
 /* ---- BF16 training (tensor cores, FP32 master weights) ------------------ */
 

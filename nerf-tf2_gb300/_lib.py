@@ -78,6 +78,8 @@ SIGNATURES = {
     "nerfgb_mlp_forward_train": (I, [P, P, P, LL, I, P, P, P, P]),
     "nerfgb_mlp_backward_workspace_bytes": (LL, [LL]),
     "nerfgb_mlp_backward": (I, [P, P, LL, P, P, P, P, P]),
+    "nerfgb_mlp_backward_checked": (I, [P, P, LL, P, P, P, P, P, P]),
+    "nerfgb_mlp_backward_wait_test": (I, [P, I, P, LL, P, P, P, P, P, ULL, I, P]),
     "nerfgb_mlp_forward_train_bf16": (I, [P, P, P, LL, I, P, P, P, P, P]),
     "nerfgb_mlp_backward_bf16_workspace_bytes": (LL, [LL]),
     "nerfgb_mlp_backward_bf16": (I, [P, P, LL, P, P, P, P, P, P]),

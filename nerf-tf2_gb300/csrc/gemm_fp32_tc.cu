@@ -52,8 +52,9 @@
 // 88 for the conversion.
 //
 // Every mbarrier wait is bounded (tc::wait_bar): on a timeout every role
-// stops, the issuer drains its MMAs, TMEM is freed and the CTA writes NaN into
-// every layer's gradient.
+// stops, the issuer drains its MMAs, TMEM is freed and the CTA makes the whole
+// gradient NaN (what others add to it stays NaN) and reports to the caller's
+// error word, if there is one.
 #include <stdint.h>
 
 #include <mutex>
@@ -150,7 +151,7 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 
 // Barriers, TMEM (all 512 columns of both CTAs; its address) and the pair's start.
 __device__ __forceinline__ uint32_t begin(uint8_t *smem, uint32_t sbase, volatile int *abort_flag, int *err,
-                                          bool aligned) {
+                                          bool aligned, unsigned long long wait_ns) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(sbase + kBarFull + 8 * s, 2 * kConvWarps);
@@ -163,7 +164,7 @@ __device__ __forceinline__ uint32_t begin(uint8_t *smem, uint32_t sbase, volatil
     mbar_init(sbase + kBarDrain, 1);
     *abort_flag = aligned ? 0 : 1;
     *err = 0;
-    set_wait_limit(abort_flag, kWaitNs);
+    set_wait_limit(abort_flag, wait_ns != 0 ? wait_ns : kWaitNs);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < 32) {
@@ -240,10 +241,14 @@ __device__ __forceinline__ void drain(uint32_t sbase) {
 }
 
 // The pair's end. After a timeout the gradient is not a number. `ran`: the issuer drains.
-__device__ __forceinline__ void finish(uint32_t sbase, uint32_t tmem, volatile int *abort_flag, float *grads, bool ran) {
+__device__ __forceinline__ void finish(uint32_t sbase, uint32_t tmem, volatile int *abort_flag, const int *err,
+                                       float *grads, int *err_word, bool ran) {
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x < 11) grads[flat_offset(threadIdx.x)] = __int_as_float(0x7fffffff);
+  if (*abort_flag) {
+    for (long long e = threadIdx.x; e < kParamCount; e += kThreads) grads[e] = __int_as_float(0x7fffffff);
+    if (threadIdx.x == 0 && err_word) atomicExch(err_word, *err != 0 ? *err : NERFGB_E_UNSUPPORTED);
+  }
   if (cluster_rank() == 1 && threadIdx.x == 0 && ran) {
     // the even CTA's MMAs read this CTA's stages: its last commit
     uint64_t t0 = globaltimer();
@@ -292,7 +297,7 @@ __device__ __forceinline__ void split_store(const float4 &u, const float4 &v, ui
 
 __global__ void __launch_bounds__(kThreads, 1)
     dw_kernel(const float *__restrict__ acts, const float *__restrict__ dz, const float *__restrict__ heads,
-              int head_blocks, long long n, float *__restrict__ grads) {
+              int head_blocks, long long n, float *grads, int *err_word, WaitTest wt) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -318,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     reinterpret_cast<Share *>(smem + kShare)[threadIdx.x] = sh;
   }
 
-  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned);
+  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned, wt.wait_ns);
 
   if (warp >= kSumWarps) {
     // ---------------- conversion ----------------
@@ -423,7 +428,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(peer_addr(sbase + kBarFull + 8 * k, 0));
+        if (lane == 0 && !(wt.withhold != 0 && q == 1 && w == 0))
+          mbar_arrive_remote(peer_addr(sbase + kBarFull + 8 * k, 0));
       }
       if (job.bias) {
         // the lanes of a chunk, then the warps (and pairs) by atomics
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (issuer && stages > 0) drain(sbase);
   }
 
-  finish(sbase, tmem, abort_flag, grads, stages > 0);
+  finish(sbase, tmem, abort_flag, err, grads, err_word, stages > 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -543,7 +549,8 @@ __global__ void pack_kernel(const float *__restrict__ W, uint8_t *__restrict__ o
 // rows; in their waits for the stages 550; 490 - 526 here).
 __global__ void __launch_bounds__(kThreads, 1)
     chain_kernel(const float *__restrict__ sigma_w, const float *__restrict__ acts, const float *__restrict__ dsp,
-                 long long n, float *dz, float *__restrict__ grads, const __grid_constant__ CUtensorMap weights) {
+                 long long n, float *dz, float *__restrict__ grads, int *err_word, WaitTest wt,
+                 const __grid_constant__ CUtensorMap weights) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -556,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tiles = aligned ? (int)((n + 255) / 256) : 0;
   // the tiles dealt evenly and contiguously
   const int first = (int)((long long)pair * tiles / pairs), count = (int)((long long)(pair + 1) * tiles / pairs) - first;
-  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned);
+  const uint32_t tmem = begin(smem, sbase, abort_flag, err, aligned, wt.wait_ns);
 
   if (warp >= kSumWarps) {
     // ---------------- conversion, weight copies ----------------
@@ -627,7 +634,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               ok = false;
               break;
             }
-            if (w == 0 && lane == 0) {
+            if (w == 0 && lane == 0 && !(wt.withhold != 0 && q == 1)) {
               const uint32_t bar = sbase + kBarB + 8 * k, to = sbase + k * kStage + kOperand;
               if (crank == 0) mbar_expect_tx(bar, 2 * kOperand);
               const int y = ((first_chunk(g) + ch) * 2 + (int)crank) * (int)(kOperand / 256);
@@ -758,7 +765,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (issuer && tiles > 0) drain(sbase);
   }
 
-  finish(sbase, tmem, abort_flag, grads, tiles > 0);
+  finish(sbase, tmem, abort_flag, err, grads, err_word, tiles > 0);
 }
 
 }  // namespace split
@@ -771,7 +778,7 @@ struct Pairs {
   std::unordered_map<int, int> of_device;
 };
 template <typename... P, typename... A>
-static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cudaStream_t st, A... args) {
+static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cudaStream_t st, const A &...args) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
     return NERFGB_E_CUDA;
   const int sms = num_sms();
@@ -809,11 +816,12 @@ static int launch_pairs(void (*kernel)(P...), Pairs &pairs, long long work, cuda
 }  // namespace split
 
 int launch_fp32_dw(const float *acts, const float *dz, const float *heads, int head_blocks, long long n, float *grads,
-                   cudaStream_t st) {
+                   int *err_word, cudaStream_t st, const WaitTest &wt) {
   using namespace split;
   if (n == 0) return NERFGB_OK;
   static Pairs pairs;
-  return launch_pairs(dw_kernel, pairs, kJobs * ((n + kRows - 1) / kRows), st, acts, dz, heads, head_blocks, n, grads);
+  return launch_pairs(dw_kernel, pairs, kJobs * ((n + kRows - 1) / kRows), st, acts, dz, heads, head_blocks, n, grads,
+                      err_word, wt);
 }
 
 long long fp32_chain_pack_bytes() { return split::kPackBytes; }
@@ -824,7 +832,7 @@ int launch_fp32_chain_pack(const float *packed, void *wpack, cudaStream_t st) {
 }
 
 int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts, const float *dsp, long long n,
-                      float *dz, float *grads, cudaStream_t st) {
+                      float *dz, float *grads, int *err_word, cudaStream_t st, const WaitTest &wt) {
   using namespace split;
   if (n == 0) return NERFGB_OK;
   static Pairs pairs;
@@ -833,7 +841,8 @@ int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts
   const unsigned box[2] = {128, kPart / 256};
   const int rc = encode_tensor_map_u16(&weights, wpack, 2, dims, strides, box);
   if (rc != NERFGB_OK) return rc;
-  return launch_pairs(chain_kernel, pairs, (n + 255) / 256, st, sigma_w, acts, dsp, n, dz, grads, weights);
+  return launch_pairs(chain_kernel, pairs, (n + 255) / 256, st, sigma_w, acts, dsp, n, dz, grads, err_word, wt,
+                      weights);
 }
 
 }  // namespace nerfgb

@@ -120,7 +120,7 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    dw_kernel(float *__restrict__ part, int *__restrict__ err, long long n, int window,
+    dw_kernel(float *__restrict__ part, int *__restrict__ err, long long n, int window, WaitTest wt,
               const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     mbar_init(sbase + kBarDrain, 1);
     *abort_flag = 0;
-    set_wait_limit(abort_flag, kWaitNs);
+    set_wait_limit(abort_flag, wt.wait_ns != 0 ? wt.wait_ns : kWaitNs);
     if ((sbase & 1023u) != 0) atomicExch(err, NERFGB_E_UNSUPPORTED);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       uint32_t used = 0;  // bit st: parity of the copies issued into stage st
       int st = 0;
-      bool ok = true;
+      bool ok = true, withheld = wt.withhold == 0;
       for (int j = 0; j < kJobs && ok; ++j) {
         const Job job = job_of(j);
         long long sb, se;
@@ -179,9 +179,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           const uint32_t full = sbase + kBarFull + 8 * st, to = sbase + st * kStage;
           const uint32_t bar = crank == 0 ? full : peer_addr(full, 0);
-          if (crank == 0) mbar_expect_tx(full, (uint32_t)job.atoms() * kAtomBytes);
-          if (na) tma_load_3d_pair(to, ma, (int)(i * kRows), a0, bar);
-          if (nb) tma_load_3d_pair(to + kOperand, mb, (int)(i * kRows), b0, bar);
+          if (st == 1 && crank == 0 && !withheld) {
+            withheld = true;  // (test hook: this stage's copies are left out)
+          } else {
+            if (crank == 0) mbar_expect_tx(full, (uint32_t)job.atoms() * kAtomBytes);
+            if (na) tma_load_3d_pair(to, ma, (int)(i * kRows), a0, bar);
+            if (nb) tma_load_3d_pair(to + kOperand, mb, (int)(i * kRows), b0, bar);
+          }
           used ^= 1u << st;
           if (++st == kNst) st = 0;
         }
@@ -377,7 +381,8 @@ __global__ void __launch_bounds__(kRedElems)
 long long gemm_dw_partial_floats() { return (gemm::kMaxPairs + gemm::kJobs) * 65536LL; }
 
 int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
-                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t st) {
+                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t st,
+                   const WaitTest &wt) {
   using namespace gemm;
   if (n == 0) return NERFGB_OK;
   if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
@@ -440,7 +445,7 @@ int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, f
   // 2.81 ms of backward).
   const long long each = kJobs * stages / pairs;
   const int window = each <= 32 ? 1 : each <= 512 ? 2 : 4;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, window, maps);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_kernel, part, err, n, window, wt, maps);
   if ((rc = launch_status()) != NERFGB_OK) return rc;  // (clears a failed launch's error)
   if (e != cudaSuccess) return NERFGB_E_CUDA;
   static_assert(kChainBias % kRedElems == 0 && kHeadSums % (kRedElems / 32) == 0, "whole blocks of bias and head sums");

@@ -177,7 +177,7 @@ __device__ __forceinline__ void add_columns(const float (&sum)[16], int lane, fl
 
 __global__ void __launch_bounds__(kThreads, 1)
     chain_kernel(const float *__restrict__ ws, const float *__restrict__ dsp, long long n, float *__restrict__ bias,
-                 int *__restrict__ err, const __grid_constant__ Maps maps) {
+                 int *__restrict__ err, WaitTest wt, const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     mbar_init(sbase + kBarDrain, 1);
     *abort_flag = 0;
-    set_wait_limit(abort_flag, kWaitNs);
+    set_wait_limit(abort_flag, wt.wait_ns != 0 ? wt.wait_ns : kWaitNs);
     if ((sbase & 1023u) != 0) atomicExch(err, NERFGB_E_UNSUPPORTED);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -240,9 +240,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           const uint32_t full = sbase + kBarFull + 8 * st;
-          if (crank == 0) mbar_expect_tx(full, 2 * kPairStage);
-          tma_2d_pair(sbase + st * kPairStage, &maps.w, 0, (int)((src + crank * kPairStage) >> 8),
-                      crank == 0 ? full : peer_addr(full, 0));
+          // (test hook: the even CTA leaves out the tile's second chunk)
+          if (!(wt.withhold != 0 && crank == 0 && src == 2 * kPairStage)) {
+            if (crank == 0) mbar_expect_tx(full, 2 * kPairStage);
+            tma_2d_pair(sbase + st * kPairStage, &maps.w, 0, (int)((src + crank * kPairStage) >> 8),
+                        crank == 0 ? full : peer_addr(full, 0));
+          }
           used ^= 1u << st;
           if (++st == kNst) st = 0;
         }
@@ -460,7 +463,7 @@ int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t st
 }
 
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
-                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream) {
+                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream, const WaitTest &wt) {
   using namespace tcb;
   *ctas = 0;
   if (n == 0) return NERFGB_OK;
@@ -518,7 +521,7 @@ int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *ta
     if ((rc = encode_tensor_map_u16(&maps.dz[l], dz + (long long)l * n * 256, 3, dims, strides, box, true)) != NERFGB_OK)
       return rc;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, bias, err, maps);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, chain_kernel, sigma_w, dsp, n, bias, err, wt, maps);
   rc = launch_status();  // (clears a failed launch's error)
   return e == cudaSuccess ? rc : NERFGB_E_CUDA;
 }

@@ -45,6 +45,14 @@ int launch_mlp_bf16(const void *packed, const float *xyz, const float *dirs, lon
 int launch_mlp_bf16_train(const void *packed, const float *xyz, const float *dirs, long long n, int rows_per_dir,
                           float *rgb, float *sigma, uint16_t *tape, int *err_word, cudaStream_t stream);
 
+// The failure path's test hook of a tensor-core kernel of the backward: a limit
+// on its bounded waits (ns; 0: its own) and, withheld, one of the copies or
+// arrivals that they wait for.
+struct WaitTest {
+  unsigned long long wait_ns = 0;
+  int withhold = 0;
+};
+
 // Backward of the sigma and rgb heads (mlp_train.cu) from an FP32 or a BF16
 // activation tape: dz9 = dL/d(dense_9 pre-activation), row stride 256 (128
 // used), FP32 or BF16; dsp [n] = dL/d(sigma pre-activation). sums
@@ -74,7 +82,8 @@ __device__ __forceinline__ void add_head_sums(const float *__restrict__ sums, in
   const long long at = e < 387   ? flat_offset(11) + e
                        : e < 644 ? flat_offset(8) + (e - 387)
                                  : flat_offset(10) + (long long)flat_in(10) * flat_out(10) + (e - 644);
-  if (lane == 0) grads[at] += sum.total();
+  // (atomic: what marks the gradient after a timeout may be on its way)
+  if (lane == 0) atomicAdd(grads + at, sum.total());
 }
 
 // The dX products of the BF16 backward (mlp_bwd_tc.cu): dz [10][n][256] BF16,
@@ -86,23 +95,26 @@ constexpr int kChainMaxPairs = 76, kChainBias = 9 * 256;
 long long mlp_chain_pack_bytes();
 int launch_mlp_chain_pack(const float *packed_fp32, void *wpack, cudaStream_t stream);
 int launch_mlp_chain(const void *wpack, const float *sigma_w, const uint16_t *tape, const float *dsp, long long n,
-                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream);
+                     __nv_bfloat16 *dz, float *bias, int *ctas, int *err, cudaStream_t stream,
+                     const WaitTest &wt = WaitTest());
 
 // The dX products of the FP32 backward (gemm_fp32_tc.cu): dz [10][n][256],
 // dz[9] in (128 columns), dz[8] .. dz[0] out. wpack (fp32_chain_pack_bytes,
 // 16-byte aligned) from the FP32 pack's weights by launch_fp32_chain_pack;
-// sigma_w: the sigma head's weights; grads: not a number after a timeout.
+// sigma_w: the sigma head's weights. After a timeout all of grads is not a
+// number and, unless NULL, *err_word the status; launch_fp32_dw likewise.
 long long fp32_chain_pack_bytes();
 int launch_fp32_chain_pack(const float *packed, void *wpack, cudaStream_t stream);
 int launch_fp32_chain(const void *wpack, const float *sigma_w, const float *acts, const float *dsp, long long n,
-                      float *dz, float *grads, cudaStream_t stream);
+                      float *dz, float *grads, int *err_word, cudaStream_t stream,
+                      const WaitTest &wt = WaitTest());
 
 // Weight and bias gradients of dense_0 .. dense_9 in the FP32 backward
 // (gemm_fp32_tc.cu): every layer's In^T dZ and column sums of dZ over n rows
 // added to the flat gradient blob, In from the FP32 tape, dz [10][n][256]. With
 // them the heads' sums of `head_blocks` blocks.
 int launch_fp32_dw(const float *acts, const float *dz, const float *heads, int head_blocks, long long n, float *grads,
-                   cudaStream_t stream);
+                   int *err_word, cudaStream_t stream, const WaitTest &wt = WaitTest());
 
 // Tensor-core weight gradients of the BF16 backward (gemm_tc.cu): every
 // layer's In^T dZ over n rows added to the flat gradient blob, In from the
@@ -110,7 +122,8 @@ int launch_fp32_dw(const float *acts, const float *dz, const float *heads, int h
 // them the chain's bias sums (of `ctas` CTAs) and the heads' (of `head_blocks`
 // blocks).
 int launch_gemm_dw(const uint16_t *tape, const __nv_bfloat16 *dz, long long n, float *grads, float *part,
-                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t stream);
+                   const float *bias, int ctas, const float *heads, int head_blocks, int *err, cudaStream_t stream,
+                   const WaitTest &wt = WaitTest());
 long long gemm_dw_partial_floats();
 // The BF16 (pair) or FP8 tensor-core forward with a chosen limit on every
 // bounded wait (ns) and the weight chunk at position `withhold` of the load
@@ -123,6 +136,12 @@ int launch_mlp_wait_test(const void *packed, bool fp8, const float *xyz, const f
 // FP8-e4m3 tcgen05 forward (mlp_tc.cu).
 int launch_mlp_fp8(const void *packed, const float *xyz, const float *dirs, long long n, int rows_per_dir,
                    float *rgb, float *sigma, int *err_word, cudaStream_t stream, const RowMap &rm = RowMap());
+
+// The BF16 backward (mlp_train_bf16.cu), nerfgb_mlp_backward_bf16 with the test
+// hooks of its two tensor-core kernels.
+int mlp_backward_bf16(const void *packed_fp32, const void *tape, long long n_rows, const float *d_rgb,
+                      const float *d_sigma, float *grad_params, void *workspace, int *err_word, void *stream,
+                      const WaitTest &chain, const WaitTest &dw);
 
 // Dispatch on precision (render.cu).
 int launch_mlp(const void *packed, int precision, const float *xyz, const float *dirs, long long n, int rpd,

@@ -289,8 +289,9 @@ extern "C" int nerfgb_mlp_forward_train(const void *packed, const float *xyz, co
   return launch_mlp_fp32_store(packed, xyz, dirs, n_rows, rows_per_dir, rgb, sigma, acts, as_stream(stream));
 }
 
-extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long long n_rows, const float *d_rgb,
-                                   const float *d_sigma, float *grad_params, void *workspace, void *stream) {
+static int mlp_backward_fp32(const void *packed, const float *acts, long long n_rows, const float *d_rgb,
+                             const float *d_sigma, float *grad_params, void *workspace, int *err_word, void *stream,
+                             const WaitTest &chain, const WaitTest &dw) {
   using namespace train;
   if (n_rows < 0) return NERFGB_E_INVALID_ARG;
   if (n_rows == 0) return NERFGB_OK;
@@ -310,9 +311,39 @@ extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long l
     if ((rc = launch_head_bwd(table, a, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * kDzLd,
                               w.dsp, w.heads, &head_blocks, st)) != NERFGB_OK)
       return rc;
-    if ((rc = launch_fp32_chain(w.wpack, table + kSigmaWOff, a, w.dsp, n, w.dz, grad_params, st)) != NERFGB_OK)
+    if ((rc = launch_fp32_chain(w.wpack, table + kSigmaWOff, a, w.dsp, n, w.dz, grad_params, err_word, st, chain)) !=
+        NERFGB_OK)
       return rc;
-    if ((rc = launch_fp32_dw(a, w.dz, w.heads, head_blocks, n, grad_params, st)) != NERFGB_OK) return rc;
+    if ((rc = launch_fp32_dw(a, w.dz, w.heads, head_blocks, n, grad_params, err_word, st, dw)) != NERFGB_OK) return rc;
   }
   return NERFGB_OK;
+}
+
+extern "C" int nerfgb_mlp_backward(const void *packed, const float *acts, long long n_rows, const float *d_rgb,
+                                   const float *d_sigma, float *grad_params, void *workspace, void *stream) {
+  return mlp_backward_fp32(packed, acts, n_rows, d_rgb, d_sigma, grad_params, workspace, nullptr, stream, WaitTest(),
+                           WaitTest());
+}
+
+extern "C" int nerfgb_mlp_backward_checked(const void *packed, const float *acts, long long n_rows, const float *d_rgb,
+                                           const float *d_sigma, float *grad_params, void *workspace, int *err_word,
+                                           void *stream) {
+  if (n_rows > 0 && !err_word) return NERFGB_E_INVALID_ARG;
+  return mlp_backward_fp32(packed, acts, n_rows, d_rgb, d_sigma, grad_params, workspace, err_word, stream, WaitTest(),
+                           WaitTest());
+}
+
+extern "C" int nerfgb_mlp_backward_wait_test(const void *packed_fp32, int precision, const void *tape, long long n_rows,
+                                             const float *d_rgb, const float *d_sigma, float *grad_params,
+                                             void *workspace, int *err_word, unsigned long long wait_ns, int withhold,
+                                             void *stream) {
+  if (precision != NERFGB_PREC_FP32 && precision != NERFGB_PREC_BF16) return NERFGB_E_UNSUPPORTED;
+  if (wait_ns < 1000ull || wait_ns > 10000000000ull || withhold < 0 || withhold > 2) return NERFGB_E_INVALID_ARG;
+  if (n_rows > 0 && !err_word) return NERFGB_E_INVALID_ARG;
+  const WaitTest chain{wait_ns, withhold == 1}, dw{wait_ns, withhold == 2};
+  if (precision == NERFGB_PREC_BF16)
+    return mlp_backward_bf16(packed_fp32, tape, n_rows, d_rgb, d_sigma, grad_params, workspace, err_word, stream, chain,
+                             dw);
+  return mlp_backward_fp32(packed_fp32, reinterpret_cast<const float *>(tape), n_rows, d_rgb, d_sigma, grad_params,
+                           workspace, err_word, stream, chain, dw);
 }

@@ -74,9 +74,10 @@ extern "C" int nerfgb_mlp_forward_train_bf16(const void *packed_bf16, const floa
                                reinterpret_cast<uint16_t *>(tape), err_word, as_stream(stream));
 }
 
-extern "C" int nerfgb_mlp_backward_bf16(const void *packed_fp32, const void *tape, long long n_rows,
-                                        const float *d_rgb, const float *d_sigma, float *grad_params,
-                                        void *workspace, int *err_word, void *stream) {
+namespace nerfgb {
+int mlp_backward_bf16(const void *packed_fp32, const void *tape, long long n_rows, const float *d_rgb,
+                      const float *d_sigma, float *grad_params, void *workspace, int *err_word, void *stream,
+                      const WaitTest &chain, const WaitTest &dw) {
   using namespace train16;
   if (n_rows < 0) return NERFGB_E_INVALID_ARG;
   if (n_rows == 0) return NERFGB_OK;
@@ -97,12 +98,20 @@ extern "C" int nerfgb_mlp_backward_bf16(const void *packed_fp32, const void *tap
     if ((rc = launch_head_bwd(table, t, n, d_rgb + 3 * r0, d_sigma ? d_sigma + r0 : nullptr, w.dz + 9 * n * 256, w.dsp,
                               w.heads, &head_blocks, st)) != NERFGB_OK)
       return rc;
-    if ((rc = launch_mlp_chain(w.wpack, table + kSigmaWOff, t, w.dsp, n, w.dz, w.bias, &ctas, err_word, st)) !=
+    if ((rc = launch_mlp_chain(w.wpack, table + kSigmaWOff, t, w.dsp, n, w.dz, w.bias, &ctas, err_word, st, chain)) !=
         NERFGB_OK)
       return rc;
-    if ((rc = launch_gemm_dw(t, w.dz, n, grad_params, w.part, w.bias, ctas, w.heads, head_blocks, err_word, st)) !=
+    if ((rc = launch_gemm_dw(t, w.dz, n, grad_params, w.part, w.bias, ctas, w.heads, head_blocks, err_word, st, dw)) !=
         NERFGB_OK)
       return rc;
   }
   return NERFGB_OK;
+}
+}  // namespace nerfgb
+
+extern "C" int nerfgb_mlp_backward_bf16(const void *packed_fp32, const void *tape, long long n_rows,
+                                        const float *d_rgb, const float *d_sigma, float *grad_params,
+                                        void *workspace, int *err_word, void *stream) {
+  return mlp_backward_bf16(packed_fp32, tape, n_rows, d_rgb, d_sigma, grad_params, workspace, err_word, stream,
+                           WaitTest(), WaitTest());
 }

@@ -134,7 +134,8 @@ class NerfMLP:
         into grad_params (flat Keras layout). An FP32 tape takes the FP32
         backward; a BF16 tape (from ``forward_train(precision="bf16")``) the
         BF16 one (BF16 tensor-core GEMMs, FP32 accumulation, FP32
-        gradients; a bounded-wait timeout lands in err_word)."""
+        gradients). A bounded-wait timeout of either lands in err_word
+        (``check_device_errors``)."""
         n = acts.shape[0]
         d_rgb = as_cuda(d_rgb, shape=(n, 3), name="d_rgb")
         d_sigma = as_cuda(d_sigma, shape=(n,), name="d_sigma")
@@ -146,8 +147,8 @@ class NerfMLP:
             _lib.call("nerfgb_mlp_backward_bf16", ptr(self.packed("fp32")), ptr(acts), n, ptr(d_rgb),
                       ptr(d_sigma), ptr(grad_params), ptr(ws), ptr(self.err_word), stream())
         else:
-            _lib.call("nerfgb_mlp_backward", ptr(self.packed("fp32")), ptr(acts), n, ptr(d_rgb), ptr(d_sigma),
-                      ptr(grad_params), ptr(ws), stream())
+            _lib.call("nerfgb_mlp_backward_checked", ptr(self.packed("fp32")), ptr(acts), n, ptr(d_rgb), ptr(d_sigma),
+                      ptr(grad_params), ptr(ws), ptr(self.err_word), stream())
         return grad_params
 
     def check_device_errors(self):
