@@ -209,7 +209,10 @@ inline int num_sms() {
 // kernel's first statement is after_previous(): until the kernel before is
 // complete and its writes are visible nothing of it is read or written. The
 // kernel after may be set up from there on (not before: it would then have been
-// started, its caches cleared, while the kernel before last was running). Not
+// started, its caches cleared, while the kernel before last was running). Such a
+// kernel exists while its inputs are still being written: they are not
+// const __restrict__ and not read by ld.global.nc, which are for memory that
+// nothing writes while the kernel exists and so may be read before the wait. Not
 // during stream capture, where the launch is an ordinary one. A 61-ray render
 // (five kernels) 84 -> 78 us, an MLP launch of 1,000 rows 29.2 -> 27.0; launches
 // that fill the chip take no part: their waiting CTAs would hold SMs that another

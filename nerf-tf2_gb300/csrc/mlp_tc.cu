@@ -334,12 +334,12 @@ __device__ __forceinline__ void store_frag64(uint32_t addr, uint32_t cx, uint32_
 // ---------------------------------------------------------------------------
 // Epilogue of the head layers: a row per lane, 32 columns at a time.
 // ---------------------------------------------------------------------------
-// A read-only load that stays where it is written: hoisted and batched by the
-// compiler, the head weights' loads would take the registers of everything
-// else (and spill).
+// A load that stays where it is written: hoisted and batched by the compiler,
+// the head weights' loads would take the registers of everything else (and
+// spill).
 __device__ __forceinline__ float4 ld_here(const float *p) {
   float4 v;
-  asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float4 lds_here(uint32_t addr) {
@@ -461,8 +461,8 @@ __device__ __forceinline__ void issue_solo(uint32_t sbase, uint32_t acc, RingPos
 // BF16 values per row at the columns of the FP32 tape (acts_offset).
 template <bool F8, bool STORE>
 __global__ void __launch_bounds__(threads_of(STORE), 1)
-    mlp_tc_kernel(const uint8_t *__restrict__ packed, const float *__restrict__ xyz,
-                    const float *__restrict__ dirs, long long n_max, int rpd, float *__restrict__ rgb_out,
+    mlp_tc_kernel(const uint8_t *packed, const float *xyz,
+                    const float *dirs, long long n_max, int rpd, float *__restrict__ rgb_out,
                     float *__restrict__ sigma_out, int *__restrict__ err, RowMap rm, uint16_t *__restrict__ tape,
                     unsigned long long wait_ns, long long withhold, const __grid_constant__ PairMaps maps) {
   static_assert(!(STORE && F8), "the activation tape is BF16");

@@ -17,9 +17,9 @@ namespace nerfgb {
 
 // u NULL with perturb: the uniform of (ray r, bin i) is element r*S + i of
 // the Philox stream keyed by seed (nerfgb_uniform's element), drawn here.
-__global__ void coarse_sample_kernel(const float *__restrict__ rays_o, const float *__restrict__ rays_d,
-                                     const float *__restrict__ near, const float *__restrict__ far,
-                                     const float *__restrict__ u, unsigned long long seed, int R, int S,
+__global__ void coarse_sample_kernel(const float *rays_o, const float *rays_d,
+                                     const float *near, const float *far,
+                                     const float *u, unsigned long long seed, int R, int S,
                                      int perturb, int lin_inv, float *__restrict__ xyz, float *__restrict__ dirs,
                                      float *__restrict__ t_out, float *__restrict__ edges,
                                      float *__restrict__ widths) {
@@ -77,8 +77,8 @@ constexpr int kCompWarps = 4;
 // from there. With gate_map != NULL the weights also gate the samples
 // (sample j on where w > tau, NaN off; gate_ray).
 __global__ void __launch_bounds__(32 * kCompWarps)
-    composite_kernel(const float *__restrict__ rgb, const float *__restrict__ sigma,
-                     const float *__restrict__ t, int R, int S, int white_bg, int mode, float last_delta,
+    composite_kernel(const float *rgb, const float *sigma,
+                     const float *t, int R, int S, int white_bg, int mode, float last_delta,
                      float *__restrict__ weights, float *__restrict__ pred_rgb,
                      float *__restrict__ pred_depth, float *__restrict__ acc_map, float tau,
                      unsigned char *__restrict__ gate_mask, int *__restrict__ gate_map, int *__restrict__ gate_count,
@@ -212,10 +212,10 @@ __host__ __device__ __forceinline__ int fine_smem_floats(int Sc, int Sf, int P) 
 }
 
 __global__ void __launch_bounds__(32 * kFineWarps, 8)
-    fine_sample_kernel(const float *__restrict__ rays_o, const float *__restrict__ rays_d,
-                       const float *__restrict__ bin_weights, const float *__restrict__ left_edges,
-                       int ld_left, const float *__restrict__ bin_widths,
-                       const float *__restrict__ t_coarse, const float *__restrict__ u, int R, int Sc,
+    fine_sample_kernel(const float *rays_o, const float *rays_d,
+                       const float *bin_weights, const float *left_edges,
+                       int ld_left, const float *bin_widths,
+                       const float *t_coarse, const float *u, int R, int Sc,
                        int Sf, float *__restrict__ xyz, float *__restrict__ dirs,
                        float *__restrict__ t_out, int *__restrict__ piece_idxs,
                        int *__restrict__ sort_perm, int P, FineFuse fz) {
