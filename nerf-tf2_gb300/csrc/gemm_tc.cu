@@ -11,8 +11,8 @@
 // row k at k*128 bytes (desc_mn_sw128, the instruction descriptor's transpose
 // bits set), rows past the bounds zero-filled.
 //
-// Bound by HBM (every byte of tape and dZ once, dZ_0, dZ_5 and dZ_9 twice:
-// 11.2 GB of a 4,096-ray step). All layers are one launch; the 64-row stages of
+// Bound by HBM (every byte of tape and dZ once, dZ_5, dZ_9 and enc_xyz twice:
+// 11.1 GB of a 4,096-ray step). All layers are one launch; the 64-row stages of
 // all jobs in order are dealt evenly to the pairs, so a pair has one or two
 // layers' sums at a time. The tensor core's FP32 accumulation
 // truncates (4e-6 relative over 4,096 rows of random signs), so an accumulator

@@ -7,9 +7,11 @@
 // in 256..319, later enc_dir in 256..287); the product and its tiling are
 // fp32_tile.cuh's. 100,003 rows: 2.12 ms, 56 TFLOP/s (3.18 ms with one CTA per
 // SM, scalar FMAs and warps of 8 rows x 256 columns), the same outputs bit for
-// bit. (The split products of gemm_fp32_tc.cu would be several times faster, but
-// not the same bits: the training forward's ReLU masks decide the gradient, and
-// the forward and the training forward give the same values.)
+// bit. (The split products of gemm_fp32_tc.cu would be several times faster. They
+// would need a second accumulator and sums in registers like those to be as
+// accurate, and not every output then has the bits that it has had: a
+// pre-activation near 0 on the other side turns a ReLU, and with it the row's
+// gradient.)
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 

@@ -51,10 +51,10 @@
 //   where the sigma head reads it a row per lane: the heads' sums run along a
 //   row in a fixed order. The head weights sit in shared memory (a broadcast
 //   LDS.128 costs two wavefronts).
-// - Eight epilogue warps and four side warps with 128 registers: nothing may
-//   spill, as the 28 KB of L1 beside this much shared memory do not hold
-//   spills and a reload is a trip to L2 (sixteen epilogue warps with 96: 648
-//   us, and 1,190 with 200 bytes of spills, against 610).
+// - Eight epilogue warps and four side warps with 128 registers, of which a
+//   thread spills at most two words: the 28 KB of L1 beside this much shared
+//   memory do not hold spills, and a reload is a trip to L2 (sixteen epilogue
+//   warps with 96: 648 us, and 1,190 with 200 bytes of spills, against 610).
 // - The encodings and dense_9 are the side warps': with the epilogue's eight
 //   warps doing them the tensor core waited ~7k cycles per tile for the heads
 //   at the tile's end and ~2k more behind the sigma head (BF16 607 us, FP8
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
     };
     constexpr int kPk = 64 / (F8 ? 4 : 2);
     const float4 bias9 = ld_here(table + bias_offset(9) + 4 * lane);  // dense_9's of columns 4 lane .. + 3 (BF16)
-        auto from_lane = [](const float4 &v, int src) {
+    auto from_lane = [](const float4 &v, int src) {
       return float4{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
                     __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src)};
     };
@@ -909,9 +909,9 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
     // All eight warps serve whichever sub-tile's accumulator is ready (A, then
     // B, every layer but dense_9). Warp w reads TMEM lane quadrant qd = w % 4
     // (rows 32*qd ..) and column part cq: kCols columns, in BF16 as 64 in either
-    // half of the layer, so that its first half is written first. (Nothing here may
-    // spill: the 28 KB of L1 beside this much shared memory do not hold
-    // spilled registers, and each reload is a trip to L2.)
+    // half of the layer, so that its first half is written first. (Spilled registers
+    // would not stay in the 28 KB of L1 beside this much shared memory: each reload
+    // is a trip to L2.)
     constexpr int kCols = 256 / kParts;
     const int qd = warp & 3, cq = (warp - 2) >> 2;
     const uint32_t tlane = tmem + ((uint32_t)(32 * qd) << 16);
@@ -994,18 +994,17 @@ __global__ void __launch_bounds__(threads_of(STORE), 1)
                 first_half();
               }
             }
-          } else if (g != 7) {
+          } else if (g != 7) {  // (E4M3)
             uint32_t ra[16], rb[16];
             tmem_ld_frag32(ta, ra);
 #pragma unroll
             for (int c = 0; c < kCols / 32; ++c) {
-              const uint32_t dst = fr + (F8 ? 0u : (uint32_t)(c / 2) * kAtom), ch = F8 ? 2u * c : 4u * (c % 2);
               tmem_wait16(ra);
               tmem_ld_frag32(ta + (16u << 16) + 32 * c, rb);
-              store_frag<F8, false>(dst, cx, ch, ra, fb[c % 2], g != 8);
+              store_frag<F8, false>(fr, cx, 2u * c, ra, fb[c % 2], g != 8);
               tmem_wait16(rb);
               if (c + 1 < kCols / 32) tmem_ld_frag32(ta + 32 * (c + 1), ra);
-              store_frag<F8, false>(dst + 16 * 128, cx, ch, rb, fb[c % 2], g != 8);
+              store_frag<F8, false>(fr + 16 * 128, cx, 2u * c, rb, fb[c % 2], g != 8);
               if (c + 2 < kCols / 32) fb[c].load(fbias + 32 * (c + 2), fscale + 32 * (c + 2), lane & 3);
             }
           } else {
