@@ -13,6 +13,7 @@ GEMMs with per-output-channel weight scales (``precision="fp8"``), both
 accumulating in FP32.
 """
 import ctypes
+import operator
 
 import torch
 
@@ -336,6 +337,7 @@ class NeRF:
             raise ValueError("the proposal paths have no coarse maps")
         if int(streams) < 1:
             raise ValueError(f"streams must be at least 1, not {streams}")
+        chunk = operator.index(chunk)
         lib = _lib.lib()
         ws_bytes = (lib.nerfgb_render_gated_workspace_bytes if gated else lib.nerfgb_render_workspace_bytes)(
             min(chunk, R), Sc, Sf)
