@@ -29,12 +29,12 @@
 //
 // Six BF16 products are still four to five times the rate of the FP32 FMA
 // pipe, which bound the kernels before: of a 1,024-ray step's two networks
-// (262,144 rows) dW took 6.2 ms, 1.65 here, and the chain 5.5, 2.1 here. A stage
+// (262,144 rows) dW took 6.2 ms, 1.45 here, and the chain 5.5, 1.97 here. A stage
 // is 3,072 cycles of MMAs, and ~450 KB through an SM's shared memory and L1 (the
 // MMAs' operands 288, the parts' stores, the loads), 3.6k cycles at 128 bytes per
 // cycle. dw_kernel converts both operands with eight warps, which takes longer
-// than the MMAs and the reading of their sums in turn (with four of them 7k
-// cycles per stage, and 12.7k with the MMAs issued by one of them). In
+// than a stage's MMAs (with four of them 7k cycles per stage, and 12.7k with the
+// MMAs issued by one of them). In
 // chain_kernel the sums' warps also write dZ, and a CTA moves ~0.6 MB per layer
 // and tile through L2 (half the stores, of 16 bytes, took as long, tensor stores
 // through shared memory longer).
@@ -195,6 +195,14 @@ __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64
                   idesc, (i == 5 && s == 0) || (first && i + s == 0) ? 0u : 1u);
 }
 
+// A stage is issued in two parts: kEarly of its low products as soon as its
+// operands are there, under the reading of the accumulators of the stage before
+// (unless that reads the low sums too), then the rest. (65,536 rows' backward:
+// 1,055 us without, 955 with 2 in chain_kernel, 936 with 4, 890 in both kernels;
+// with all five low products the issuing warp waits for the tensor core's queue
+// before it reads: 1,028.)
+constexpr int kEarly = 4;
+
 // A warp's part (cols of 128) of an accumulator added to its sums: eight
 // fragments of 16 rows x 32 columns, those from column `cols` on left out.
 __device__ __forceinline__ void add_accumulator(uint32_t taddr, int cols, float (&sum)[4][2][16]) {
@@ -212,10 +220,13 @@ __device__ __forceinline__ void add_accumulator(uint32_t taddr, int cols, float 
   }
 }
 // By a sums' warp: stage q's high sums, at the end of a window also its low ones,
-// added. False after a timeout.
+// added; `begin` runs before they are read. False after a timeout.
+template <typename F>
 __device__ __forceinline__ bool add_stage(uint32_t sbase, uint32_t taddr, uint32_t q, bool low, int cols, int lane,
-                                          float (&sum)[4][2][16], volatile int *abort_flag, int *err) {
+                                          float (&sum)[4][2][16], volatile int *abort_flag, int *err, F begin) {
   if (!__all_sync(0xffffffffu, wait_bar(sbase + kBarDone + 8 * (q & 1u), (q >> 1) & 1u, abort_flag, err))) return false;
+  begin();
+  __syncwarp();
   tc_fence_after();
 #pragma unroll 1
   for (uint32_t at = 0; at <= (low ? 256u : 0u); at += 256u) add_accumulator(taddr + at, cols, sum);
@@ -461,16 +472,22 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool issuer = crank == 0 && threadIdx.x == 0;
     if (issuer) check_tmem(sbase, tmem, abort_flag);
     const volatile Share *share = reinterpret_cast<const volatile Share *>(smem + kShare);
-    auto issue = [&](uint32_t q, uint32_t idesc, bool first) {
+    auto early = [&](uint32_t q, uint32_t idesc, bool first) {
+      const uint32_t sa = sbase + (q & 1u) * kStage;
+      tc_fence_after();
+      issue_products<0, kEarly>(tmem, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc, first);
+    };
+    auto issue = [&](uint32_t q, uint32_t idesc, bool first, bool begun) {
       const uint32_t k = q & 1u, sa = sbase + k * kStage;
-      if (!wait_bar(sbase + kBarFull + 8 * k, (q >> 1) & 1u, abort_flag, err) ||
+      if ((!begun && !wait_bar(sbase + kBarFull + 8 * k, (q >> 1) & 1u, abort_flag, err)) ||
           !wait_bar(sbase + kBarRead, k ^ 1u, abort_flag, err))
         return;
+      if (!begun) early(q, idesc, first);
       tc_fence_after();
-      issue_products<0, 6>(tmem, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc, first);
+      issue_products<kEarly, 6>(tmem, desc_mn_sw128(sa), desc_mn_sw128(sa + kOperand), 2048 >> 4, idesc, false);
       tc_commit_pair(sbase + kBarDone + 8 * k);
     };
-    bool ok = true;
+    bool ok = true, begun = false;  // (of the next stage the early part is issued)
     uint32_t q = 0;  // stages so far
 #pragma unroll 1
     for (int j = 0; j < kJobs && ok; ++j) {
@@ -485,10 +502,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       int window = 0;  // stages in the window of low sums
 #pragma unroll 1
       for (; left > 0 && ok; --left, ++q) {
-        if (issuer) issue(q, share[j].idesc, window == 0);
+        if (issuer) issue(q, share[j].idesc, window == 0, begun);
         __syncwarp();
         const bool end = left == 1 || ++window == kLow;
-        ok = add_stage(sbase, tl + c0, q, end, cols, lane, sum, abort_flag, err);
+        begun = false;
+        ok = add_stage(sbase, tl + c0, q, end, cols, lane, sum, abort_flag, err, [&] {
+          const uint32_t k = (q + 1) & 1u;
+          if (!issuer || end || !mbar_test(sbase + kBarFull + 8 * k, ((q + 1) >> 1) & 1u)) return;
+          early(q + 1, share[j].idesc, false);
+          begun = true;
+        });
         if (end) window = 0;
       }
       if (!ok) break;
@@ -674,10 +697,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t total = (uint32_t)count * first_chunk(0);
     if (issuer) check_tmem(sbase, tmem, abort_flag);
     auto desc = [&](uint32_t addr) { return (uint64_t)kDescHiA << 32 | ((addr & 0x3FFFFu) >> 4) | (1u << 16); };
-    // Stage q is issued in two parts: kEarly of its low products as soon as its
-    // operands are there, under the reading of the accumulators of the stage
-    // before (unless that reads the low sums too), then the rest.
-    constexpr int kEarly = 2;
     auto early = [&](uint32_t q, bool first) {
       const uint32_t sa = sbase + (q & 1u) * kStage;
       tc_fence_after();
@@ -717,12 +736,20 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool last = ch + 1 == chunks;
             if (issuer) {
               if (iq == q) issue(iq++, ch == 0, begun);
-              const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
-              begun = !last && mbar_test(sbase + kBarFull + 8 * k, ph) && mbar_test(sbase + kBarB + 8 * k, ph);
-              if (begun) early(iq, false);
+              begun = false;
             }
+            // (tried as the stage before is issued and, if its operands are not there yet, as that is complete)
+            auto try_early = [&]() {
+              const uint32_t k = iq & 1u, ph = (iq >> 1) & 1u;
+              if (!issuer || last || begun || !mbar_test(sbase + kBarFull + 8 * k, ph) ||
+                  !mbar_test(sbase + kBarB + 8 * k, ph))
+                return;
+              early(iq, false);
+              begun = true;
+            };
+            try_early();
             __syncwarp();
-            if (!(ok = add_stage(sbase, tl, q, last, 128, lane, sum, abort_flag, err))) break;
+            if (!(ok = add_stage(sbase, tl, q, last, 128, lane, sum, abort_flag, err, try_early))) break;
             // the next layer's (the other tile's) first stage under the writing of
             // dZ, unless it waits for that (a tile alone)
             if (issuer && last && subs == 2 && iq < total) issue(iq++, true, false);
