@@ -12,7 +12,7 @@
 // mask) in and 512 bytes of dZ out, ~5.7k cycles of an SM's share of the
 // copy bandwidth per 128 rows against 2,048 cycles of MMAs. A GEMM kernel and
 // a mask kernel per layer moved 2.5 KB per row and layer for the same: 4.4 ms of
-// a 4,096-ray step's two networks against 1.78 here (10.1 GB, 5.7 TB/s).
+// a 4,096-ray step's two networks against 1.63 here (10.1 GB, 6.2 TB/s).
 //
 // The machinery is the forward's (mlp_tc.cu): cluster pairs on two 256-row
 // sub-tiles (128 rows per CTA), 2-SM MMAs (M = 256, N = 256, B = W as [k][n],
@@ -25,7 +25,7 @@
 //     fragments its accumulator has) and stores the masked result in their
 //     place with stmatrix, so the mask needs no room of its own. The copy's
 //     latency (~1.5k cycles) hides behind the other sub-tile; what the region
-//     takes next was fetched into L2 a layer earlier (1.80 -> 1.78 ms);
+//     takes next was fetched into L2 a layer earlier (1 % of the time);
 //   - stores the region to the layer's dZ.
 // Bias sums: a thread's rows, then a reduce-scatter over the warp's row groups
 // and one atomic per column, warp and sub-tile into the CTA's own sums in the
